@@ -133,7 +133,8 @@ def h_diagonals(p, ne, nh, VC, Ee, Eh, gap, excitons=True, stream=None):
     model = abi.model_array(HBAR)
     _lib.call("psb_calch_f64", device.ptr(d_tab), 1, device.ptr(d_td), d_td.numel(),
               device.ptr(d_w), 1, device.ptr(d_y), device.ptr(d_h), nk, nk,
-              flags & (abi.PSB_TAB_SHARED_V | abi.PSB_TAB_SCREENED), abi.as_ptr(model),
+              flags & (abi.PSB_TAB_SHARED_V | abi.PSB_TAB_SCREENED) | abi.PSB_TAB_ONE_CLASS,
+              abi.as_ptr(model),
               device.stream_ptr(stream))
     h = d_h.cpu().numpy()
     return h[:, 0] + 1j * h[:, 1], h[:, 2].copy(), h[:, 3].copy()
@@ -707,7 +708,8 @@ class SBESolver:
         from . import device as _dev
 
         _lib.call("psb_leapfrog_f64", *b._common(), _dev.ptr(order), 1, _dev.ptr(b.y1),
-                  _dev.ptr(b.y), b.n_state, self.Nk, b.tab_flags, _dev.ptr(self._field), 2,
+                  _dev.ptr(b.y), b.n_state, self.Nk, b.tab_flags | abi.PSB_TAB_ONE_CLASS,
+                  _dev.ptr(self._field), 2,
                   self._field.numel(), 1, float(dt), _dev.ptr(b.P), b.P.shape[0], 1,
                   b.p_cap, abi.as_ptr(b.model), _dev.stream_ptr())
         st = int(b.wires()["status"][i])

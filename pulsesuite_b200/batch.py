@@ -61,25 +61,29 @@ class WireBatch:
         self.y1 = None
         self.P = torch.zeros((max(1, self.nw * self.p_cap), 2), dtype=torch.float64,
                              device="cuda")
-        # Launch classes by grid size (registers and shared memory are sized
-        # for a class's largest grid); largest grids first inside a class
-        # balances uneven batches on the CTA scheduler.
+        # Launch classes by grid size: the widths of the FP64 step kernel (a
+        # CTA's threads, registers and shared memory follow from its class).
+        # Several classes run concurrently on side streams, the largest grids
+        # first: alone, a small class leaves most of the GPU idle.
         self.classes = []
         order = np.argsort(-nks, kind="stable").astype(np.int32)
-        for lo, hi in ((0, 256), (256, 512), (512, abi.PSB_MAX_NK)):
+        for lo, hi in ((512, abi.PSB_MAX_NK), (256, 512), (128, 256), (64, 128), (0, 64)):
             sel = order[(nks[order] > lo) & (nks[order] <= hi)]
             if sel.size == 0:
                 continue
             tabs = np.unique(w["table"][sel])
             tf = self.h_tables["flags"][tabs]
-            flags = 0
+            flags = abi.PSB_TAB_ONE_CLASS
             if (tf & abi.PSB_TAB_SCREENED).any():
                 flags |= abi.PSB_TAB_SCREENED
             if (tf & abi.PSB_TAB_SHARED_V).all():
                 flags |= abi.PSB_TAB_SHARED_V
             self.classes.append((torch.as_tensor(sel, device="cuda"), int(nks[sel].max()), flags))
+        self.side_streams = []
         if form == "split":
             self._setup_split()
+        elif len(self.classes) > 1:
+            self.side_streams = self._streams(len(self.classes))
         self.tab_flags = 0
         if (self.h_tables["flags"] & abi.PSB_TAB_SCREENED).any():
             self.tab_flags |= abi.PSB_TAB_SCREENED
@@ -177,14 +181,35 @@ class WireBatch:
             nkmax = int(nks[ga["table"]].max())
             self.wire_launches.append((key[0], device.to_device(ga), len(ga), nkmax, key[1]))
         self.wire_launches.sort(key=lambda l: -l[3])
-        # one stream per class, priorities by grid size (the largest grid's
-        # CTAs run longest, so the CTA scheduler serves them first)
-        least, greatest = torch.cuda.Stream.priority_range()
-        nl = len(self.split_launches) + len(self.wire_launches)
-        self.side_streams = [torch.cuda.Stream(priority=min(least, greatest + r))
-                             for r in range(nl)]
+        self.side_streams = self._streams(len(self.split_launches) + len(self.wire_launches))
         self.ws = torch.zeros(int(lib.psb_split_ws_bytes(self.n_state)), dtype=torch.uint8,
                               device="cuda")
+
+    @staticmethod
+    def _streams(n):
+        """One stream per class, priorities by grid size (the largest grid's
+        CTAs run longest, so the CTA scheduler serves them first)."""
+        least, greatest = torch.cuda.Stream.priority_range()
+        return [torch.cuda.Stream(priority=min(least, greatest + r)) for r in range(n)]
+
+    def _concurrent(self, calls, stream):
+        """Run ``calls`` (one per class, each taking its stream) concurrently
+        on the side streams, ordered after the work queued on ``stream``
+        (default: the current stream) and before what follows on it; a single
+        class without a side stream runs on it."""
+        main = stream if stream is not None else torch.cuda.current_stream()
+        if not self.side_streams:
+            for c in calls:
+                c(main)
+            return
+        fork = torch.cuda.Event()
+        fork.record(main)
+        for c, s in zip(calls, self.side_streams):
+            s.wait_event(fork)
+            c(s)
+            join = torch.cuda.Event()
+            join.record(s)
+            main.wait_event(join)
 
     # -- state --------------------------------------------------------------
     def set_state(self, y, y1=None):
@@ -230,36 +255,23 @@ class WireBatch:
         return dy
 
     def rk4(self, nsteps, dt, p_stride=1, stream=None):
+        tail = (int(nsteps), float(dt), device.ptr(self.P), self.P.shape[0], int(p_stride),
+                self.p_cap, abi.as_ptr(self.model))
+        calls = []
         if self.form == "split":
-            main = stream if stream is not None else torch.cuda.current_stream()
-            streams = self.side_streams
-            fork = torch.cuda.Event()
-            fork.record(main)
-            for s in streams:
-                s.wait_event(fork)
-            for (wg, groups, ng, nkmax), s in zip(self.split_launches, streams):
-                _lib.call("psb_rk4_split", *self._common(), device.ptr(groups), ng, wg, nkmax,
-                          device.ptr(self.y), self.n_state, device.ptr(self.ws), self.ws.numel(),
-                          int(nsteps), float(dt), device.ptr(self.P), self.P.shape[0],
-                          int(p_stride), self.p_cap, abi.as_ptr(self.model),
-                          device.stream_ptr(s))
-            for (wg, groups, ng, nkmax, tflags), s in zip(self.wire_launches,
-                                                         streams[len(self.split_launches):]):
-                _lib.call("psb_rk4_split_wire", *self._common(), device.ptr(groups), ng, wg,
-                          nkmax, tflags, device.ptr(self.y), self.n_state, device.ptr(self.ws),
-                          self.ws.numel(), int(nsteps), float(dt), device.ptr(self.P),
-                          self.P.shape[0], int(p_stride), self.p_cap, abi.as_ptr(self.model),
-                          device.stream_ptr(s))
-            for s in streams:
-                join = torch.cuda.Event()
-                join.record(s)
-                main.wait_event(join)
-            return
-        for order, nkmax, flags in self.classes:
-            _lib.call("psb_rk4_f64", *self._common(), device.ptr(order), order.numel(),
-                      device.ptr(self.y), self.n_state, nkmax, flags, int(nsteps), float(dt),
-                      device.ptr(self.P), self.P.shape[0], int(p_stride), self.p_cap,
-                      abi.as_ptr(self.model), device.stream_ptr(stream))
+            ws = (device.ptr(self.y), self.n_state, device.ptr(self.ws), self.ws.numel())
+            for wg, groups, ng, nkmax in self.split_launches:
+                calls.append(lambda s, a=(device.ptr(groups), ng, wg, nkmax): _lib.call(
+                    "psb_rk4_split", *self._common(), *a, *ws, *tail, device.stream_ptr(s)))
+            for wg, groups, ng, nkmax, tflags in self.wire_launches:
+                calls.append(lambda s, a=(device.ptr(groups), ng, wg, nkmax, tflags): _lib.call(
+                    "psb_rk4_split_wire", *self._common(), *a, *ws, *tail, device.stream_ptr(s)))
+        else:
+            for order, nkmax, flags in self.classes:
+                calls.append(lambda s, o=order, nkm=nkmax, f=flags: _lib.call(
+                    "psb_rk4_f64", *self._common(), device.ptr(o), o.numel(), device.ptr(self.y),
+                    self.n_state, nkm, f, *tail, device.stream_ptr(s)))
+        self._concurrent(calls, stream)
 
     def capture(self, nsteps, dt, p_stride=1):
         """A CUDA graph of one ``rk4(nsteps, dt, p_stride)`` call (every size
@@ -286,9 +298,10 @@ class WireBatch:
         if self.y1 is None:
             self.y1 = self.y.clone()
         assert field.is_cuda and field.dtype == torch.float64 and field.dim() == 2
-        for order, nkmax, flags in self.classes:
-            _lib.call("psb_leapfrog_f64", *self._common(), device.ptr(order), order.numel(),
-                      device.ptr(self.y1), device.ptr(self.y), self.n_state, nkmax, flags,
-                      device.ptr(field), field.shape[1], field.numel(), int(nsteps), float(dt),
-                      device.ptr(self.P), self.P.shape[0], int(p_stride), self.p_cap,
-                      abi.as_ptr(self.model), device.stream_ptr(stream))
+        calls = [lambda s, o=order, nkm=nkmax, f=flags: _lib.call(
+            "psb_leapfrog_f64", *self._common(), device.ptr(o), o.numel(), device.ptr(self.y1),
+            device.ptr(self.y), self.n_state, nkm, f, device.ptr(field), field.shape[1],
+            field.numel(), int(nsteps), float(dt), device.ptr(self.P), self.P.shape[0],
+            int(p_stride), self.p_cap, abi.as_ptr(self.model), device.stream_ptr(s))
+            for order, nkmax, flags in self.classes]
+        self._concurrent(calls, stream)

@@ -1,0 +1,758 @@
+// sbe_conv.cu -- the FP64 SBE step (right-hand side, RK4, leapfrog) of one
+// quantum wire per CTA, with the exchange sums by fast convolution, sm_100a.
+//
+// The exchange sums of a right-hand side (pulsesuite/PSTD3D/SBEs.py:896-921)
+// are three Toeplitz products with the real, even tables V(|k - k'|):
+//   Omega_k += sum_k' Veh p_k'   Se_k -= sum Vee ne   Sh_k -= sum Vhh nh
+// i.e. 8 Nk FP64 flops per point when summed directly.  As cyclic
+// convolutions of length M >= 2 Nk of the complex signals p and ne + i nh
+// (zero beyond Nk) they take one forward and one inverse transform each:
+// about 100 log2(M) flops per point, in FP64 as before (the rounding error
+// is that of a sum: ~1e-16 of the largest term).  A real, even table has a
+// real spectrum, so with one shared table both signals are multiplied by the
+// same real numbers; with distinct Vee and Vhh the second signal's product
+// is Z (Vee + Vhh)/2 + conj(Z(-f)) (Vee - Vhh)/2.
+//
+// Transform.  M = 16 q, q = 8 L with L = 1, 2, 4, 8, 16 lanes (Nk <= 64 L);
+// T = 32 L threads with 8 complex points each:
+//   A   thread (signal, half, a): the 8 points x[a + q r] (the upper 8 of 16
+//       are zero padding and cost nothing); a 16-point transform over r
+//       splits into two of 8 points, the even outputs and (after the roots
+//       of 16) the odd ones; times exp(-2 pi i a g / M), into row g column a;
+//   B   row (signal, g), q points over L lanes of one warp: 8 points per
+//       lane, the roots of q, then L points per lane (a transposition inside
+//       the row, between the lanes of a warp), times the spectrum, and back;
+//   A'  the inverse of A, of whose 16 outputs the 8 wanted ones are formed.
+// So a stage takes four CTA barriers.  The row stride keeps the column and
+// the row accesses of 16-byte elements free of bank conflicts.  8 points per
+// thread and not 16: with 16 (half the threads, M = 32 q, fewer shared-memory
+// passes) the state and a transform did not fit 168 registers, and a lone
+// wire's stage took 1.5 to 2 times as long.  Lengths between the powers of
+// two (rows of 5, 6, 7 points per lane) gained at most 10 % at Nk <= 192 and
+// nothing above: the same instructions with fewer active lanes.
+//
+// The elementwise right-hand side, RK4 combination and sums follow in the
+// same kernel; each thread keeps the base state and the RK accumulator of
+// its (at most 2) points in registers for the whole call.  A wire's
+// arithmetic depends on its own Nk only: threads beyond its own T leave at
+// the start, so its result never depends on the other wires of a launch.
+#include <math.h>
+
+#include "fft64.cuh"
+#include "sbe_f64.cuh"
+
+namespace psb {
+namespace conv {
+
+using fft::Dft;
+using fft::mulw;
+
+constexpr int kEpt = 2;  // points of k per thread
+
+// Lanes of a row.
+__host__ __device__ constexpr int lanes_of(int nk) {
+  return nk <= 64 ? 1 : (nk <= 128 ? 2 : (nk <= 256 ? 4 : (nk <= 512 ? 8 : 16)));
+}
+// Row stride (16-byte elements): room for the transposed row, whose element
+// (l, f) lies at l + (L + 1) f, and the residue modulo 8 that spreads the
+// 8 / L rows of a quarter warp over the banks.
+__host__ __device__ constexpr int stride_of(int L) {
+  return L == 1 ? 9 : (L == 2 ? 26 : (L == 4 ? 44 : 8 * L + 7));
+}
+
+// What a wire's steps need besides its points (shared memory).
+struct Par {
+  double gamma, gap, pscale, L, dens_max, hm;  // hm = mscale / hbar
+  double pulse[2][4];  // t0, 1 / fwhm, -mscale amp (cos, sin)(phase) / hbar
+  double2 drive[2][2]; // [step & 1]: M(t + h/2), M(t + h), over hbar
+  int64_t p_off;
+  double red[3][3][16];  // partial sums [slot][value][warp]
+};
+
+// Shared memory of one wire (bytes) with NT tables.
+template <int L>
+struct Lay {
+  static constexpr int q = 8 * L, np = 8 * q, rs = stride_of(L), T = 32 * L;
+  // pass B's second transform: of D points in one lane, or of 16 over H = 2
+  // lanes; lane l holds f = l % (L / H) + (L / H) it, b = l / (L / H) and the
+  // frequencies g + 16 (f + 8 (H i + b)), whose spectra lie at
+  // (it D + i) 16 L + g L + l
+  static constexpr int H = L == 16 ? 2 : 1, D = L / H, nf = 8 / D;
+  static constexpr int sl = 16 * q;
+  static constexpr uint32_t yp = 32u * rs * 16u;   // after E, [32 rows][rs] complex: p,
+  static constexpr uint32_t yn = yp + np * 16u;    // ne + i nh of the stage point
+  static constexpr uint32_t twa = yn + np * 16u;   // exp(-2 pi i a 2^s / M), [4][q]
+  static constexpr uint32_t twb = twa + 4u * q * 16u;  // exp(-2 pi i l 2^s / q), [3][L]
+  static constexpr uint32_t par = twb + 3u * L * 16u;
+  static constexpr uint32_t s = par + (uint32_t)sizeof(Par);  // spectra [NT][sl]
+  // The tables on their way to S: one table fits the rows of the second
+  // signal, which its transform leaves free; three follow the spectra.
+  static constexpr uint32_t vq1 = 16u * rs * 16u, vq3 = s + 3u * sl * 8u;
+  static constexpr uint32_t total1 = s + sl * 8u, total3 = vq3 + 3u * np * 8u;
+};
+
+// Barrier over the CTA.
+template <int L>
+__device__ __forceinline__ void cta_sync() {
+  if constexpr (L == 1)
+    __syncwarp();
+  else
+    __syncthreads();
+}
+
+// The roots exp(-2 pi i a (2 f + half) / M), f = 4 b + c, as t[c] (v: b = 1).
+template <int q>
+__device__ __forceinline__ void roots_a(const double2* tw, bool half, double2 (&t)[4],
+                                        double2& v) {
+  const double2 u1 = tw[q];
+  t[0] = half ? tw[0] : make_double2(1.0, 0.0);
+  t[1] = mulw<-1>(t[0], u1);
+  const double2 u2 = tw[2 * q];
+  t[2] = mulw<-1>(t[0], u2);
+  t[3] = mulw<-1>(t[1], u2);
+  v = tw[3 * q];
+}
+
+// Pass A on the 8 points in x: output f to o[2 f rs] (row 2 f + half of the
+// signal, column a); tw points at column a of the roots.
+template <int q, int rs>
+__device__ __forceinline__ void pass_a(double2 (&x)[8], double2* o, const double2* tw,
+                                       bool half) {
+  if (half)
+    fft::unroll<8>([&](auto R) {
+      constexpr int r = decltype(R)::value;
+      x[r] = fft::rot16<r, -1>(x[r]);
+    });
+  Dft<8, -1>::run(x);
+  double2 t[4], v;
+  roots_a<q>(tw, half, t, v);
+#pragma unroll
+  for (int f = 0; f < 8; ++f) {
+    double2 z = x[f];
+    if (f >= 4) z = mulw<-1>(z, v);
+    o[2 * f * rs] = mulw<-1>(z, t[f & 3]);
+  }
+}
+
+// Pass A': this half's share of the 8 points a + q r, into its own slots.
+template <int q, int rs>
+__device__ __forceinline__ void pass_a_inv(double2* o, const double2* tw, bool half) {
+  double2 x[8], t[4], v;
+  roots_a<q>(tw, half, t, v);
+#pragma unroll
+  for (int f = 0; f < 8; ++f) {
+    double2 z = mulw<1>(o[2 * f * rs], t[f & 3]);
+    if (f >= 4) z = mulw<1>(z, v);
+    x[f] = z;
+  }
+  Dft<8, 1>::run(x);
+  if (half)
+    fft::unroll<8>([&](auto R) {
+      constexpr int r = decltype(R)::value;
+      x[r] = fft::rot16<r, 1>(x[r]);
+    });
+#pragma unroll
+  for (int r = 0; r < 8; ++r) o[2 * r * rs] = x[r];
+}
+
+// x[f] times the roots exp(SG 2 pi i l f / q) of lane l.
+template <int L, int SG>
+__device__ __forceinline__ void roots_b(double2 (&x)[8], const double2* twb) {
+  const double2 w1 = twb[0], w2 = twb[L], w4 = twb[2 * L];
+  x[1] = mulw<SG>(x[1], w1);
+  x[2] = mulw<SG>(x[2], w2);
+  x[4] = mulw<SG>(x[4], w4);
+  x[5] = mulw<SG>(x[5], mulw<-1>(w1, w4));
+  x[6] = mulw<SG>(x[6], mulw<-1>(w2, w4));
+  const double2 w3 = mulw<-1>(w1, w2);
+  x[3] = mulw<SG>(x[3], w3);
+  x[7] = mulw<SG>(x[7], mulw<-1>(w3, w4));
+}
+
+// What pass B does with a row.
+enum RowOp {
+  kTables = 0,    // forward only: the spectra 2 Re(.) scale of the tables in
+                  // signals 0 and 1 into S[d0], S[d1] (negative: not wanted)
+  kOneTable = 1,  // times S[0], and back
+  kDistinct = 2   // p times S[0]; ne + i nh with S[1], S[2] (half the sum and
+                  // half the difference of the Vee and Vhh spectra), and back
+};
+
+template <int L>
+__device__ __forceinline__ void pass_b(RowOp op, double2* E, double* S, const double2* twb,
+                                       int d0, int d1, double scale) {
+  using Y = Lay<L>;
+  constexpr int H = Y::H, D = Y::D, NF = Y::nf, SL = Y::sl;
+  constexpr int LS = L > 1 ? L + 1 : 1;  // stride of f in the transposed row
+  const int row = (int)threadIdx.x / L, l = (int)threadIdx.x % L, g = row & 15;
+  const int f0 = l % D, b = l / D;
+  double2* R = E + row * Y::rs;
+  double2 z[NF][D];
+  // the radix-2 step between the two lanes of a 16-point transform
+  auto lane_step = [&](double2(&v)[D]) {
+    const double sg = b ? -1.0 : 1.0;
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+      const double ox = __shfl_xor_sync(0xffffffffu, v[i].x, 8);
+      const double oy = __shfl_xor_sync(0xffffffffu, v[i].y, 8);
+      v[i] = make_double2(fma(sg, v[i].x, ox), fma(sg, v[i].y, oy));
+    }
+  };
+  {
+    double2 x[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) x[r] = R[l + L * r];
+    Dft<8, -1>::run(x);
+    if constexpr (L > 1) {
+      roots_b<L, -1>(x, twb + l);
+      __syncwarp();
+#pragma unroll
+      for (int f = 0; f < 8; ++f) R[l + LS * f] = x[f];
+      __syncwarp();
+#pragma unroll
+      for (int it = 0; it < NF; ++it) {
+#pragma unroll
+        for (int i = 0; i < D; ++i) z[it][i] = R[i + D * b + LS * (f0 + D * it)];
+        if constexpr (H == 2) {
+          lane_step(z[it]);
+          if (b)
+            fft::unroll<D>([&](auto I) {
+              constexpr int i = decltype(I)::value;
+              z[it][i] = fft::rot16<i, -1>(z[it][i]);
+            });
+        }
+        Dft<D, -1>::run(z[it]);
+      }
+    } else {
+#pragma unroll
+      for (int f = 0; f < 8; ++f) z[f][0] = x[f];
+    }
+  }
+  double* Sg = S + g * L + l;
+  if (op == kTables) {
+    const int d = row < 16 ? d0 : d1;
+    if (d < 0) return;
+#pragma unroll
+    for (int it = 0; it < NF; ++it)
+#pragma unroll
+      for (int i = 0; i < D; ++i) Sg[d * SL + (it * D + i) * 16 * L] = 2.0 * z[it][i].x * scale;
+    return;
+  }
+  if (op == kOneTable || row < 16) {
+#pragma unroll
+    for (int it = 0; it < NF; ++it)
+#pragma unroll
+      for (int i = 0; i < D; ++i) {
+        const double v = Sg[(it * D + i) * 16 * L];
+        z[it][i].x *= v;
+        z[it][i].y *= v;
+      }
+  }
+  if (op == kDistinct) {
+    // the second signal's product needs its mirrored frequency, which
+    // another row holds; it travels through E
+    if constexpr (H == 2) __syncwarp();
+    if (row >= 16) {
+#pragma unroll
+      for (int it = 0; it < NF; ++it)
+#pragma unroll
+        for (int i = 0; i < D; ++i) R[H * i + b + LS * (f0 + D * it)] = z[it][i];
+    }
+    cta_sync<L>();
+    if (row >= 16) {
+      // frequency g + 16 j, j = f + 8 k; its mirror is row -g, index
+      // q - 1 - j (row 0: q - j, modulo q)
+      const double2* M = E + (16 + ((16 - g) & 15)) * Y::rs;
+#pragma unroll
+      for (int it = 0; it < NF; ++it) {
+        const int f = f0 + D * it;
+        const int fm = g != 0 ? 7 - f : (f > 0 ? 8 - f : 0);
+#pragma unroll
+        for (int i = 0; i < D; ++i) {
+          const int k = H * i + b, im = g == 0 && f == 0 ? (L - k) % L : L - 1 - k;
+          const double2 m = M[im + LS * fm];
+          const double sp = Sg[SL + (it * D + i) * 16 * L];
+          const double sm = Sg[2 * SL + (it * D + i) * 16 * L];
+          z[it][i] = make_double2(fma(m.x, sm, z[it][i].x * sp), fma(-m.y, sm, z[it][i].y * sp));
+        }
+      }
+    }
+    cta_sync<L>();
+  }
+  double2 x[8];
+  if constexpr (L > 1) {
+#pragma unroll
+    for (int it = 0; it < NF; ++it) {
+      Dft<D, 1>::run(z[it]);
+      if constexpr (H == 2) {
+        if (b)
+          fft::unroll<D>([&](auto I) {
+            constexpr int i = decltype(I)::value;
+            z[it][i] = fft::rot16<i, 1>(z[it][i]);
+          });
+        lane_step(z[it]);
+      }
+#pragma unroll
+      for (int i = 0; i < D; ++i) R[i + D * b + LS * (f0 + D * it)] = z[it][i];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int f = 0; f < 8; ++f) x[f] = R[l + LS * f];
+    __syncwarp();
+    roots_b<L, 1>(x, twb + l);
+  } else {
+#pragma unroll
+    for (int f = 0; f < 8; ++f) x[f] = z[f][0];
+  }
+  Dft<8, 1>::run(x);
+#pragma unroll
+  for (int r = 0; r < 8; ++r) R[l + L * r] = x[r];
+}
+
+// CTAs per SM the registers are limited for (16, 16, 20, 24, 16 warps): the
+// best of 16, 20 and 24 warps of 128, 96 and 80 registers per size.
+__host__ __device__ constexpr int ctas_of(int L) {
+  return L == 1 ? 16 : (L == 2 ? 8 : (L == 4 ? 5 : (L == 8 ? 3 : 1)));
+}
+
+// All steps of one wire whose descriptor and table have been checked.
+template <int L>
+__device__ __forceinline__ void wire_steps(const Batch& bt, int mode, bool scr, uint8_t* smem,
+                                           int wi, const PsbTable& tb) {
+  using Y = Lay<L>;
+  constexpr int q = Y::q, np = Y::np, rs = Y::rs, T = Y::T;
+  PsbWire* wp = bt.wires + wi;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nk = tb.nk;
+  const int64_t off = wp->off;
+  const bool one = (tb.flags & PSB_TAB_SHARED_V) != 0;  // one table for all columns
+  const bool exc = (tb.flags & PSB_TAB_EXCITONS) != 0;
+  scr = scr && exc && (tb.flags & PSB_TAB_SCREENED) != 0;
+  double2* E = reinterpret_cast<double2*>(smem);
+  double2* yp = reinterpret_cast<double2*>(smem + Y::yp);
+  double2* yn = reinterpret_cast<double2*>(smem + Y::yn);
+  double2* twa = reinterpret_cast<double2*>(smem + Y::twa);
+  double2* twb = reinterpret_cast<double2*>(smem + Y::twb);
+  double* S = reinterpret_cast<double*>(smem + Y::s);
+  Par& par = *reinterpret_cast<Par*>(smem + Y::par);
+  const double* blk = bt.tabdata + tb.off;
+
+  // ---- roots, parameters, state ----------------------------------------------
+  if (exc) {
+    for (int i = tid; i < 4 * q; i += T) {
+      double sn, cs;
+      sincospi(2.0 / (16 * q) * (double)((i % q) << (i / q)), &sn, &cs);
+      twa[i] = make_double2(cs, -sn);
+    }
+    for (int i = tid; i < 3 * L; i += T) {
+      double sn, cs;
+      sincospi(2.0 / q * (double)((i % L) << (i / L)), &sn, &cs);
+      twb[i] = make_double2(cs, -sn);
+    }
+  }
+  const double ih = 1.0 / bt.hbar;
+  if (tid < 2) {
+    // the drive is a sum of Gaussian pulses (SBEs drive, E(t))
+    double* pc = par.pulse[tid];
+    pc[0] = pc[1] = pc[2] = pc[3] = 0.0;
+    if (tid < wp->npulse && mode != kLeapfrog) {
+      double sn, cs;
+      sincos(wp->phase[tid], &sn, &cs);
+      const double am = -wp->mscale * wp->amp[tid] * ih;
+      pc[0] = wp->t0[tid];
+      pc[1] = 1.0 / wp->fwhm[tid];
+      pc[2] = am * cs;
+      pc[3] = am * sn;
+    }
+    if (tid == 0) {
+      par.gamma = wp->gamma;
+      par.gap = wp->gap;
+      par.pscale = wp->pscale;
+      par.L = tb.L;
+      par.dens_max = tb.dens_max;
+      par.hm = wp->mscale * ih;
+      par.p_off = wp->p_off;
+    }
+  }
+  // pass A: signal (p, ne + i nh), half, column
+  const int grp = tid / (8 * L), col = tid - grp * 8 * L, sig = grp >> 1;
+  const bool half = (grp & 1) != 0;
+  double2* ea = E + (16 * sig + half) * rs + col;  // rows 2 f further
+  double yb[kEpt][4];  // base state / leapfrog X1
+  double acc[kEpt][3];  // RK accumulator of p and of n (dn_e/dt = dn_h/dt)
+  double ekh[kEpt];     // (Ee + Eh + gap) / hbar
+  int eo[kEpt];  // place of k's sums in E: rows 2 r and 2 r + 1, column a of k = a + q r
+  double nsum = 0.0;
+  {
+    const double2* y2 = reinterpret_cast<const double2*>(bt.y + 4 * off);
+    const double2* y1 = reinterpret_cast<const double2*>(bt.y1 + 4 * off);
+    const double gap = wp->gap;
+#pragma unroll
+    for (int e = 0; e < kEpt; ++e) {
+      const int k = tid + e * T;
+      double2 a = make_double2(0.0, 0.0), b = a;
+      eo[e] = 2 * (k / q) * rs + k % q;
+      ekh[e] = 0.0;
+      if (k < nk) {
+        a = y2[2 * k];
+        b = y2[2 * k + 1];
+        ekh[e] = (blk[3 * nk + k] + gap + blk[4 * nk + k]) * ih;
+        nsum += b.x + b.y;
+      }
+      yp[k] = a;
+      yn[k] = b;
+      if (mode == kLeapfrog && k < nk) {
+        a = y1[2 * k];
+        b = y1[2 * k + 1];
+      }
+      yb[e][0] = a.x;
+      yb[e][1] = a.y;
+      yb[e][2] = b.x;
+      yb[e][3] = b.y;
+      acc[e][0] = acc[e][1] = acc[e][2] = 0.0;
+    }
+  }
+  // M / hbar at t0 and t1 into dst[0], dst[1]: lanes 0, 1 of the calling warp
+  // take the two pulses at t0, lanes 2, 3 the same at t1
+  auto drive2 = [&](double t0, double t1, double2* dst) {
+    double vr = 0.0, vi = 0.0;
+    if (lane < 4) {
+      const double* pc = par.pulse[lane & 1];
+      const double u = ((lane & 2 ? t1 : t0) - pc[0]) * pc[1];
+      const double env = exp(-4.0 * 0.69314718055994530942 * u * u);
+      vr = pc[2] * env;
+      vi = pc[3] * env;
+    }
+    vr += __shfl_xor_sync(0xffffffffu, vr, 1);
+    vi += __shfl_xor_sync(0xffffffffu, vi, 1);
+    if (lane < 4 && (lane & 1) == 0) dst[lane >> 1] = make_double2(vr, vi);
+  };
+  // partial sums: [slot][value][warp]
+  auto put = [&](int slot, int v, double x) {
+    x = warp_sum(x);
+    if (lane == 0) par.red[slot][v][warp] = x;
+  };
+  auto get = [&](int slot, int v) {
+    double t = 0.0;
+#pragma unroll 1
+    for (int i = 0; i < L; ++i) t += par.red[slot][v][i];
+    return t;
+  };
+  if (scr) put(0, 0, nsum);
+  const double h = bt.dt;
+  double t = wp->t;
+  const int steps0 = wp->steps;
+  __syncwarp();
+  if (mode != kLeapfrog && warp == 0) drive2(t, t, par.drive[1]);
+  cta_sync<L>();
+
+  const int nst = (mode == kRhs || mode == kCalcH) ? 1 : bt.nsteps;
+  const int nstage = mode == kRk4 ? 4 : 1;
+  for (int s = 0; s < nst; ++s) {
+    double2 m_lf = make_double2(0.0, 0.0);
+    if (mode == kLeapfrog) {
+      const int64_t fi = (int64_t)wi * bt.field_stride + 2 * ((int64_t)steps0 + s);
+      if (bt.field && fi >= 0 && fi + 1 < bt.n_field) {
+        m_lf = make_double2(-par.hm * bt.field[fi], -par.hm * bt.field[fi + 1]);
+      }
+    } else if (mode == kRk4) {
+      // read by all after the next barrier; M(t) is the last step's M(t + h)
+      if (warp == 0) drive2(t + h / 2.0, t + h, par.drive[s & 1]);
+      if (!exc) cta_sync<L>();
+    }
+    for (int st = 0; st < nstage; ++st) {
+      if (exc) {
+        // the stage's tables: once per call, or screened by the stage point
+        // (coulomb.py:1218-1230) every time
+        const bool build = scr || (s == 0 && st == 0);
+        double* vq = reinterpret_cast<double*>(smem + (one ? Y::vq1 : Y::vq3));
+        if (build) {
+          double n1d = 0.0;
+          if (scr) {
+            n1d = get(0, 0) / 2.0 / par.L;
+            n1d = n1d < par.dens_max ? n1d : par.dens_max;
+          }
+          for (int d = tid; d < np; d += T) {
+            const bool in = d > 0 && d < nk;
+            const double ie = in && scr ? 1.0 / eps1d(blk, nk, d, n1d) : 1.0;
+            for (int n = 0; n < (one ? 1 : 3); ++n)
+              vq[n * np + d] = in ? blk[n * nk + d] * ie : 0.0;
+          }
+          cta_sync<L>();
+        }
+        // rounds: the tables' spectra (Veh and Vee, then Vhh), the stage point
+        for (int rnd = build ? (one ? 1 : 0) : 2; rnd < 3; ++rnd) {
+          if (rnd == 2 || sig == 0 || (rnd == 0 && !one)) {
+            double2 x[8];
+            if (rnd == 2) {
+              const double2* src = (sig == 0 ? yp : yn) + col;
+#pragma unroll
+              for (int r = 0; r < 8; ++r) x[r] = src[q * r];
+            } else {
+              const double* src = vq + (rnd == 0 ? sig : (one ? 0 : 2)) * np + col;
+#pragma unroll
+              for (int r = 0; r < 8; ++r) x[r] = make_double2(src[q * r], 0.0);
+            }
+            pass_a<q, rs>(x, ea, twa + col, half);
+          }
+          cta_sync<L>();
+          pass_b<L>(rnd < 2 ? kTables : (one ? kOneTable : kDistinct), E, S, twb,
+                       rnd == 0 || one ? 0 : 2, rnd == 0 ? 1 : -1, 1.0 / (bt.hbar * (16 * q)));
+          cta_sync<L>();
+          if (rnd == 1 && !one) {
+            // half the sum and half the difference of the Vee and Vhh spectra
+            for (int i = tid; i < Y::sl; i += T) {
+              const double e = S[Y::sl + i], hh = S[2 * Y::sl + i];
+              S[Y::sl + i] = 0.5 * (e + hh);
+              S[2 * Y::sl + i] = 0.5 * (e - hh);
+            }
+          }
+        }
+        pass_a_inv<q, rs>(ea, twa + col, half);
+        cta_sync<L>();
+      }
+      // M(t), M(t + h/2) twice, M(t + h)
+      const double2 m = mode == kLeapfrog
+                            ? m_lf
+                            : (st == 0 ? par.drive[(s + 1) & 1][1]
+                                       : par.drive[s & 1][st == 3 ? 1 : 0]);
+      const double gamma = par.gamma;
+      double v0 = 0.0, v1 = 0.0;
+      nsum = 0.0;
+#pragma unroll
+      for (int e = 0; e < kEpt; ++e) {
+        const int k = tid + e * T;
+        if (k >= nk) continue;
+        double2 om = m;
+        double xe = 0.0, xh = 0.0;
+        if (exc) {
+          const double2* o = E + eo[e];
+          const double2 p0 = o[0], p1 = o[rs], n0 = o[16 * rs], n1 = o[17 * rs];
+          om.x += p0.x + p1.x;
+          om.y += p0.y + p1.y;
+          xe = n0.x + n1.x;
+          xh = n0.y + n1.y;
+        }
+        if (mode == kCalcH) {
+          // renormalised H diagonals (CalcH, SBEs.py:819-935): Heh (Rabi
+          // frequency), Hee, Hhh in the slots of dy
+          const double hb = bt.hbar;
+          double2* d2 = reinterpret_cast<double2*>(bt.dy + 4 * off);
+          d2[2 * k] = make_double2(om.x * hb, om.y * hb);
+          d2[2 * k + 1] = make_double2((blk[3 * nk + k] + par.gap) - xe * hb,
+                                       blk[4 * nk + k] - xh * hb);
+          continue;
+        }
+        // diagonal of dpdt, dCdt, dDdt (SBEs.py:1962-1975, 2325-2337,
+        // 2623-2636), everything over hbar
+        const double2 p = yp[k], n = yn[k];
+        const double sh = ekh[e] - (xe + xh), nn = n.x + n.y - 1.0;
+        const double f0 = sh * p.y - om.y * nn - gamma * p.x;
+        const double f1 = om.x * nn - sh * p.x - gamma * p.y;
+        const double f2 = 2.0 * (om.y * p.x - om.x * p.y);
+        if (mode == kRhs) {
+          double2* d2 = reinterpret_cast<double2*>(bt.dy + 4 * off);
+          d2[2 * k] = make_double2(f0, f1);
+          d2[2 * k + 1] = make_double2(f2, f2);
+        } else if (mode == kRk4) {
+          // stages of integrator.py:143-157; acc = k1 + 2 k2 + 2 k3
+          double g0 = f0, g1 = f1, g2 = f2;
+          const double c = st == 2 ? h : (st == 3 ? h / 6.0 : h / 2.0);
+          if (st == 0) {
+            acc[e][0] = f0;
+            acc[e][1] = f1;
+            acc[e][2] = f2;
+          } else if (st < 3) {
+            acc[e][0] += 2.0 * f0;
+            acc[e][1] += 2.0 * f1;
+            acc[e][2] += 2.0 * f2;
+          } else {
+            g0 += acc[e][0];
+            g1 += acc[e][1];
+            g2 += acc[e][2];
+          }
+          const double2 zp = make_double2(yb[e][0] + c * g0, yb[e][1] + c * g1);
+          const double2 zn = make_double2(yb[e][2] + c * g2, yb[e][3] + c * g2);
+          yp[k] = zp;
+          yn[k] = zn;
+          if (st == 3) {
+            yb[e][0] = zp.x;
+            yb[e][1] = zp.y;
+            yb[e][2] = zn.x;
+            yb[e][3] = zn.y;
+            v0 += zp.x;
+            v1 += zp.y;
+          }
+          nsum += zn.x + zn.y;
+        } else {
+          // leapfrog X3 = X1 + 2 dt f(X2) (SBEs.py:5685-5687), in the place of
+          // X2 (this thread's own points; all sums over X2 are done), and the
+          // occupations |n| for the rescale (SBEs.py:5704-5711)
+          yp[k] = make_double2(yb[e][0] + f0 * h * 2.0, yb[e][1] + f1 * h * 2.0);
+          const double2 n3 = make_double2(fabs(yb[e][2] + f2 * h * 2.0),
+                                          fabs(yb[e][3] + f2 * h * 2.0));
+          yn[k] = n3;
+          v0 += n3.x;
+          v1 += n3.y;
+        }
+      }
+      if (mode == kRhs || mode == kCalcH) return;
+      if (mode == kRk4) {
+        if (scr) put(0, 0, nsum);
+        if (st == 3) {
+          put(1, 0, v0);
+          put(1, 1, v1);
+        }
+      } else {
+        put(2, 0, v0);
+        put(2, 1, v1);
+        cta_sync<L>();
+        const double te = get(2, 0), th = get(2, 1);
+        const double total = (te + th) / 2.0, small = 1e-200;
+        const double ce = total / (te + small), ch = total / (th + small);
+        v0 = v1 = 0.0;
+#pragma unroll
+        for (int e = 0; e < kEpt; ++e) {
+          const int k = tid + e * T;
+          if (k >= nk) continue;
+          const double2 x3 = yp[k];
+          double2 n3 = yn[k];
+          n3 = make_double2(n3.x * ce, n3.y * ch);
+          yn[k] = n3;
+          yb[e][0] = (yb[e][0] + x3.x) / 2.0;
+          yb[e][1] = (yb[e][1] + x3.y) / 2.0;
+          yb[e][2] = (yb[e][2] + n3.x) / 2.0;
+          yb[e][3] = (yb[e][3] + n3.y) / 2.0;
+          nsum += n3.x + n3.y;
+          v0 += x3.x;
+          v1 += x3.y;
+        }
+        if (scr) put(0, 0, nsum);
+        put(1, 0, v0);
+        put(1, 1, v1);
+      }
+      cta_sync<L>();
+    }
+    t = t + h;
+    // P(t) record (qwoptics.py:815-946, diagonal: pscale * sum_k p_k)
+    if (tid == 0 && bt.P && bt.p_stride > 0 && (s + 1) % bt.p_stride == 0) {
+      const int r = (s + 1) / bt.p_stride - 1;
+      const int64_t po = par.p_off;
+      if (r < bt.p_cap && po >= 0 && po + r < bt.n_P) {
+        const double ps = par.pscale;
+        bt.P[2 * (po + r)] = ps * get(1, 0);
+        bt.P[2 * (po + r) + 1] = ps * get(1, 1);
+      }
+    }
+  }
+
+  // Write the state back; flag non-finite wires.
+  bool bad = false;
+  double2* yo = reinterpret_cast<double2*>(bt.y + 4 * off);
+  double2* y1o = reinterpret_cast<double2*>(bt.y1 + 4 * off);
+#pragma unroll
+  for (int e = 0; e < kEpt; ++e) {
+    const int k = tid + e * T;
+    if (k >= nk) continue;
+    const double2 a = yp[k], b = yn[k];
+    yo[2 * k] = a;
+    yo[2 * k + 1] = b;
+    bad |= !(isfinite(a.x) && isfinite(a.y) && isfinite(b.x) && isfinite(b.y));
+    if (mode == kLeapfrog) {
+      y1o[2 * k] = make_double2(yb[e][0], yb[e][1]);
+      y1o[2 * k + 1] = make_double2(yb[e][2], yb[e][3]);
+      bad |= !(isfinite(yb[e][0]) && isfinite(yb[e][1]) && isfinite(yb[e][2]) &&
+               isfinite(yb[e][3]));
+    }
+  }
+  put(2, 2, bad ? 1.0 : 0.0);
+  cta_sync<L>();
+  if (tid == 0) {
+    wp->t = t;
+    wp->steps = steps0 + nst;
+    if (get(2, 2) != 0.0 && wp->status == PSB_OK) wp->status = PSB_ERR_NONFINITE;
+  }
+}
+
+// A launch covers the wires of its grid whose own Nk takes L lanes; the others
+// are another launch's, unless the caller said that there are none (strict).
+// check: this launch reports bad descriptors.
+template <int L>
+__global__ void __launch_bounds__(32 * L, ctas_of(L))
+    sbe_conv_kernel(Batch bt, int mode, bool screened, bool shared, bool check, bool strict) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  const int wi = bt.order ? bt.order[blockIdx.x] : (int)blockIdx.x;
+  if (wi < 0 || wi >= bt.nw) return;
+  PsbWire* wp = bt.wires + wi;
+  const int table = wp->table;
+  int bad = PSB_OK;
+  PsbTable tb{};
+  if (table < 0 || table >= bt.ntab) {
+    bad = PSB_ERR_INVALID;
+  } else {
+    tb = bt.tables[table];
+    const int64_t off = wp->off;
+    if (tb.nk < 2 || tb.nk > bt.nk_limit || off < 0 || off + tb.nk > bt.n_state || tb.off < 0 ||
+        tb.off + 9 * (int64_t)tb.nk > bt.n_tabdata || (strict && lanes_of(tb.nk) != L))
+      bad = PSB_ERR_SIZE;
+    else if (shared && (tb.flags & PSB_TAB_SHARED_V) == 0)
+      bad = PSB_ERR_INVALID;
+  }
+  if (bad != PSB_OK) {
+    if (check && threadIdx.x == 0) wp->status = bad;
+    return;
+  }
+  if (lanes_of(tb.nk) == L) wire_steps<L>(bt, mode, screened, smem, wi, tb);
+}
+
+template <int L>
+uint32_t smem_of(bool shared) {
+  return shared ? Lay<L>::total1 : Lay<L>::total3;
+}
+
+template <int L>
+int launch_lanes(const Batch& bt, int mode, int grid, bool screened, bool shared, bool check,
+                 bool strict, cudaStream_t st) {
+  const uint32_t smem = smem_of<L>(shared);
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(
+        sbe_conv_kernel<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess)
+      return set_error(PSB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  }
+  sbe_conv_kernel<L><<<grid, 32 * L, smem, st>>>(bt, mode, screened, shared, check, strict);
+  return check_cuda("sbe_conv_kernel");
+}
+
+// One launch per width from that of nkmax down to that of nkmin + 1.
+template <int L>
+int launch_down(const Batch& bt, int mode, int grid, int nkmax, int nkmin, bool screened,
+                bool shared, bool one_class, cudaStream_t st) {
+  const int top = lanes_of(nkmax);
+  if (L <= top && L >= lanes_of(nkmin + 1)) {
+    const int rc =
+        launch_lanes<L>(bt, mode, grid, screened, shared, L == top, one_class, st);
+    if (rc != PSB_OK || one_class) return rc;
+  }
+  if constexpr (L > 1)
+    return launch_down<L / 2>(bt, mode, grid, nkmax, nkmin, screened, shared, one_class, st);
+  return PSB_OK;
+}
+
+}  // namespace conv
+
+size_t conv_smem_bytes(int nk, bool shared) {
+  switch (conv::lanes_of(nk)) {
+    case 1: return conv::smem_of<1>(shared);
+    case 2: return conv::smem_of<2>(shared);
+    case 4: return conv::smem_of<4>(shared);
+    case 8: return conv::smem_of<8>(shared);
+    default: return conv::smem_of<16>(shared);
+  }
+}
+
+int launch_sbe_conv(const Batch& bt, int mode, int grid, int nkmax, int nkmin, bool screened,
+                    bool shared, bool one_class, cudaStream_t st) {
+  return conv::launch_down<16>(bt, mode, grid, nkmax, nkmin, screened, shared, one_class, st);
+}
+
+}  // namespace psb

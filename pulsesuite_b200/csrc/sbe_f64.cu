@@ -1,11 +1,14 @@
-// sbe_f64.cu -- fused FP64 SBE right-hand side, RK4 step and leapfrog step.
+// sbe_f64.cu -- the FP64 SBE entry points and the direct kernel of a single
+// right-hand side.
 //
-// One CTA owns one wire for the whole call: the wire's state stays in shared
-// memory and registers across all `nsteps` steps, so HBM sees the state once
-// in and once out per call.  Work per right-hand side is dominated by the
-// three Toeplitz exchange sums (pulsesuite/PSTD3D/SBEs.py:896-921):
+// RK4, leapfrog and the right-hand sides of large grids run in sbe_conv.cu.
+// One right-hand side (or one CalcH) of a grid of Nk <= kDirectNk sums its
+// three Toeplitz exchange products directly here (pulsesuite/PSTD3D/SBEs.py:
+// 896-921),
 //   Omega_k += sum_k' Veh(|k-k'|) p_k'   Se_k -= sum Vee ne   Sh_k -= sum Vhh nh
-// i.e. 4 FP64 FMAs per (k, k') pair.
+// i.e. 4 FP64 FMAs per (k, k') pair, one CTA per wire: a transform has its
+// roots and the tables' spectra to make first, which only many right-hand
+// sides on the same grid repay.
 //
 // Exchange mapping.  Thread (ob, kc) owns R consecutive outputs
 // k = ob*R .. ob*R+R-1 and a chunk of sources k' (kc selects the chunk).  For
@@ -21,14 +24,16 @@
 // of the launch.
 #include <math.h>
 
-#include "psb_common.cuh"
+#include "sbe_f64.cuh"
 
 namespace psb {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-
-enum Mode { kRhs = 0, kRk4 = 1, kLeapfrog = 2, kCalcH = 3 };
+// Largest grid of the direct kernel: one point of k per thread.  Measured on
+// B200, one right-hand side, direct / transforms (us): Nk 256, 16 wires 15.7 /
+// 16.5, 2048 wires 68 / 35; Nk 512, 16 wires 20.6 / 17.6, 2048 wires 215 / 69.
+constexpr int kDirectNk = kThreads;
 
 struct Geo {
   int nk, nkp, nb, kc, chunk, yslen, doff, vlen, vphys;
@@ -55,7 +60,7 @@ __host__ __device__ inline Geo geometry(int nk) {
 
 // Shared-memory layout (doubles) of one wire.
 struct Smem {
-  int ys, red, v, eps, stage, scratch, total;
+  int ys, red, v, eps, scratch, total;
 };
 
 template <int R>
@@ -65,8 +70,7 @@ __host__ __device__ inline Smem smem_layout(const Geo& g, int ntab) {
   s.red = s.ys + 4 * g.yslen;        // [kc][4][nkp] partial exchange sums
   s.v = s.red + 4 * g.kc * g.nkp;    // ntab skewed symmetric tables of vphys
   s.eps = s.v + ntab * g.vphys;      // eps(q) when screened (nkp)
-  s.stage = s.eps + g.nkp;           // [8][nkp]: RK4 k1 and k2/k2+k3, leapfrog X3
-  s.scratch = s.stage + 8 * g.nkp;   // block reductions: kWarps*4 + 4
+  s.scratch = s.eps + g.nkp;         // block reductions: kWarps*4 + 4
   s.total = s.scratch + kWarps * 4 + 4;
   return s;
 }
@@ -75,31 +79,6 @@ template <int R>
 __device__ __forceinline__ int skew(int i) {
   return i + i / R;
 }
-
-struct Batch {
-  const PsbTable* tables;
-  int ntab;
-  const double* tabdata;
-  int64_t n_tabdata;
-  PsbWire* wires;
-  int nw;
-  const int32_t* order;
-  double* y;   // RK4 state, leapfrog X2, RHS input
-  double* y1;  // leapfrog X1
-  double* dy;  // RHS output
-  int64_t n_state;
-  const double* field;
-  int64_t field_stride;
-  int64_t n_field;
-  int nsteps;
-  double dt;
-  double* P;
-  int64_t n_P;
-  int p_stride;
-  int p_cap;
-  double hbar;
-  int nk_limit;  // largest nk the launch's shared memory was sized for
-};
 
 // Sum of n <= 4 values over the block; every thread returns the same totals.
 __device__ __forceinline__ void block_sum(double* v, int n, double* scratch) {
@@ -281,34 +260,34 @@ __device__ __forceinline__ void rhs_element(const Geo& g, int k, const double* y
   f[3] = dn;
 }
 
-template <int R, int EPT, int MODE, bool SCREEN, int NT>
-__global__ void __launch_bounds__(kThreads, EPT <= 2 ? 2 : 1) sbe_f64_kernel(Batch bt) {
+template <int R, int MODE, bool SCREEN, int NT>
+__global__ void __launch_bounds__(kThreads, 2) sbe_f64_kernel(Batch bt, bool check) {
   extern __shared__ double smem[];
   const int wi = bt.order ? bt.order[blockIdx.x] : (int)blockIdx.x;
   if (wi < 0 || wi >= bt.nw) return;
   PsbWire* wp = bt.wires + wi;
   const PsbWire w = *wp;
   if (w.table < 0 || w.table >= bt.ntab) {
-    if (threadIdx.x == 0) wp->status = PSB_ERR_INVALID;
+    if (check && threadIdx.x == 0) wp->status = PSB_ERR_INVALID;
     return;
   }
   const PsbTable tb = bt.tables[w.table];
   if (tb.nk < 2 || tb.nk > bt.nk_limit || w.off < 0 || w.off + tb.nk > bt.n_state ||
       tb.off < 0 || tb.off + 9 * (int64_t)tb.nk > bt.n_tabdata) {
-    if (threadIdx.x == 0) wp->status = PSB_ERR_SIZE;
+    if (check && threadIdx.x == 0) wp->status = PSB_ERR_SIZE;
     return;
   }
   if (NT == 1 && (tb.flags & PSB_TAB_SHARED_V) == 0) {
-    if (threadIdx.x == 0) wp->status = PSB_ERR_INVALID;
+    if (check && threadIdx.x == 0) wp->status = PSB_ERR_INVALID;
     return;
   }
+  if (tb.nk > kDirectNk) return;  // the transforms' wire
   const Geo g = geometry<R>(tb.nk);
   const Smem L = smem_layout<R>(g, NT);
   double* ys = smem + L.ys;
   double* red = smem + L.red;
   double* vs = smem + L.v;
   double* eps = smem + L.eps;
-  double* stage = smem + L.stage;
   double* scratch = smem + L.scratch;
   const double* blk = bt.tabdata + tb.off;
   const double* Ee = blk + 3 * tb.nk;
@@ -316,223 +295,56 @@ __global__ void __launch_bounds__(kThreads, EPT <= 2 ? 2 : 1) sbe_f64_kernel(Bat
   const bool exc = (tb.flags & PSB_TAB_EXCITONS) != 0;
   const bool scr = SCREEN && (tb.flags & PSB_TAB_SCREENED) != 0;
   const double hbar = bt.hbar;
-  const double hg = hbar * w.gamma;
   const int tid = threadIdx.x;
-  const int nkp = g.nkp;
 
   // Zero the padded sources, load the state.
   for (int i = tid; i < 4 * g.yslen; i += kThreads) ys[i] = 0.0;
   __syncthreads();
-  double yb[EPT][4];  // RK4 base state / leapfrog X1
-  const double2* y2 = reinterpret_cast<const double2*>(bt.y + 4 * w.off);
-  const double2* y1g = MODE == kLeapfrog ? reinterpret_cast<const double2*>(bt.y1 + 4 * w.off)
-                                         : nullptr;
-#pragma unroll
-  for (int e = 0; e < EPT; ++e) {
-    int k = tid + e * kThreads;
-    if (k < g.nk) {
-      double2 pa = y2[2 * k], pb = y2[2 * k + 1];
-      ys[k] = pa.x;
-      ys[g.yslen + k] = pa.y;
-      ys[2 * g.yslen + k] = pb.x;
-      ys[3 * g.yslen + k] = pb.y;
-      if (MODE == kLeapfrog) {
-        double2 qa = y1g[2 * k], qb = y1g[2 * k + 1];
-        yb[e][0] = qa.x;
-        yb[e][1] = qa.y;
-        yb[e][2] = qb.x;
-        yb[e][3] = qb.y;
-      } else {
-        yb[e][0] = pa.x;
-        yb[e][1] = pa.y;
-        yb[e][2] = pb.x;
-        yb[e][3] = pb.y;
-      }
-    }
+  const int k = tid;
+  if (k < g.nk) {
+    const double2* y2 = reinterpret_cast<const double2*>(bt.y + 4 * w.off);
+    const double2 pa = y2[2 * k], pb = y2[2 * k + 1];
+    ys[k] = pa.x;
+    ys[g.yslen + k] = pa.y;
+    ys[2 * g.yslen + k] = pb.x;
+    ys[3 * g.yslen + k] = pb.y;
   }
   if (exc && !scr) fill_tables<R, NT, false>(g, blk, vs, eps);
   __syncthreads();
-
-  const int nst = (MODE == kRhs || MODE == kCalcH) ? 1 : bt.nsteps;
-  const int nstage = MODE == kRk4 ? 4 : 1;
-  const double h = bt.dt;
-  double t = w.t;
-  int steps = w.steps;
-  for (int s = 0; s < nst; ++s) {
-    double er_lf = 0.0, ei_lf = 0.0;
-    if (MODE == kLeapfrog) {
-      int64_t fi = (int64_t)wi * bt.field_stride + 2 * (int64_t)steps;
-      if (bt.field && fi >= 0 && fi + 1 < bt.n_field) {
-        er_lf = bt.field[fi];
-        ei_lf = bt.field[fi + 1];
-      }
-    }
-    for (int st = 0; st < nstage; ++st) {
-      if (exc) {
-        if (scr) {
-          screen_stage(g, tb, blk, ys, eps, scratch);
-          fill_tables<R, NT, true>(g, blk, vs, eps);
-          __syncthreads();
-        }
-        exchange<R, NT>(g, ys, vs, red);
-      }
-      __syncthreads();
-      double er, ei;
-      if (MODE == kLeapfrog) {
-        er = er_lf;
-        ei = ei_lf;
-      } else {
-        double ts = st == 0 ? t : (st == 3 ? t + h : t + h / 2.0);
-        drive(w, ts, er, ei);
-      }
-      const double mr = -w.mscale * er, mi = -w.mscale * ei;
-#pragma unroll
-      for (int e = 0; e < EPT; ++e) {
-        const int k = tid + e * kThreads;
-        if (k >= g.nk) continue;
-        double f[4];
-        if (MODE == kCalcH) {
-          // renormalised H diagonals (CalcH, SBEs.py:819-935): Heh (Rabi
-          // frequency), Hee, Hhh in the slots of dy
-          double omr = mr, omi = mi, xe = 0.0, xh = 0.0;
-          if (exc) {
-            for (int c = 0; c < g.kc; ++c) {
-              const double* rr = red + (size_t)c * 4 * g.nkp;
-              omr += rr[k];
-              omi += rr[g.nkp + k];
-              xe += rr[2 * g.nkp + k];
-              xh += rr[3 * g.nkp + k];
-            }
-          }
-          double2* d2 = reinterpret_cast<double2*>(bt.dy + 4 * w.off);
-          d2[2 * k] = make_double2(omr, omi);
-          d2[2 * k + 1] = make_double2((Ee[k] + w.gap) - xe, Eh[k] - xh);
-          continue;
-        }
-        rhs_element(g, k, ys, red, Ee, Eh, w.gap, hg, hbar, mr, mi, exc, f);
-        if (MODE == kRhs) {
-          double2* d2 = reinterpret_cast<double2*>(bt.dy + 4 * w.off);
-          d2[2 * k] = make_double2(f[0], f[1]);
-          d2[2 * k + 1] = make_double2(f[2], f[3]);
-        } else if (MODE == kRk4) {
-          // Stage order of integrator.py:143-157; k1 in stage[c], k2 and
-          // then k3 + k2 in stage[4 + c] (owner-thread slots, no sync needed).
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            double* k1 = stage + c * nkp + k;
-            double* dym = stage + (4 + c) * nkp + k;
-            double v;
-            if (st == 0) {
-              *k1 = f[c];
-              v = yb[e][c] + (h / 2.0) * f[c];
-            } else if (st == 1) {
-              *dym = f[c];
-              v = yb[e][c] + (h / 2.0) * f[c];
-            } else if (st == 2) {
-              v = yb[e][c] + h * f[c];
-              *dym = f[c] + *dym;
-            } else {
-              yb[e][c] = yb[e][c] + (h / 6.0) * ((*k1 + f[c]) + 2.0 * *dym);
-              v = yb[e][c];
-            }
-            ys[c * g.yslen + k] = v;
-          }
-        } else {
-          // Leapfrog X3 = X1 + 2 dt f(X2) (SBEs.py:5685-5687), kept in stage[c].
-#pragma unroll
-          for (int c = 0; c < 4; ++c) stage[c * nkp + k] = yb[e][c] + f[c] * h * 2.0;
-        }
-      }
+  if (exc) {
+    if (scr) {
+      screen_stage(g, tb, blk, ys, eps, scratch);
+      fill_tables<R, NT, true>(g, blk, vs, eps);
       __syncthreads();
     }
-    if (MODE == kRhs || MODE == kCalcH) break;
-    if (MODE == kLeapfrog) {
-      // Population neutrality and reshuffle (SBEs.py:5704-5718).
-      double v[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-      for (int e = 0; e < EPT; ++e) {
-        const int k = tid + e * kThreads;
-        if (k < g.nk) {
-          double a = fabs(stage[2 * nkp + k]), b = fabs(stage[3 * nkp + k]);
-          stage[2 * nkp + k] = a;
-          stage[3 * nkp + k] = b;
-          v[0] += a;
-          v[1] += b;
-        }
-      }
-      block_sum(v, 2, scratch);
-      const double total = (v[0] + v[1]) / 2.0;
-      const double small = 1e-200;
-#pragma unroll
-      for (int e = 0; e < EPT; ++e) {
-        const int k = tid + e * kThreads;
-        if (k < g.nk) {
-          stage[2 * nkp + k] = stage[2 * nkp + k] * total / (v[0] + small);
-          stage[3 * nkp + k] = stage[3 * nkp + k] * total / (v[1] + small);
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const double x3 = stage[c * nkp + k];
-            yb[e][c] = (yb[e][c] + x3) / 2.0;
-            ys[c * g.yslen + k] = x3;
-          }
-        }
-      }
-      __syncthreads();
-    }
-    t = t + h;
-    steps += 1;
-    // P(t) record (qwoptics.py:815-946, diagonal: pscale * sum_k p_k).
-    if (bt.P && bt.p_stride > 0 && (s + 1) % bt.p_stride == 0) {
-      const int r = (s + 1) / bt.p_stride - 1;
-      double v[2] = {0.0, 0.0};
-#pragma unroll
-      for (int e = 0; e < EPT; ++e) {
-        const int k = tid + e * kThreads;
-        if (k < g.nk) {
-          v[0] += ys[k];
-          v[1] += ys[g.yslen + k];
-        }
-      }
-      block_sum(v, 2, scratch);
-      if (tid == 0 && r < bt.p_cap && w.p_off >= 0 && w.p_off + r < bt.n_P) {
-        bt.P[2 * (w.p_off + r)] = w.pscale * v[0];
-        bt.P[2 * (w.p_off + r) + 1] = w.pscale * v[1];
-      }
-    }
+    exchange<R, NT>(g, ys, vs, red);
   }
-  if (MODE == kRhs || MODE == kCalcH) return;
-
-  // Write the state back; flag non-finite wires.
-  bool bad = false;
-  double2* yo = reinterpret_cast<double2*>(bt.y + 4 * w.off);
-  double2* y1o = MODE == kLeapfrog ? reinterpret_cast<double2*>(bt.y1 + 4 * w.off) : nullptr;
-#pragma unroll
-  for (int e = 0; e < EPT; ++e) {
-    const int k = tid + e * kThreads;
-    if (k < g.nk) {
-      double a = ys[k], b = ys[g.yslen + k], c = ys[2 * g.yslen + k], d = ys[3 * g.yslen + k];
-      if (MODE == kRk4) {
-        a = yb[e][0];
-        b = yb[e][1];
-        c = yb[e][2];
-        d = yb[e][3];
-      }
-      yo[2 * k] = make_double2(a, b);
-      yo[2 * k + 1] = make_double2(c, d);
-      bad |= !(isfinite(a) && isfinite(b) && isfinite(c) && isfinite(d));
-      if (MODE == kLeapfrog) {
-        y1o[2 * k] = make_double2(yb[e][0], yb[e][1]);
-        y1o[2 * k + 1] = make_double2(yb[e][2], yb[e][3]);
-        bad |= !(isfinite(yb[e][0]) && isfinite(yb[e][1]) && isfinite(yb[e][2]) &&
-                 isfinite(yb[e][3]));
+  __syncthreads();
+  double er, ei;
+  drive(w, w.t, er, ei);
+  const double mr = -w.mscale * er, mi = -w.mscale * ei;
+  if (k >= g.nk) return;
+  double2* d2 = reinterpret_cast<double2*>(bt.dy + 4 * w.off);
+  if (MODE == kCalcH) {
+    // renormalised H diagonals (CalcH, SBEs.py:819-935): Heh (Rabi
+    // frequency), Hee, Hhh in the slots of dy
+    double omr = mr, omi = mi, xe = 0.0, xh = 0.0;
+    if (exc) {
+      for (int c = 0; c < g.kc; ++c) {
+        const double* rr = red + (size_t)c * 4 * g.nkp;
+        omr += rr[k];
+        omi += rr[g.nkp + k];
+        xe += rr[2 * g.nkp + k];
+        xh += rr[3 * g.nkp + k];
       }
     }
-  }
-  bad = __syncthreads_or(bad);
-  if (tid == 0) {
-    wp->t = t;
-    wp->steps = steps;
-    if (bad && wp->status == PSB_OK) wp->status = PSB_ERR_NONFINITE;
+    d2[2 * k] = make_double2(omr, omi);
+    d2[2 * k + 1] = make_double2((Ee[k] + w.gap) - xe, Eh[k] - xh);
+  } else {
+    double f[4];
+    rhs_element(g, k, ys, red, Ee, Eh, w.gap, hbar * w.gamma, hbar, mr, mi, exc, f);
+    d2[2 * k] = make_double2(f[0], f[1]);
+    d2[2 * k + 1] = make_double2(f[2], f[3]);
   }
 }
 
@@ -544,52 +356,51 @@ size_t smem_bytes_for(int nk, int ntab) {
 }
 
 template <int MODE, bool SCREEN, int NT>
-static int launch_ept(const Batch& bt, int ept, int grid, size_t smem, cudaStream_t st) {
-  void (*kern)(Batch) = nullptr;
-  switch (ept) {
-    case 1: kern = sbe_f64_kernel<kR, 1, MODE, SCREEN, NT>; break;
-    case 2: kern = sbe_f64_kernel<kR, 2, MODE, SCREEN, NT>; break;
-    case 4: kern = sbe_f64_kernel<kR, 4, MODE, SCREEN, NT>; break;
-    default: return set_error(PSB_ERR_SIZE, "unsupported elements per thread %d", ept);
+static int launch_direct(const Batch& bt, int grid, int nkmax, bool check, cudaStream_t st) {
+  size_t smem = 0;
+  for (int nk = 2; nk <= nkmax && nk <= kDirectNk; ++nk) {
+    const size_t b = smem_bytes_for(nk, NT);
+    if (b > smem) smem = b;
   }
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
+  const cudaError_t e = cudaFuncSetAttribute(
+      sbe_f64_kernel<kR, MODE, SCREEN, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess)
     return set_error(PSB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-  kern<<<grid, kThreads, smem, st>>>(bt);
+  sbe_f64_kernel<kR, MODE, SCREEN, NT><<<grid, kThreads, smem, st>>>(bt, check);
   return check_cuda("sbe_f64_kernel");
 }
 
 template <int MODE>
-static int launch_mode(const Batch& bt, int ept, int grid, size_t smem, bool screened,
-                       bool shared, cudaStream_t st) {
+static int launch_direct_mode(const Batch& bt, int grid, int nkmax, bool screened, bool shared,
+                              bool check, cudaStream_t st) {
   if (screened)
-    return shared ? launch_ept<MODE, true, 1>(bt, ept, grid, smem, st)
-                  : launch_ept<MODE, true, 3>(bt, ept, grid, smem, st);
-  return shared ? launch_ept<MODE, false, 1>(bt, ept, grid, smem, st)
-                : launch_ept<MODE, false, 3>(bt, ept, grid, smem, st);
+    return shared ? launch_direct<MODE, true, 1>(bt, grid, nkmax, check, st)
+                  : launch_direct<MODE, true, 3>(bt, grid, nkmax, check, st);
+  return shared ? launch_direct<MODE, false, 1>(bt, grid, nkmax, check, st)
+                : launch_direct<MODE, false, 3>(bt, grid, nkmax, check, st);
 }
 
-// Host-side launch: sizes shared memory for the largest grid of the launch.
+// Host-side launch of a mode over n_order wires (bt.order) or all nw.
 int launch_sbe_f64(Batch bt, int mode, int n_order, int nkmax, int tab_flags, cudaStream_t st) {
   if (nkmax < 2 || nkmax > PSB_MAX_NK)
     return set_error(PSB_ERR_SIZE, "nk %d outside [2, %d]", nkmax, PSB_MAX_NK);
   const bool screened = (tab_flags & PSB_TAB_SCREENED) != 0;
   const bool shared = (tab_flags & PSB_TAB_SHARED_V) != 0;
+  const bool one_class = (tab_flags & PSB_TAB_ONE_CLASS) != 0;
   bt.nk_limit = nkmax;
-  size_t smem = 0;
-  for (int nk = 2; nk <= nkmax; ++nk) {
-    size_t b = smem_bytes_for(nk, shared ? 1 : 3);
-    if (b > smem) smem = b;
-  }
-  int ept = (nkmax + kThreads - 1) / kThreads;
-  if (ept == 3) ept = 4;
   const int grid = bt.order ? n_order : bt.nw;
   if (grid <= 0) return PSB_OK;
-  if (mode == kRhs) return launch_mode<kRhs>(bt, ept, grid, smem, screened, shared, st);
-  if (mode == kCalcH) return launch_mode<kCalcH>(bt, ept, grid, smem, screened, shared, st);
-  if (mode == kRk4) return launch_mode<kRk4>(bt, ept, grid, smem, screened, shared, st);
-  return launch_mode<kLeapfrog>(bt, ept, grid, smem, screened, shared, st);
+  const bool once = mode == kRhs || mode == kCalcH;
+  if (!once) return launch_sbe_conv(bt, mode, grid, nkmax, 0, screened, shared, one_class, st);
+  if (nkmax > kDirectNk) {
+    const int rc =
+        launch_sbe_conv(bt, mode, grid, nkmax, kDirectNk, screened, shared, one_class, st);
+    if (rc != PSB_OK || one_class) return rc;
+  }
+  const bool check = nkmax <= kDirectNk;
+  return mode == kRhs
+             ? launch_direct_mode<kRhs>(bt, grid, nkmax, screened, shared, check, st)
+             : launch_direct_mode<kCalcH>(bt, grid, nkmax, screened, shared, check, st);
 }
 
 }  // namespace psb
@@ -598,7 +409,13 @@ using namespace psb;
 
 extern "C" int psb_f64_smem_bytes(int nk, int tab_flags) {
   if (nk < 2 || nk > PSB_MAX_NK) return set_error(PSB_ERR_SIZE, "nk %d out of range", nk);
-  return (int)smem_bytes_for(nk, (tab_flags & PSB_TAB_SHARED_V) ? 1 : 3);
+  const bool shared = (tab_flags & PSB_TAB_SHARED_V) != 0;
+  size_t b = conv_smem_bytes(nk, shared);
+  if (nk <= kDirectNk) {
+    const size_t d = smem_bytes_for(nk, shared ? 1 : 3);
+    b = d > b ? d : b;
+  }
+  return (int)b;
 }
 
 static int common_checks(const PsbTable* d_tables, int ntab, const double* d_tabdata,

@@ -452,7 +452,8 @@ class Server:
                                self.P.shape[0], 1, self.max_steps, self._model_ptr,
                                self.device.stream_ptr(sm))
             else:
-                flags = abi.PSB_TAB_SHARED_V if (self.h_tables["flags"][ti] & abi.PSB_TAB_SHARED_V) else 0
+                flags = abi.PSB_TAB_ONE_CLASS | int(self.h_tables["flags"][ti]
+                                                    & abi.PSB_TAB_SHARED_V)
                 self._lib.call("psb_rk4_f64", *common, ptr, n_launch, self._y_ptr,
                                self.n_state, nk, flags, self.chunk, dt, self._P_ptr,
                                self.P.shape[0], 1, self.max_steps, self._model_ptr,
