@@ -20,22 +20,35 @@
 //       splits into two of 8 points, the even outputs and (after the roots
 //       of 16) the odd ones; times exp(-2 pi i a g / M), into row g column a;
 //   B   row (signal, g), q points over L lanes of one warp: 8 points per
-//       lane, the roots of q, then L points per lane (a transposition inside
-//       the row, between the lanes of a warp), times the spectrum, and back;
+//       lane, the roots of q, then L points (between the two lanes by
+//       shuffles for L = 2, by a transposition inside the row above), times the
+//       spectrum, and back;
 //   A'  the inverse of A, of whose 16 outputs the 8 wanted ones are formed.
 // So a stage takes four CTA barriers.  The row stride keeps the column and
 // the row accesses of 16-byte elements free of bank conflicts.  8 points per
-// thread and not 16: with 16 (half the threads, M = 32 q, fewer shared-memory
-// passes) the state and a transform did not fit 168 registers, and a lone
-// wire's stage took 1.5 to 2 times as long.  Lengths between the powers of
-// two (rows of 5, 6, 7 points per lane) gained at most 10 % at Nk <= 192 and
-// nothing above: the same instructions with fewer active lanes.
+// thread and not 16: with 16 (half the threads, fewer shared-memory passes)
+// the state and a transform did not fit 168 registers, and a lone wire's stage
+// took 1.5 to 2 times as long.  Lengths between the powers of two (rows of 5,
+// 6, 7 points per lane) gained at most 10 % at Nk <= 192 and nothing above:
+// the same instructions with fewer active lanes.
 //
 // The elementwise right-hand side, RK4 combination and sums follow in the
 // same kernel; each thread keeps the base state and the RK accumulator of
 // its (at most 2) points in registers for the whole call.  A wire's
-// arithmetic depends on its own Nk only: threads beyond its own T leave at
-// the start, so its result never depends on the other wires of a launch.
+// arithmetic depends on its own Nk only (a launch takes the wires of its own
+// L), so its result never depends on the other wires of a launch.
+//
+// What bounds it: shared-memory traffic, about 460 wavefronts per warp and
+// stage (86 % of the pipe at Nk 512), with the FP64 pipe at 54 % beside it; a
+// lone wire is bound by the latency of its stages.  Measured
+// on B200 against the direct sums it replaces (us per wire-stage and SM, 3552
+// wires; in brackets us per stage of one wire; screened):
+//   Nk      direct                transforms
+//   64      1.44 (2.47)  2.1      0.22 (1.88)  0.45
+//   128     1.98 (3.07)  2.9      0.52 (2.15)  0.96
+//   256     4.49 (5.79)  5.7      1.08 (2.39)  1.85
+//   512     14.9 (16.6)  17.0     2.35 (3.56)  3.98
+//   1024    60.0 (60.2)  58.7     6.10 (6.44)  9.98
 #include <math.h>
 
 #include "fft64.cuh"
@@ -47,37 +60,39 @@ namespace conv {
 using fft::Dft;
 using fft::mulw;
 
-constexpr int kEpt = 2;  // points of k per thread
+constexpr int kEpt = 2;    // points of k per thread
+constexpr int kDrive = 8;  // steps whose drive is evaluated at once
 
 // Lanes of a row.
 __host__ __device__ constexpr int lanes_of(int nk) {
   return nk <= 64 ? 1 : (nk <= 128 ? 2 : (nk <= 256 ? 4 : (nk <= 512 ? 8 : 16)));
 }
-// Row stride (16-byte elements): room for the transposed row, whose element
-// (l, f) lies at l + (L + 1) f, and the residue modulo 8 that spreads the
-// 8 / L rows of a quarter warp over the banks.
+// Row stride (16-byte elements): the residue modulo 8 that spreads the 8 / L
+// rows of a quarter warp over the banks, and from L = 4 room for the
+// transposed row, whose element (l, f) lies at l + (L + 1) f.
 __host__ __device__ constexpr int stride_of(int L) {
-  return L == 1 ? 9 : (L == 2 ? 26 : (L == 4 ? 44 : 8 * L + 7));
+  return L == 1 ? 9 : (L == 2 ? 18 : (L == 4 ? 44 : 8 * L + 7));
 }
 
 // What a wire's steps need besides its points (shared memory).
 struct Par {
-  double gamma, gap, pscale, L, dens_max, hm;  // hm = mscale / hbar
+  double gamma, gap, pscale, half_l, dens_max, hm;  // 1 / (2 L), mscale / hbar
   double pulse[2][4];  // t0, 1 / fwhm, -mscale amp (cos, sin)(phase) / hbar
-  double2 drive[2][2]; // [step & 1]: M(t + h/2), M(t + h), over hbar
+  double2 drive[kDrive + 1][2];  // M / hbar at t + h/2, t + h of kDrive steps; M(t)
   int64_t p_off;
-  double red[3][3][16];  // partial sums [slot][value][warp]
+  double red[2][4][16];  // partial sums [parity][value][warp]
 };
 
 // Shared memory of one wire (bytes) with NT tables.
 template <int L>
 struct Lay {
   static constexpr int q = 8 * L, np = 8 * q, rs = stride_of(L), T = 32 * L;
-  // pass B's second transform: of D points in one lane, or of 16 over H = 2
-  // lanes; lane l holds f = l % (L / H) + (L / H) it, b = l / (L / H) and the
-  // frequencies g + 16 (f + 8 (H i + b)), whose spectra lie at
-  // (it D + i) 16 L + g L + l
-  static constexpr int H = L == 16 ? 2 : 1, D = L / H, nf = 8 / D;
+  // pass B's second transform, of L points: over H lanes by shuffles, D = L /
+  // H points in each; lane l holds f = l % D + D it and the frequencies
+  // g + 16 (f + 8 (H i + b)), b the lane's place among the H, whose spectra
+  // lie at (it D + i) 16 L + g L + l
+  static constexpr int H = L == 16 || L == 2 ? 2 : 1, D = L / H, nf = 8 / D;
+  static constexpr int LS = L >= 4 ? L + 1 : L;  // stride of f in the transposed row
   static constexpr int sl = 16 * q;
   static constexpr uint32_t yp = 32u * rs * 16u;   // after E, [32 rows][rs] complex: p,
   static constexpr uint32_t yn = yp + np * 16u;    // ne + i nh of the stage point
@@ -171,40 +186,42 @@ __device__ __forceinline__ void roots_b(double2 (&x)[8], const double2* twb) {
 
 // What pass B does with a row.
 enum RowOp {
-  kTables = 0,    // forward only: the spectra 2 Re(.) scale of the tables in
-                  // signals 0 and 1 into S[d0], S[d1] (negative: not wanted)
+  kTables = 0,    // forward only, of the even tables: Veh in signal 0 (its
+                  // spectrum, the real part, into S[0]) and Vee + i Vhh in
+                  // signal 1 (half sum and half difference into S[1], S[2])
   kOneTable = 1,  // times S[0], and back
-  kDistinct = 2   // p times S[0]; ne + i nh with S[1], S[2] (half the sum and
-                  // half the difference of the Vee and Vhh spectra), and back
+  kDistinct = 2   // p times S[0]; ne + i nh with S[1], S[2], and back
 };
 
 template <int L>
-__device__ __forceinline__ void pass_b(RowOp op, double2* E, double* S, const double2* twb,
-                                       int d0, int d1, double scale) {
+__device__ __forceinline__ void pass_b(RowOp op, bool one, double2* E, double* S,
+                                       const double2* twb, double scale) {
   using Y = Lay<L>;
-  constexpr int H = Y::H, D = Y::D, NF = Y::nf, SL = Y::sl;
-  constexpr int LS = L > 1 ? L + 1 : 1;  // stride of f in the transposed row
+  constexpr int H = Y::H, D = Y::D, NF = Y::nf, SL = Y::sl, LS = Y::LS;
   const int row = (int)threadIdx.x / L, l = (int)threadIdx.x % L, g = row & 15;
   const int f0 = l % D, b = l / D;
   double2* R = E + row * Y::rs;
   double2 z[NF][D];
-  // the radix-2 step between the two lanes of a 16-point transform
-  auto lane_step = [&](double2(&v)[D]) {
-    const double sg = b ? -1.0 : 1.0;
-#pragma unroll
-    for (int i = 0; i < D; ++i) {
-      const double ox = __shfl_xor_sync(0xffffffffu, v[i].x, 8);
-      const double oy = __shfl_xor_sync(0xffffffffu, v[i].y, 8);
-      v[i] = make_double2(fma(sg, v[i].x, ox), fma(sg, v[i].y, oy));
-    }
+  // a radix-2 step between lanes `mask` apart: sums below, differences above
+  auto step = [&](double2& v, int mask) {
+    const double sg = (l & mask) ? -1.0 : 1.0;
+    const double ox = __shfl_xor_sync(0xffffffffu, v.x, mask);
+    const double oy = __shfl_xor_sync(0xffffffffu, v.y, mask);
+    v = make_double2(fma(sg, v.x, ox), fma(sg, v.y, oy));
   };
   {
     double2 x[8];
 #pragma unroll
     for (int r = 0; r < 8; ++r) x[r] = R[l + L * r];
     Dft<8, -1>::run(x);
-    if constexpr (L > 1) {
-      roots_b<L, -1>(x, twb + l);
+    if constexpr (L > 1) roots_b<L, -1>(x, twb + l);
+    if constexpr (D == 1) {
+#pragma unroll
+      for (int f = 0; f < 8; ++f) {
+        if constexpr (L == 2) step(x[f], 1);
+        z[f][0] = x[f];
+      }
+    } else {
       __syncwarp();
 #pragma unroll
       for (int f = 0; f < 8; ++f) R[l + LS * f] = x[f];
@@ -214,7 +231,8 @@ __device__ __forceinline__ void pass_b(RowOp op, double2* E, double* S, const do
 #pragma unroll
         for (int i = 0; i < D; ++i) z[it][i] = R[i + D * b + LS * (f0 + D * it)];
         if constexpr (H == 2) {
-          lane_step(z[it]);
+#pragma unroll
+          for (int i = 0; i < D; ++i) step(z[it][i], 8);
           if (b)
             fft::unroll<D>([&](auto I) {
               constexpr int i = decltype(I)::value;
@@ -223,19 +241,21 @@ __device__ __forceinline__ void pass_b(RowOp op, double2* E, double* S, const do
         }
         Dft<D, -1>::run(z[it]);
       }
-    } else {
-#pragma unroll
-      for (int f = 0; f < 8; ++f) z[f][0] = x[f];
     }
   }
   double* Sg = S + g * L + l;
   if (op == kTables) {
-    const int d = row < 16 ? d0 : d1;
-    if (d < 0) return;
+    if (row >= 16 && one) return;
+    double* d = Sg + (row < 16 ? 0 : SL);
 #pragma unroll
     for (int it = 0; it < NF; ++it)
 #pragma unroll
-      for (int i = 0; i < D; ++i) Sg[d * SL + (it * D + i) * 16 * L] = 2.0 * z[it][i].x * scale;
+      for (int i = 0; i < D; ++i) {
+        const double2 c = z[it][i];
+        const int o = (it * D + i) * 16 * L;
+        d[o] = row < 16 ? c.x * scale : 0.5 * scale * (c.x + c.y);
+        if (row >= 16) d[SL + o] = 0.5 * scale * (c.x - c.y);
+      }
     return;
   }
   if (op == kOneTable || row < 16) {
@@ -251,7 +271,7 @@ __device__ __forceinline__ void pass_b(RowOp op, double2* E, double* S, const do
   if (op == kDistinct) {
     // the second signal's product needs its mirrored frequency, which
     // another row holds; it travels through E
-    if constexpr (H == 2) __syncwarp();
+    __syncwarp();
     if (row >= 16) {
 #pragma unroll
       for (int it = 0; it < NF; ++it)
@@ -280,7 +300,13 @@ __device__ __forceinline__ void pass_b(RowOp op, double2* E, double* S, const do
     cta_sync<L>();
   }
   double2 x[8];
-  if constexpr (L > 1) {
+  if constexpr (D == 1) {
+#pragma unroll
+    for (int f = 0; f < 8; ++f) {
+      x[f] = z[f][0];
+      if constexpr (L == 2) step(x[f], 1);
+    }
+  } else {
 #pragma unroll
     for (int it = 0; it < NF; ++it) {
       Dft<D, 1>::run(z[it]);
@@ -290,7 +316,8 @@ __device__ __forceinline__ void pass_b(RowOp op, double2* E, double* S, const do
             constexpr int i = decltype(I)::value;
             z[it][i] = fft::rot16<i, 1>(z[it][i]);
           });
-        lane_step(z[it]);
+#pragma unroll
+        for (int i = 0; i < D; ++i) step(z[it][i], 8);
       }
 #pragma unroll
       for (int i = 0; i < D; ++i) R[i + D * b + LS * (f0 + D * it)] = z[it][i];
@@ -299,28 +326,78 @@ __device__ __forceinline__ void pass_b(RowOp op, double2* E, double* S, const do
 #pragma unroll
     for (int f = 0; f < 8; ++f) x[f] = R[l + LS * f];
     __syncwarp();
-    roots_b<L, 1>(x, twb + l);
-  } else {
-#pragma unroll
-    for (int f = 0; f < 8; ++f) x[f] = z[f][0];
   }
+  if constexpr (L > 1) roots_b<L, 1>(x, twb + l);
   Dft<8, 1>::run(x);
 #pragma unroll
   for (int r = 0; r < 8; ++r) R[l + L * r] = x[r];
 }
 
-// CTAs per SM the registers are limited for (16, 16, 20, 24, 16 warps): the
-// best of 16, 20 and 24 warps of 128, 96 and 80 registers per size.
-__host__ __device__ constexpr int ctas_of(int L) {
-  return L == 1 ? 16 : (L == 2 ? 8 : (L == 4 ? 5 : (L == 8 ? 3 : 1)));
+// log |a / b| with one division: with x = |a| 2^-e, y = |b|, x / y in
+// [0.7, 1.42], it is e log 2 + 2 atanh((x - y) / (x + y)), the inverse
+// hyperbolic tangent by its Taylor series (|argument| < 0.172: the terms left
+// out are below 3e-17 of it).  far: a or b is zero, not finite or near the
+// ends of the range, and the result is not it.
+__device__ __forceinline__ double log_ratio(double a, double b, bool& far) {
+  double x = fabs(a);
+  const double y = fabs(b);
+  far |= !(x > 1e-290 && y > 1e-290 && x < 1e290 && y < 1e290);
+  int e = (__double2hiint(x) >> 20) - (__double2hiint(y) >> 20);
+  x = __hiloint2double(__double2hiint(x) - e * (1 << 20), __double2loint(x));  // x / y in (1/2, 2)
+  const int up = x > 1.41 * y ? 1 : (x < 0.705 * y ? -1 : 0);
+  x = __hiloint2double(__double2hiint(x) - up * (1 << 20), __double2loint(x));
+  e += up;
+  const double s = (x - y) / (x + y), s2 = s * s;
+  double p = 1.0 / 19.0;
+#pragma unroll
+  for (int k = 8; k >= 1; --k) p = fma(p, s2, 1.0 / (2 * k + 1));
+  return fma((double)e, 0.69314718055994530942, fma(2.0 * s * s2, p, 2.0 * s));
 }
 
-// All steps of one wire whose descriptor and table have been checked.
+// CTAs per SM the registers are limited for: 16 warps of 128 registers, the
+// best of 16, 20 and 24 for L = 1, 2, 16; 20 of 96 for L = 4 (Nk 256: 1.08
+// against 1.15 us per wire-stage and SM); 24 of 80 for L = 8, as fast as 16 on
+// full waves and with a third more wires in flight on short ones.
+__host__ __device__ constexpr int ctas_of(int L) {
+  return L == 16 ? 1 : (L == 4 ? 5 : (L == 8 ? 3 : 16 / L));
+}
+
+// Sums over the CTA in a fixed order: a warp's K = 2 or 4 sums at once (each
+// step of the butterfly halves the values a lane carries, so K values take K + 2
+// or so shuffles of a double, not 5 K) into red[v][warp].
+template <int K>
+__device__ __forceinline__ void put_sums(double (&v)[K], double (*red)[16], int lane, int warp) {
+  int o = 16;
+#pragma unroll
+  for (int c = K / 2; c >= 1; c /= 2, o /= 2) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < c; ++i) {
+      const double send = up ? v[i] : v[i + c], keep = up ? v[i + c] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  for (; o >= 1; o /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  // lane bits from 16 down chose the value
+  constexpr int S = 32 / K;
+  if (lane % S == 0) red[lane / S][warp] = v[0];
+}
 template <int L>
+__device__ __forceinline__ double get_sum(const double (*red)[16], int v) {
+  double t = red[v][0];
+#pragma unroll
+  for (int i = 1; i < L; ++i) t += red[v][i];
+  return t;
+}
+
+// All steps of one wire whose descriptor and table have been checked.  ONCE:
+// one right-hand side or CalcH (mode), else RK4 or leapfrog steps (MODE).
+template <int L, int MODE>
 __device__ __forceinline__ void wire_steps(const Batch& bt, int mode, bool scr, uint8_t* smem,
                                            int wi, const PsbTable& tb) {
   using Y = Lay<L>;
   constexpr int q = Y::q, np = Y::np, rs = Y::rs, T = Y::T;
+  constexpr bool ONCE = MODE == kRhs;
   PsbWire* wp = bt.wires + wi;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nk = tb.nk;
   const int64_t off = wp->off;
@@ -354,7 +431,7 @@ __device__ __forceinline__ void wire_steps(const Batch& bt, int mode, bool scr, 
     // the drive is a sum of Gaussian pulses (SBEs drive, E(t))
     double* pc = par.pulse[tid];
     pc[0] = pc[1] = pc[2] = pc[3] = 0.0;
-    if (tid < wp->npulse && mode != kLeapfrog) {
+    if (tid < wp->npulse && MODE != kLeapfrog) {
       double sn, cs;
       sincos(wp->phase[tid], &sn, &cs);
       const double am = -wp->mscale * wp->amp[tid] * ih;
@@ -367,7 +444,7 @@ __device__ __forceinline__ void wire_steps(const Batch& bt, int mode, bool scr, 
       par.gamma = wp->gamma;
       par.gap = wp->gap;
       par.pscale = wp->pscale;
-      par.L = tb.L;
+      par.half_l = 1.0 / (2.0 * tb.L);
       par.dens_max = tb.dens_max;
       par.hm = wp->mscale * ih;
       par.p_off = wp->p_off;
@@ -377,11 +454,10 @@ __device__ __forceinline__ void wire_steps(const Batch& bt, int mode, bool scr, 
   const int grp = tid / (8 * L), col = tid - grp * 8 * L, sig = grp >> 1;
   const bool half = (grp & 1) != 0;
   double2* ea = E + (16 * sig + half) * rs + col;  // rows 2 f further
-  double yb[kEpt][4];  // base state / leapfrog X1
+  double yb[kEpt][4];   // base state / leapfrog X1
   double acc[kEpt][3];  // RK accumulator of p and of n (dn_e/dt = dn_h/dt)
   double ekh[kEpt];     // (Ee + Eh + gap) / hbar
-  int eo[kEpt];  // place of k's sums in E: rows 2 r and 2 r + 1, column a of k = a + q r
-  double nsum = 0.0;
+  double nsum = 0.0;    // sum of n_e + n_h over this thread's points
   {
     const double2* y2 = reinterpret_cast<const double2*>(bt.y + 4 * off);
     const double2* y1 = reinterpret_cast<const double2*>(bt.y1 + 4 * off);
@@ -390,7 +466,6 @@ __device__ __forceinline__ void wire_steps(const Batch& bt, int mode, bool scr, 
     for (int e = 0; e < kEpt; ++e) {
       const int k = tid + e * T;
       double2 a = make_double2(0.0, 0.0), b = a;
-      eo[e] = 2 * (k / q) * rs + k % q;
       ekh[e] = 0.0;
       if (k < nk) {
         a = y2[2 * k];
@@ -400,7 +475,7 @@ __device__ __forceinline__ void wire_steps(const Batch& bt, int mode, bool scr, 
       }
       yp[k] = a;
       yn[k] = b;
-      if (mode == kLeapfrog && k < nk) {
+      if (MODE == kLeapfrog && k < nk) {
         a = y1[2 * k];
         b = y1[2 * k + 1];
       }
@@ -411,55 +486,63 @@ __device__ __forceinline__ void wire_steps(const Batch& bt, int mode, bool scr, 
       acc[e][0] = acc[e][1] = acc[e][2] = 0.0;
     }
   }
-  // M / hbar at t0 and t1 into dst[0], dst[1]: lanes 0, 1 of the calling warp
-  // take the two pulses at t0, lanes 2, 3 the same at t1
-  auto drive2 = [&](double t0, double t1, double2* dst) {
-    double vr = 0.0, vi = 0.0;
-    if (lane < 4) {
-      const double* pc = par.pulse[lane & 1];
-      const double u = ((lane & 2 ? t1 : t0) - pc[0]) * pc[1];
-      const double env = exp(-4.0 * 0.69314718055994530942 * u * u);
-      vr = pc[2] * env;
-      vi = pc[3] * env;
-    }
+  const double h = bt.dt, h2 = h / 2.0, h6 = h / 6.0;
+  double t = wp->t;
+  const int steps0 = wp->steps, nst = ONCE ? 1 : bt.nsteps;
+  // warp 0: the drive of steps s .. s + kDrive - 1, whose first begins at t
+  // (t advances by repeated addition, as the steps' t does); lane bits: pulse,
+  // t + h/2 or t + h, step.  M(t) of step s, the last value before, moves to
+  // the end of the table.
+  auto drive_ahead = [&](double t0) {
+    const int j = lane >> 2;
+    for (int i = 0; i < kDrive - 1; ++i)
+      if (i < j) t0 = t0 + h;
+    const double* pc = par.pulse[lane & 1];
+    const double u = ((lane & 2 ? t0 + h : t0 + h2) - pc[0]) * pc[1];
+    const double env = exp(-4.0 * 0.69314718055994530942 * u * u);
+    double vr = pc[2] * env, vi = pc[3] * env;
     vr += __shfl_xor_sync(0xffffffffu, vr, 1);
     vi += __shfl_xor_sync(0xffffffffu, vi, 1);
-    if (lane < 4 && (lane & 1) == 0) dst[lane >> 1] = make_double2(vr, vi);
+    if (lane == 0) par.drive[kDrive][0] = par.drive[kDrive - 1][1];
+    __syncwarp();
+    if ((lane & 1) == 0) par.drive[j][(lane >> 1) & 1] = make_double2(vr, vi);
   };
-  // partial sums: [slot][value][warp]
-  auto put = [&](int slot, int v, double x) {
-    x = warp_sum(x);
-    if (lane == 0) par.red[slot][v][warp] = x;
-  };
-  auto get = [&](int slot, int v) {
-    double t = 0.0;
-#pragma unroll 1
-    for (int i = 0; i < L; ++i) t += par.red[slot][v][i];
-    return t;
-  };
-  if (scr) put(0, 0, nsum);
-  const double h = bt.dt;
-  double t = wp->t;
-  const int steps0 = wp->steps;
   __syncwarp();
-  if (mode != kLeapfrog && warp == 0) drive2(t, t, par.drive[1]);
+  if (MODE != kLeapfrog && warp == 0) {
+    // M(t) of the first step
+    if (lane == 0) {
+      double2 m = make_double2(0.0, 0.0);
+      for (int j = 0; j < 2; ++j) {
+        const double* pc = par.pulse[j];
+        const double u = (t - pc[0]) * pc[1];
+        const double env = exp(-4.0 * 0.69314718055994530942 * u * u);
+        m.x += pc[2] * env;
+        m.y += pc[3] * env;
+      }
+      par.drive[kDrive - 1][1] = m;
+    }
+    __syncwarp();
+  }
+  double ntot = 0.0;  // sum of n_e + n_h of the stage point, for its screening
+  int par_red = 0;    // parity of the partial sums: read one barrier after they are put
+  if (scr) {
+    double v[2] = {nsum, 0.0};
+    put_sums<2>(v, par.red[0], lane, warp);
+  }
   cta_sync<L>();
 
-  const int nst = (mode == kRhs || mode == kCalcH) ? 1 : bt.nsteps;
-  const int nstage = mode == kRk4 ? 4 : 1;
   for (int s = 0; s < nst; ++s) {
     double2 m_lf = make_double2(0.0, 0.0);
-    if (mode == kLeapfrog) {
+    if (MODE == kLeapfrog) {
       const int64_t fi = (int64_t)wi * bt.field_stride + 2 * ((int64_t)steps0 + s);
-      if (bt.field && fi >= 0 && fi + 1 < bt.n_field) {
+      if (bt.field && fi >= 0 && fi + 1 < bt.n_field)
         m_lf = make_double2(-par.hm * bt.field[fi], -par.hm * bt.field[fi + 1]);
-      }
-    } else if (mode == kRk4) {
-      // read by all after the next barrier; M(t) is the last step's M(t + h)
-      if (warp == 0) drive2(t + h / 2.0, t + h, par.drive[s & 1]);
+    } else if (s % kDrive == 0) {
+      // read by all after the next barrier
+      if (warp == 0) drive_ahead(t);
       if (!exc) cta_sync<L>();
     }
-    for (int st = 0; st < nstage; ++st) {
+    for (int st = 0; st < (MODE == kRk4 ? 4 : 1); ++st) {
       if (exc) {
         // the stage's tables: once per call, or screened by the stage point
         // (coulomb.py:1218-1230) every time
@@ -468,78 +551,111 @@ __device__ __forceinline__ void wire_steps(const Batch& bt, int mode, bool scr, 
         if (build) {
           double n1d = 0.0;
           if (scr) {
-            n1d = get(0, 0) / 2.0 / par.L;
+            if (MODE != kLeapfrog || s == 0) ntot = get_sum<L>(par.red[par_red], 0);
+            n1d = ntot * par.half_l;
             n1d = n1d < par.dens_max ? n1d : par.dens_max;
           }
-          for (int d = tid; d < np; d += T) {
-            const bool in = d > 0 && d < nk;
-            const double ie = in && scr ? 1.0 / eps1d(blk, nk, d, n1d) : 1.0;
+          double ie[kEpt];
+          bool far = false;
+          // eps(q; n1D) of Eps1D (coulomb.py:1185-1190)
+          auto eps = [&](int d, double le, double lh) {
+            return (1.0 - 2.0 * blk[5 * nk + d] * le) - 2.0 * blk[6 * nk + d] * lh;
+          };
+#pragma unroll
+          for (int e = 0; e < kEpt; ++e) {
+            const int d = min(tid + e * T, nk - 1);
+            ie[e] = 1.0;
+            if (scr) {
+              const double qe = blk[7 * nk + d], qh = blk[8 * nk + d];
+              const double le = log_ratio(qe - kPi * n1d, qe + n1d, far);
+              const double lh = log_ratio(qh - kPi * n1d, qh + n1d, far);
+              ie[e] = 1.0 / eps(d, le, lh);
+            }
+          }
+          if (far) {
+#pragma unroll 1
+            for (int e = 0; e < kEpt; ++e) {
+              const int d = min(tid + e * T, nk - 1);
+              const double qe = blk[7 * nk + d], qh = blk[8 * nk + d];
+              const double v = 1.0 / eps(d, log(fabs((qe - kPi * n1d) / (qe + n1d))),
+                                         log(fabs((qh - kPi * n1d) / (qh + n1d))));
+              if (e == 0) ie[0] = v;
+              else ie[kEpt - 1] = v;
+            }
+          }
+#pragma unroll
+          for (int e = 0; e < kEpt; ++e) {
+            const int d = tid + e * T;
             for (int n = 0; n < (one ? 1 : 3); ++n)
-              vq[n * np + d] = in ? blk[n * nk + d] * ie : 0.0;
+              vq[n * np + d] = d > 0 && d < nk ? blk[n * nk + d] * ie[e] : 0.0;
           }
           cta_sync<L>();
         }
-        // rounds: the tables' spectra (Veh and Vee, then Vhh), the stage point
-        for (int rnd = build ? (one ? 1 : 0) : 2; rnd < 3; ++rnd) {
-          if (rnd == 2 || sig == 0 || (rnd == 0 && !one)) {
+        // rounds: the tables' spectra, the stage point
+        for (int rnd = build ? 0 : 1; rnd < 2; ++rnd) {
+          if (rnd == 1 || sig == 0 || !one) {
             double2 x[8];
-            if (rnd == 2) {
+            if (rnd == 1) {
               const double2* src = (sig == 0 ? yp : yn) + col;
 #pragma unroll
               for (int r = 0; r < 8; ++r) x[r] = src[q * r];
             } else {
-              const double* src = vq + (rnd == 0 ? sig : (one ? 0 : 2)) * np + col;
+              // the even table c[d] = c[M - d] = V(d): the points a + q r and
+              // a + q (r + 8), added (even outputs) or subtracted
+              const double* v0 = vq + (sig == 0 ? 0 : np);
+              const double* v1 = vq + 2 * np;
+              const double sg = half ? -1.0 : 1.0;
 #pragma unroll
-              for (int r = 0; r < 8; ++r) x[r] = make_double2(src[q * r], 0.0);
+              for (int r = 0; r < 8; ++r) {
+                const int d = col + q * r, dm = np - d;  // M - (d + np); np: no such point
+                x[r] = make_double2(fma(sg, dm < np ? v0[dm] : 0.0, v0[d]), 0.0);
+                if (sig) x[r].y = fma(sg, dm < np ? v1[dm] : 0.0, v1[d]);
+              }
             }
             pass_a<q, rs>(x, ea, twa + col, half);
           }
           cta_sync<L>();
-          pass_b<L>(rnd < 2 ? kTables : (one ? kOneTable : kDistinct), E, S, twb,
-                       rnd == 0 || one ? 0 : 2, rnd == 0 ? 1 : -1, 1.0 / (bt.hbar * (16 * q)));
+          pass_b<L>(rnd == 0 ? kTables : (one ? kOneTable : kDistinct), one, E, S, twb,
+                    ih * (1.0 / (16 * q)));
           cta_sync<L>();
-          if (rnd == 1 && !one) {
-            // half the sum and half the difference of the Vee and Vhh spectra
-            for (int i = tid; i < Y::sl; i += T) {
-              const double e = S[Y::sl + i], hh = S[2 * Y::sl + i];
-              S[Y::sl + i] = 0.5 * (e + hh);
-              S[2 * Y::sl + i] = 0.5 * (e - hh);
-            }
-          }
         }
         pass_a_inv<q, rs>(ea, twa + col, half);
         cta_sync<L>();
       }
       // M(t), M(t + h/2) twice, M(t + h)
-      const double2 m = mode == kLeapfrog
-                            ? m_lf
-                            : (st == 0 ? par.drive[(s + 1) & 1][1]
-                                       : par.drive[s & 1][st == 3 ? 1 : 0]);
+      const int sd = s % kDrive;
+      const double2 m = MODE == kLeapfrog ? m_lf
+                        : st == 0         ? (sd == 0 ? par.drive[kDrive][0] : par.drive[sd - 1][1])
+                                          : par.drive[sd][st == 3 ? 1 : 0];
       const double gamma = par.gamma;
-      double v0 = 0.0, v1 = 0.0;
-      nsum = 0.0;
+      // sums over k: Re p, Im p, and n_e + n_h or n_e, n_h
+      double v[4] = {0.0, 0.0, 0.0, 0.0};
+      // (points beyond Nk go through the same arithmetic and stay zero)
 #pragma unroll
       for (int e = 0; e < kEpt; ++e) {
         const int k = tid + e * T;
-        if (k >= nk) continue;
+        const bool in = k < nk;
         double2 om = m;
         double xe = 0.0, xh = 0.0;
         if (exc) {
-          const double2* o = E + eo[e];
+          // k = a + q r: rows 2 r and 2 r + 1, column a
+          const double2* o = E + 2 * (k / q) * rs + k % q;
           const double2 p0 = o[0], p1 = o[rs], n0 = o[16 * rs], n1 = o[17 * rs];
           om.x += p0.x + p1.x;
           om.y += p0.y + p1.y;
           xe = n0.x + n1.x;
           xh = n0.y + n1.y;
         }
-        if (mode == kCalcH) {
+        if (ONCE && mode == kCalcH) {
           // renormalised H diagonals (CalcH, SBEs.py:819-935): Heh (Rabi
           // frequency), Hee, Hhh in the slots of dy
-          const double hb = bt.hbar;
-          double2* d2 = reinterpret_cast<double2*>(bt.dy + 4 * off);
-          d2[2 * k] = make_double2(om.x * hb, om.y * hb);
-          d2[2 * k + 1] = make_double2((blk[3 * nk + k] + par.gap) - xe * hb,
-                                       blk[4 * nk + k] - xh * hb);
+          if (in) {
+            const double hb = bt.hbar;
+            double2* d2 = reinterpret_cast<double2*>(bt.dy + 4 * off);
+            d2[2 * k] = make_double2(om.x * hb, om.y * hb);
+            d2[2 * k + 1] = make_double2((blk[3 * nk + k] + par.gap) - xe * hb,
+                                         blk[4 * nk + k] - xh * hb);
+          }
           continue;
         }
         // diagonal of dpdt, dCdt, dDdt (SBEs.py:1962-1975, 2325-2337,
@@ -549,88 +665,81 @@ __device__ __forceinline__ void wire_steps(const Batch& bt, int mode, bool scr, 
         const double f0 = sh * p.y - om.y * nn - gamma * p.x;
         const double f1 = om.x * nn - sh * p.x - gamma * p.y;
         const double f2 = 2.0 * (om.y * p.x - om.x * p.y);
-        if (mode == kRhs) {
-          double2* d2 = reinterpret_cast<double2*>(bt.dy + 4 * off);
-          d2[2 * k] = make_double2(f0, f1);
-          d2[2 * k + 1] = make_double2(f2, f2);
-        } else if (mode == kRk4) {
-          // stages of integrator.py:143-157; acc = k1 + 2 k2 + 2 k3
-          double g0 = f0, g1 = f1, g2 = f2;
-          const double c = st == 2 ? h : (st == 3 ? h / 6.0 : h / 2.0);
-          if (st == 0) {
-            acc[e][0] = f0;
-            acc[e][1] = f1;
-            acc[e][2] = f2;
-          } else if (st < 3) {
-            acc[e][0] += 2.0 * f0;
-            acc[e][1] += 2.0 * f1;
-            acc[e][2] += 2.0 * f2;
-          } else {
-            g0 += acc[e][0];
-            g1 += acc[e][1];
-            g2 += acc[e][2];
+        if (ONCE) {
+          if (in) {
+            double2* d2 = reinterpret_cast<double2*>(bt.dy + 4 * off);
+            d2[2 * k] = make_double2(f0, f1);
+            d2[2 * k + 1] = make_double2(f2, f2);
           }
-          const double2 zp = make_double2(yb[e][0] + c * g0, yb[e][1] + c * g1);
-          const double2 zn = make_double2(yb[e][2] + c * g2, yb[e][3] + c * g2);
-          yp[k] = zp;
-          yn[k] = zn;
-          if (st == 3) {
-            yb[e][0] = zp.x;
-            yb[e][1] = zp.y;
-            yb[e][2] = zn.x;
-            yb[e][3] = zn.y;
-            v0 += zp.x;
-            v1 += zp.y;
-          }
-          nsum += zn.x + zn.y;
+          continue;
+        }
+        double2 zp, zn;
+        if (MODE == kRk4) {
+          // stages of integrator.py:143-157; acc = k1 + 2 k2 + 2 k3, and at
+          // the last stage k1 + 2 k2 + 2 k3 + k4
+          const double w = st == 1 || st == 2 ? 2.0 : 1.0;
+          acc[e][0] = fma(w, f0, st == 0 ? 0.0 : acc[e][0]);
+          acc[e][1] = fma(w, f1, st == 0 ? 0.0 : acc[e][1]);
+          acc[e][2] = fma(w, f2, st == 0 ? 0.0 : acc[e][2]);
+          const double c = st == 2 ? h : (st == 3 ? h6 : h2);
+          const double g0 = st == 3 ? acc[e][0] : f0, g1 = st == 3 ? acc[e][1] : f1;
+          const double g2 = st == 3 ? acc[e][2] : f2;
+          zp = make_double2(fma(c, g0, yb[e][0]), fma(c, g1, yb[e][1]));
+          zn = make_double2(fma(c, g2, yb[e][2]), fma(c, g2, yb[e][3]));
         } else {
-          // leapfrog X3 = X1 + 2 dt f(X2) (SBEs.py:5685-5687), in the place of
-          // X2 (this thread's own points; all sums over X2 are done), and the
+          // leapfrog X3 = X1 + 2 dt f(X2) (SBEs.py:5685-5687) and the
           // occupations |n| for the rescale (SBEs.py:5704-5711)
-          yp[k] = make_double2(yb[e][0] + f0 * h * 2.0, yb[e][1] + f1 * h * 2.0);
-          const double2 n3 = make_double2(fabs(yb[e][2] + f2 * h * 2.0),
-                                          fabs(yb[e][3] + f2 * h * 2.0));
-          yn[k] = n3;
-          v0 += n3.x;
-          v1 += n3.y;
+          zp = make_double2(yb[e][0] + f0 * h * 2.0, yb[e][1] + f1 * h * 2.0);
+          zn = make_double2(fabs(yb[e][2] + f2 * h * 2.0), fabs(yb[e][3] + f2 * h * 2.0));
         }
+        if (!in) zp = zn = make_double2(0.0, 0.0);
+        yp[k] = zp;
+        yn[k] = zn;
+        if (MODE == kRk4 && st == 3) {
+          yb[e][0] = zp.x;
+          yb[e][1] = zp.y;
+          yb[e][2] = zn.x;
+          yb[e][3] = zn.y;
+        }
+        v[0] += zp.x;
+        v[1] += zp.y;
+        v[2] += MODE == kRk4 ? zn.x + zn.y : zn.x;
+        v[3] += zn.y;
       }
-      if (mode == kRhs || mode == kCalcH) return;
-      if (mode == kRk4) {
-        if (scr) put(0, 0, nsum);
+      if (ONCE) return;
+      par_red ^= 1;
+      if (MODE == kRk4) {
+        // sums: n1D for the next stage's screening, P(t) after the last stage
         if (st == 3) {
-          put(1, 0, v0);
-          put(1, 1, v1);
+          double u[4] = {v[2], v[0], v[1], 0.0};
+          put_sums<4>(u, par.red[par_red], lane, warp);
+        } else if (scr) {
+          double u[2] = {v[2], 0.0};
+          put_sums<2>(u, par.red[par_red], lane, warp);
         }
-      } else {
-        put(2, 0, v0);
-        put(2, 1, v1);
         cta_sync<L>();
-        const double te = get(2, 0), th = get(2, 1);
+      } else {
+        double u[4] = {v[2], v[0], v[1], v[3]};
+        put_sums<4>(u, par.red[par_red], lane, warp);
+        cta_sync<L>();
+        const double te = get_sum<L>(par.red[par_red], 0), th = get_sum<L>(par.red[par_red], 3);
         const double total = (te + th) / 2.0, small = 1e-200;
         const double ce = total / (te + small), ch = total / (th + small);
-        v0 = v1 = 0.0;
 #pragma unroll
         for (int e = 0; e < kEpt; ++e) {
           const int k = tid + e * T;
-          if (k >= nk) continue;
-          const double2 x3 = yp[k];
-          double2 n3 = yn[k];
-          n3 = make_double2(n3.x * ce, n3.y * ch);
-          yn[k] = n3;
-          yb[e][0] = (yb[e][0] + x3.x) / 2.0;
-          yb[e][1] = (yb[e][1] + x3.y) / 2.0;
-          yb[e][2] = (yb[e][2] + n3.x) / 2.0;
-          yb[e][3] = (yb[e][3] + n3.y) / 2.0;
-          nsum += n3.x + n3.y;
-          v0 += x3.x;
-          v1 += x3.y;
+          const double2 zp = yp[k];
+          double2 zn = yn[k];
+          zn = make_double2(zn.x * ce, zn.y * ch);
+          yn[k] = zn;
+          yb[e][0] = (yb[e][0] + zp.x) / 2.0;
+          yb[e][1] = (yb[e][1] + zp.y) / 2.0;
+          yb[e][2] = (yb[e][2] + zn.x) / 2.0;
+          yb[e][3] = (yb[e][3] + zn.y) / 2.0;
         }
-        if (scr) put(0, 0, nsum);
-        put(1, 0, v0);
-        put(1, 1, v1);
+        ntot = te * ce + th * ch;
+        cta_sync<L>();
       }
-      cta_sync<L>();
     }
     t = t + h;
     // P(t) record (qwoptics.py:815-946, diagonal: pscale * sum_k p_k)
@@ -638,12 +747,12 @@ __device__ __forceinline__ void wire_steps(const Batch& bt, int mode, bool scr, 
       const int r = (s + 1) / bt.p_stride - 1;
       const int64_t po = par.p_off;
       if (r < bt.p_cap && po >= 0 && po + r < bt.n_P) {
-        const double ps = par.pscale;
-        bt.P[2 * (po + r)] = ps * get(1, 0);
-        bt.P[2 * (po + r) + 1] = ps * get(1, 1);
+        bt.P[2 * (po + r)] = par.pscale * get_sum<L>(par.red[par_red], 1);
+        bt.P[2 * (po + r) + 1] = par.pscale * get_sum<L>(par.red[par_red], 2);
       }
     }
   }
+  if (ONCE) return;
 
   // Write the state back; flag non-finite wires.
   bool bad = false;
@@ -657,26 +766,25 @@ __device__ __forceinline__ void wire_steps(const Batch& bt, int mode, bool scr, 
     yo[2 * k] = a;
     yo[2 * k + 1] = b;
     bad |= !(isfinite(a.x) && isfinite(a.y) && isfinite(b.x) && isfinite(b.y));
-    if (mode == kLeapfrog) {
+    if (MODE == kLeapfrog) {
       y1o[2 * k] = make_double2(yb[e][0], yb[e][1]);
       y1o[2 * k + 1] = make_double2(yb[e][2], yb[e][3]);
       bad |= !(isfinite(yb[e][0]) && isfinite(yb[e][1]) && isfinite(yb[e][2]) &&
                isfinite(yb[e][3]));
     }
   }
-  put(2, 2, bad ? 1.0 : 0.0);
-  cta_sync<L>();
+  bad = L == 1 ? __any_sync(0xffffffffu, bad) : (bool)__syncthreads_or(bad);
   if (tid == 0) {
     wp->t = t;
     wp->steps = steps0 + nst;
-    if (get(2, 2) != 0.0 && wp->status == PSB_OK) wp->status = PSB_ERR_NONFINITE;
+    if (bad && wp->status == PSB_OK) wp->status = PSB_ERR_NONFINITE;
   }
 }
 
 // A launch covers the wires of its grid whose own Nk takes L lanes; the others
 // are another launch's, unless the caller said that there are none (strict).
 // check: this launch reports bad descriptors.
-template <int L>
+template <int L, int MODE>
 __global__ void __launch_bounds__(32 * L, ctas_of(L))
     sbe_conv_kernel(Batch bt, int mode, bool screened, bool shared, bool check, bool strict) {
   extern __shared__ __align__(16) uint8_t smem[];
@@ -701,7 +809,7 @@ __global__ void __launch_bounds__(32 * L, ctas_of(L))
     if (check && threadIdx.x == 0) wp->status = bad;
     return;
   }
-  if (lanes_of(tb.nk) == L) wire_steps<L>(bt, mode, screened, smem, wi, tb);
+  if (lanes_of(tb.nk) == L) wire_steps<L, MODE>(bt, mode, screened, smem, wi, tb);
 }
 
 template <int L>
@@ -709,32 +817,33 @@ uint32_t smem_of(bool shared) {
   return shared ? Lay<L>::total1 : Lay<L>::total3;
 }
 
-template <int L>
+template <int L, int MODE>
 int launch_lanes(const Batch& bt, int mode, int grid, bool screened, bool shared, bool check,
                  bool strict, cudaStream_t st) {
   const uint32_t smem = smem_of<L>(shared);
   if (smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(
-        sbe_conv_kernel<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        sbe_conv_kernel<L, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess)
       return set_error(PSB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
   }
-  sbe_conv_kernel<L><<<grid, 32 * L, smem, st>>>(bt, mode, screened, shared, check, strict);
+  sbe_conv_kernel<L, MODE><<<grid, 32 * L, smem, st>>>(bt, mode, screened, shared, check, strict);
   return check_cuda("sbe_conv_kernel");
 }
 
-// One launch per width from that of nkmax down to that of nkmin + 1.
-template <int L>
+// One launch per width from that of nkmax down to that of nkmin + 1 (a single
+// right-hand side: of the widths above the direct kernel's only).
+template <int L, int MODE>
 int launch_down(const Batch& bt, int mode, int grid, int nkmax, int nkmin, bool screened,
                 bool shared, bool one_class, cudaStream_t st) {
   const int top = lanes_of(nkmax);
   if (L <= top && L >= lanes_of(nkmin + 1)) {
     const int rc =
-        launch_lanes<L>(bt, mode, grid, screened, shared, L == top, one_class, st);
+        launch_lanes<L, MODE>(bt, mode, grid, screened, shared, L == top, one_class, st);
     if (rc != PSB_OK || one_class) return rc;
   }
-  if constexpr (L > 1)
-    return launch_down<L / 2>(bt, mode, grid, nkmax, nkmin, screened, shared, one_class, st);
+  if constexpr (L > (MODE == kRhs ? lanes_of(kDirectNk + 1) : 1))
+    return launch_down<L / 2, MODE>(bt, mode, grid, nkmax, nkmin, screened, shared, one_class, st);
   return PSB_OK;
 }
 
@@ -752,7 +861,14 @@ size_t conv_smem_bytes(int nk, bool shared) {
 
 int launch_sbe_conv(const Batch& bt, int mode, int grid, int nkmax, int nkmin, bool screened,
                     bool shared, bool one_class, cudaStream_t st) {
-  return conv::launch_down<16>(bt, mode, grid, nkmax, nkmin, screened, shared, one_class, st);
+  if (mode == kRk4)
+    return conv::launch_down<16, kRk4>(bt, mode, grid, nkmax, nkmin, screened, shared, one_class,
+                                       st);
+  if (mode == kLeapfrog)
+    return conv::launch_down<16, kLeapfrog>(bt, mode, grid, nkmax, nkmin, screened, shared,
+                                            one_class, st);
+  return conv::launch_down<16, kRhs>(bt, mode, grid, nkmax, nkmin, screened, shared, one_class,
+                                     st);
 }
 
 }  // namespace psb

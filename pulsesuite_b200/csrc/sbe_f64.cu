@@ -30,10 +30,7 @@ namespace psb {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-// Largest grid of the direct kernel: one point of k per thread.  Measured on
-// B200, one right-hand side, direct / transforms (us): Nk 256, 16 wires 15.7 /
-// 16.5, 2048 wires 68 / 35; Nk 512, 16 wires 20.6 / 17.6, 2048 wires 215 / 69.
-constexpr int kDirectNk = kThreads;
+static_assert(kDirectNk <= kThreads, "one point of k per thread");
 
 struct Geo {
   int nk, nkp, nb, kc, chunk, yslen, doff, vlen, vphys;
@@ -260,8 +257,11 @@ __device__ __forceinline__ void rhs_element(const Geo& g, int k, const double* y
   f[3] = dn;
 }
 
-template <int R, int MODE, bool SCREEN, int NT>
-__global__ void __launch_bounds__(kThreads, 2) sbe_f64_kernel(Batch bt, bool check) {
+// CTAS per SM: 4 of 64 registers for grids up to 128 points, whose threads have
+// little work between the barriers (2048 wires, Nk 64 / 128: 24.7 / 33.1 us
+// against 30.8 / 39.0 with 2), 2 of 128 above (Nk 256: 68.9 against 71.9 with 4).
+template <int R, int MODE, bool SCREEN, int NT, int CTAS>
+__global__ void __launch_bounds__(kThreads, CTAS) sbe_f64_kernel(Batch bt, bool check) {
   extern __shared__ double smem[];
   const int wi = bt.order ? bt.order[blockIdx.x] : (int)blockIdx.x;
   if (wi < 0 || wi >= bt.nw) return;
@@ -362,11 +362,15 @@ static int launch_direct(const Batch& bt, int grid, int nkmax, bool check, cudaS
     const size_t b = smem_bytes_for(nk, NT);
     if (b > smem) smem = b;
   }
-  const cudaError_t e = cudaFuncSetAttribute(
-      sbe_f64_kernel<kR, MODE, SCREEN, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess)
-    return set_error(PSB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-  sbe_f64_kernel<kR, MODE, SCREEN, NT><<<grid, kThreads, smem, st>>>(bt, check);
+  auto kern = nkmax <= 128 ? sbe_f64_kernel<kR, MODE, SCREEN, NT, 4>
+                           : sbe_f64_kernel<kR, MODE, SCREEN, NT, 2>;
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(
+        kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess)
+      return set_error(PSB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  }
+  kern<<<grid, kThreads, smem, st>>>(bt, check);
   return check_cuda("sbe_f64_kernel");
 }
 

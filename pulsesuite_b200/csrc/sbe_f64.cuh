@@ -8,6 +8,13 @@ namespace psb {
 
 enum Mode { kRhs = 0, kRk4 = 1, kLeapfrog = 2, kCalcH = 3 };
 
+// Largest grid whose single right-hand side the direct kernel takes (one point
+// of k per thread).  Measured on B200, one call of WireBatch.rhs, direct / by
+// transforms (us): Nk 256, 16 wires 15 / 18, 2048 wires 69 / 40; Nk 512, 16
+// wires 21 / 18, 2048 wires 215 / 72.  The line lies where few wires, whose
+// call is launches and latency, break even.
+constexpr int kDirectNk = 256;
+
 struct Batch {
   const PsbTable* tables;
   int ntab;
