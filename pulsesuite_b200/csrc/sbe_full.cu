@@ -27,6 +27,7 @@
 // in the last bits).
 #include <mutex>
 
+#include "dmma.cuh"
 #include "psb_common.cuh"
 
 namespace psb {
@@ -59,20 +60,18 @@ struct Step {
   double2* L1;          // levels, [3][nk][nk] each: p, C, D
   double2* L2;
   double2* L3;
-  double2* Meh;         // work [nk][nk]
+  double* fac;          // work [3]: the occupations' common total, their sums
   double2* H;           // work [3][nk][nk]: Heh, Hee, Hhh
-  double2* dX;          // work [3][nk][nk]: dp, dC, dD
-  // many-body terms (null when off): k-dependent dephasing rates, the
-  // off-diagonal dephasing term of dpdt, and X3 written out so that the
-  // relaxation can change its occupations before the neutrality rescale
+  double2* X3;          // work or many-body scratch [3][nk][nk]: X1 + 2 dt dX
+  // many-body terms (null when off): k-dependent dephasing rates and the
+  // off-diagonal dephasing term of dpdt
   const double* GamE;   // [nk]
   const double* GamH;   // [nk]
   const double2* OffP;  // [nk][nk], OffP[kh][ke]
-  const double2* X3;    // [3][nk][nk]
   // a batch of wires of one grid, wire = blockIdx.y: byte strides between
   // the wires' V3, fields, levels, work and many-body scratch, and the
   // per-wire [nw][4] = yw, (-1)^w, dc_dk, 0 (null: prm.yw, prm.sgnw)
-  int64_t st_v3, st_e, st_lv, st_wk, st_sc;
+  int64_t st_v3, st_e, st_lv, st_wk, st_sc, st_x3;
   const double* wpar;
 };
 
@@ -89,13 +88,12 @@ __device__ __forceinline__ Step at_wire(Step s) {
   s.L1 = bump(s.L1, w * s.st_lv);
   s.L2 = bump(s.L2, w * s.st_lv);
   s.L3 = bump(s.L3, w * s.st_lv);
-  s.Meh = bump(s.Meh, w * s.st_wk);
+  s.fac = bump(s.fac, w * s.st_wk);
   s.H = bump(s.H, w * s.st_wk);
-  s.dX = bump(s.dX, w * s.st_wk);
   s.GamE = bump(s.GamE, w * s.st_sc);
   s.GamH = bump(s.GamH, w * s.st_sc);
   s.OffP = bump(s.OffP, w * s.st_sc);
-  s.X3 = bump(s.X3, w * s.st_sc);
+  s.X3 = bump(s.X3, w * s.st_x3);
   if (s.wpar) {
     s.prm.yw = s.wpar[4 * w];
     s.prm.sgnw = s.wpar[4 * w + 1];
@@ -103,248 +101,341 @@ __device__ __forceinline__ Step at_wire(Step s) {
   return s;
 }
 
-// Meh[ke][kh] = -ehint (Xcv Ex[q] + Ycv Ey[q] yw + Zcv Ez[q] (-1)^w),
-// q = kkp[ke][kh] = ke - kh + NQ0, Xcv = dcv (-1)^(kh+1), Ycv = dcv,
-// Zcv = -dcv (QWOptics dipoles, qwoptics.py:619-623).
-__global__ void meh_kernel(Step s0) {
+// CalcMeh (SBEs.py:5165-5175) and CalcH (SBEs.py:819-935).  Every element
+// (k1, k2) sums along its diagonal d = k1 - k2 of p, C, D (the exchange terms)
+// and, with LF, the whole diagonals d and -d of C and D (the direct terms,
+// the same for all its elements).  The coupling
+//   Meh[ke][kh] = -ehint (Xcv Ex[q] + Ycv Ey[q] yw + Zcv Ez[q] (-1)^w),
+// q = ke - kh + NQ0, Xcv = dcv (-1)^(kh+1), Ycv = dcv, Zcv = -dcv (QWOptics
+// dipoles, qwoptics.py:619-623) has one set of fields per diagonal too.
+//
+// One warp per diagonal and wire, neighbouring diagonals in a CTA (their
+// strided elements share cache lines).  The runs of p, C and D lie in shared
+// memory; lane b sums R = 4 neighbouring elements with the last 4 values of
+// each table in registers, so a step over the run costs one new value per
+// table and one broadcast per matrix for 24 FMAs.  The tables are stored with
+// one pad every 4 values, which spreads the lanes' stride of 4 over the banks.
+// 64 wires of Nk 114: 0.10 ms, bound by the strided reads and writes of the
+// diagonals; 0.24 with a CTA per diagonal and one element per thread.
+constexpr int kHDiags = 8, kHR = 4;  // diagonals per CTA at most (fewer when memory is short)
+__host__ __device__ inline int h_skew(int i) { return i + i / kHR; }
+// doubles of one table, positions u - t in [-(nk + 3), nk + 3], and of a run
+__host__ __device__ inline int h_vlen(int nk) { return h_skew(2 * (nk + kHR)) + 1; }
+inline size_t h_smem(int nk, int diags) {
+  const int nr = (nk + kHR - 1) / kHR * kHR;
+  return 3 * (size_t)((h_vlen(nk) + 1) / 2 * 2) * 8 + diags * 3 * (size_t)nr * 16;
+}
+
+__device__ __forceinline__ double2 warp_sum2(double2 v) {
+  return make_double2(warp_sum(v.x), warp_sum(v.y));
+}
+
+__global__ void __launch_bounds__(32 * kHDiags) calch_kernel(Step s0) {
   const Step s = at_wire(s0);
-  const int nk = s.nk;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nk * nk) return;
-  const int ke = e / nk, kh = e - ke * nk;
-  const int q = ke - kh + s.nq0;
-  double2 ex = make_double2(0.0, 0.0), ey = ex, ez = ex;
-  if (q >= 0 && q < s.nr) {
-    ex = s.E[q];
-    ey = s.E[s.nr + q];
-    ez = s.E[2 * s.nr + q];
+  const int nk = s.nk, n2 = nk * nk, lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  extern __shared__ __align__(16) double hsm[];
+  const int vlen = (h_vlen(nk) + 1) / 2 * 2, vo = nk + kHR;  // table t at t vlen, q = 0 at vo
+  const int nr = (nk + kHR - 1) / kHR * kHR;
+  double2* run = reinterpret_cast<double2*>(hsm + 3 * vlen) + wp * 3 * nr;
+  for (int i = threadIdx.x; i < 2 * vo; i += blockDim.x) {
+    const int q = i < vo ? vo - i : i - vo;
+#pragma unroll
+    for (int t = 0; t < 3; ++t)
+      hsm[t * vlen + h_skew(i)] = q > 0 && q < nk ? s.V3[t * nk + q] : 0.0;
   }
-  const double dcv = s.prm.dcv, eh = s.prm.ehint;
-  const double xcv = ((kh + 1) & 1) ? -dcv : dcv;
-  double2 m = rs(-eh * xcv, ex);
-  m = cs(m, rs(s.prm.yw, rs(eh * dcv, ey)));
-  m = cs(m, rs(s.prm.sgnw, rs(eh * -dcv, ez)));
-  s.Meh[e] = m;
-}
-
-__device__ __forceinline__ double vq(const double* V, int n, int nk, int q) {
-  const int a = q < 0 ? -q : q;
-  return (a > 0 && a < nk) ? V[n * nk + a] : 0.0;
-}
-
-// CalcH (SBEs.py:819-935): every element (k1, k2) sums along its diagonal
-// d = k1 - k2 of p, C, D (the exchange terms) and, with LF, along the
-// diagonals d and -d of C and D (the direct terms), each in the reference's
-// order.  One CTA per diagonal and wire: the five diagonals it reads are
-// loaded once into shared memory (they are strided in the row-major
-// matrices), then thread t sums for the element at position t.
-constexpr int kHThreads = 128;
-__global__ void __launch_bounds__(kHThreads) calch_kernel(Step s0) {
-  const Step s = at_wire(s0);
-  const int nk = s.nk, n2 = nk * nk;
-  const int d = (int)blockIdx.x - (nk - 1);     // k1 - k2
-  const int ad = d < 0 ? -d : d, len = nk - ad;  // elements on the diagonal
+  const int d = (int)(blockIdx.x * blockDim.x + threadIdx.x) / 32 - (nk - 1);  // k1 - k2
+  const bool mine = d < nk;
+  const int ad = d < 0 ? -d : d, len = mine ? nk - ad : 0;
   const int o1 = d > 0 ? d : 0, o2 = d < 0 ? -d : 0;  // k1 = t + o1, k2 = t + o2
-  extern __shared__ double2 hsm[];  // [5][len]: p, C, D at row - col = -d; C, D at +d
-  double2* pd = hsm;
-  double2* cd = pd + len;
-  double2* dd = cd + len;
-  double2* cm_ = dd + len;
-  double2* dm = cm_ + len;
-  const double2* p = s.L3;
-  const double2* C = s.L3 + n2;
-  const double2* D = s.L3 + 2 * n2;
-  for (int u = threadIdx.x; u < len; u += kHThreads) {
-    // element u of the run: row o2 + u, column o1 + u (col - row = d), and
-    // the mirrored run row o1 + u, column o2 + u
-    const int a = (o2 + u) * nk + (o1 + u), b = (o1 + u) * nk + (o2 + u);
-    pd[u] = p[a];
-    cd[u] = C[a];
-    dd[u] = D[a];
-    cm_[u] = C[b];
-    dm[u] = D[b];
-  }
-  __syncthreads();
-  const double* V = s.V3;
-  for (int t = threadIdx.x; t < len; t += kHThreads) {
-    const int k1 = t + o1, k2 = t + o2, e = k1 * nk + k2;
-    double2 heh = s.Meh[e];
-    double2 hee = make_double2(0.0, 0.0), hhh = hee;
-    if (k1 == k2) {
-      hee = make_double2(s.Ee[k1] + s.prm.gap, 0.0);
-      hhh = make_double2(s.Eh[k1], 0.0);
-    }
-    if (s.prm.excitons) {
-      // q runs over qmin .. qmax, i.e. positions u = t + q = 0 .. len - 1
-      // H^eh: sum_q V_eh(q) p^T[k1+q][k2+q] = p[k2+q][k1+q]
-      for (int u = 0; u < len; ++u)
-        if (u != t) heh = ca(heh, rs(vq(V, 0, nk, u - t), pd[u]));
-      if (s.prm.lf) {
-        for (int u = 0; u < len; ++u)
-          if (u != t) hee = cs(hee, rs(vq(V, 1, nk, u - t), cd[u]));
-        if (d != 0) {
-          // direct terms: k = kmin .. kmax, C[k][k + d] and D[k + d][k]
-          const double v1 = vq(V, 1, nk, d), v0 = vq(V, 0, nk, d), v2 = vq(V, 2, nk, d);
-          // with k = kmin + u: C[k][k + d] = cd[u], D[k + d][k] = dm[u],
-          // D[k][k + d] = dd[u], C[k + d][k] = cm_[u]
-          for (int u = 0; u < len; ++u) hee = ca(hee, cs(rs(v1, cd[u]), rs(v0, dm[u])));
-          for (int u = 0; u < len; ++u)
-            if (u != t) hhh = cs(hhh, rs(vq(V, 2, nk, u - t), dd[u]));
-          for (int u = 0; u < len; ++u) hhh = ca(hhh, cs(rs(v2, dd[u]), rs(v0, cm_[u])));
-        } else {
-          for (int u = 0; u < len; ++u)
-            if (u != t) hhh = cs(hhh, rs(vq(V, 2, nk, u - t), dd[u]));
-        }
-      } else if (k1 == k2) {
-        for (int u = 0; u < len; ++u)
-          if (u != t) hee = cs(hee, rs(vq(V, 1, nk, u - t), cd[u]));
-        for (int u = 0; u < len; ++u)
-          if (u != t) hhh = cs(hhh, rs(vq(V, 2, nk, u - t), dd[u]));
+  const double2* M[3] = {s.L3, s.L3 + n2, s.L3 + 2 * n2};
+  const double2 z = make_double2(0.0, 0.0);
+  double2 dir1 = z, dir2 = z;  // the direct terms of Hee and Hhh
+  const bool exc = s.prm.excitons != 0, lf = s.prm.lf != 0;
+  if (exc) {
+    // element u of the run: row o2 + u, column o1 + u; mirrored: (o1 + u, o2 + u)
+    double2 sc = z, sd = z, mc = z, md = z;
+    for (int u = lane; u < nr; u += 32) {
+      const bool in = u < len;
+      const int a = (o2 + u) * nk + o1 + u, b = (o1 + u) * nk + o2 + u;
+      const double2 pv = in ? M[0][a] : z, cv = in ? M[1][a] : z, dv = in ? M[2][a] : z;
+      run[u] = pv;
+      run[nr + u] = cv;
+      run[2 * nr + u] = dv;
+      if (lf && d != 0 && in) {
+        sc = ca(sc, cv);
+        sd = ca(sd, dv);
+        mc = ca(mc, M[1][b]);
+        md = ca(md, M[2][b]);
       }
     }
-    s.H[e] = heh;
-    s.H[n2 + e] = hee;
-    s.H[2 * n2 + e] = hhh;
+    if (lf && d != 0 && mine) {
+      // Vee(d) sum C[k][k + d] - Veh(d) sum D[k + d][k], and Vhh(d), D, C
+      const double v0 = s.V3[ad], v1 = s.V3[nk + ad], v2 = s.V3[2 * nk + ad];
+      dir1 = cs(rs(v1, warp_sum2(sc)), rs(v0, warp_sum2(md)));
+      dir2 = cs(rs(v2, warp_sum2(sd)), rs(v0, warp_sum2(mc)));
+    }
+  }
+  __syncthreads();
+  if (!mine) return;
+  const int q = d + s.nq0;
+  const bool inq = q >= 0 && q < s.nr;
+  const double dcv = s.prm.dcv, eh = s.prm.ehint;
+  const double2 ex = inq ? s.E[q] : z, ey = inq ? s.E[s.nr + q] : z,
+                ez = inq ? s.E[2 * s.nr + q] : z;
+  // sums of Hee and Hhh: everywhere with LF, else on the diagonal only
+  const bool occ = exc && (lf || d == 0);
+  for (int t0 = kHR * lane; t0 < len; t0 += kHR * 32) {
+    double2 h0[kHR], h1[kHR], h2[kHR];
+    double w0[kHR], w1[kHR], w2[kHR];
+#pragma unroll
+    for (int r = 0; r < kHR; ++r) {
+      h0[r] = h1[r] = h2[r] = z;
+      const int i = h_skew(vo - t0 - r);  // u = 0
+      w0[r] = hsm[i];
+      w1[r] = hsm[vlen + i];
+      w2[r] = hsm[2 * vlen + i];
+    }
+    if (exc) {
+      // (the runs are zero from len to a multiple of kHR)
+      for (int u0 = 0; u0 < len; u0 += kHR) {
+#pragma unroll
+        for (int uu = 0; uu < kHR; ++uu) {
+          const double2 pv = run[u0 + uu];
+#pragma unroll
+          for (int r = 0; r < kHR; ++r) {
+            h0[r].x = fma(w0[r], pv.x, h0[r].x);
+            h0[r].y = fma(w0[r], pv.y, h0[r].y);
+          }
+          if (occ) {
+            const double2 cv = run[nr + u0 + uu], dv = run[2 * nr + u0 + uu];
+#pragma unroll
+            for (int r = 0; r < kHR; ++r) {
+              h1[r].x = fma(w1[r], cv.x, h1[r].x);
+              h1[r].y = fma(w1[r], cv.y, h1[r].y);
+              h2[r].x = fma(w2[r], dv.x, h2[r].x);
+              h2[r].y = fma(w2[r], dv.y, h2[r].y);
+            }
+          }
+          // position u + 1: r takes r - 1's value, r = 0 the new one
+#pragma unroll
+          for (int r = kHR - 1; r > 0; --r) {
+            w0[r] = w0[r - 1];
+            w1[r] = w1[r - 1];
+            w2[r] = w2[r - 1];
+          }
+          const int i = h_skew(vo - t0 + u0 + uu + 1);
+          w0[0] = hsm[i];
+          w1[0] = hsm[vlen + i];
+          w2[0] = hsm[2 * vlen + i];
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < kHR; ++r) {
+      const int t = t0 + r;
+      if (t >= len) break;
+      const int k1 = t + o1, k2 = t + o2, e = k1 * nk + k2;
+      const double xcv = ((k2 + 1) & 1) ? -dcv : dcv;
+      double2 m = rs(-eh * xcv, ex);
+      m = cs(m, rs(s.prm.yw, rs(eh * dcv, ey)));
+      m = cs(m, rs(s.prm.sgnw, rs(eh * -dcv, ez)));
+      double2 hee = cs(dir1, h1[r]), hhh = cs(dir2, h2[r]);
+      if (d == 0) {
+        hee.x += s.Ee[k1] + s.prm.gap;
+        hhh.x += s.Eh[k1];
+      }
+      s.H[e] = ca(m, h0[r]);
+      s.H[n2 + e] = hee;
+      s.H[2 * n2 + e] = hhh;
+    }
   }
 }
 
-// dpdt / dCdt / dDdt (SBEs.py:1952-1975, 2318-2337, 2617-2636): one thread
-// per (i, j), the four dot products of each in the reference's order (each
-// accumulator runs over k = 0 .. nk-1 in sequence).  One CTA computes a
-// kDT x kDT block of elements: per chunk of kDT values of k, the 18 operand
-// tiles the block's 12 dot products read are staged in shared memory
-// (rows padded by one element against bank conflicts).
-constexpr int kDT = 16, kDTP = kDT + 1;
-enum DTile {  // tile [row block][col block]; I, J the element block, K the k chunk
-  T_HHH_IK, T_HHH_JK, T_HHH_KI, T_HEE_JK, T_HEE_KI, T_HEH_KI, T_HEH_JK, T_HEH_IK, T_HEH_KJ,
-  T_P_KJ, T_P_IK, T_P_KI, T_P_JK, T_C_KJ, T_C_IK, T_D_KI, T_D_IK, T_D_KJ, T_NUM
+// dpdt / dCdt / dDdt (SBEs.py:1952-1975, 2318-2337, 2617-2636) and X3 = X1 +
+// 2 dt dX (SBEs.py:5685-5687): twelve complex matrix products of nk x nk,
+//   i hbar dp = Hhh p + p Hee^T - Heh^T C - D^T Heh^T + Heh^T - i hbar G p + Off
+//   i hbar dC = C Hee^T - Hee^T C + p^H Heh^T - conj(Heh) p
+//   i hbar dD = D Hhh^T - Hhh^T D + conj(p) Heh - Heh^H p^T
+// on the FP64 matrix instructions.  One CTA computes a TM x TM block of all
+// three; per 4 values of the summation index k the 18 operand tiles its
+// products read come to shared memory by asynchronous copies, kDStages ahead.
+// A warp owns MT x 1 tiles of 8 x 8: 48 MT matrix instructions against 8 + 10
+// MT fragment loads per step.  Tiles [row][k] have rows of 4 and tiles
+// [k][column] rows of TM + 2 elements of 16 bytes: no bank conflicts.  An
+// element's sums run over k in steps of 4 whatever the block size, so its
+// bits do not depend on it.  Bound by the FP64 pipe (96 Nk^3 flops per wire,
+// 120 of 114 rows and columns computed at Nk 114): 64 wires of Nk 114 take 0.34
+// ms, 0.94 with scalar FMAs from 16 x 16 tiles in shared memory.
+constexpr int kDStages = 3;
+enum DTile {  // [row block][k]: rows of I or J; [k][column block]
+  T_HHH_IK, T_P_IK, T_C_IK, T_HEH_IK, T_D_IK, T_HEE_JK, T_HEH_JK, T_HHH_JK, T_P_JK,
+  T_HEH_KI, T_D_KI, T_HEE_KI, T_P_KI, T_HHH_KI, T_P_KJ, T_C_KJ, T_D_KJ, T_HEH_KJ, T_NUM,
+  T_ROWS = T_HEH_KI
 };
-constexpr size_t kDerivsSmem = (size_t)T_NUM * kDT * kDTP * sizeof(double2);
+// elements of a stage: T_ROWS tiles of 4 TM, the others of 4 (TM + 2)
+template <int TM>
+constexpr int kDStage = T_ROWS * 4 * TM + (T_NUM - T_ROWS) * 4 * (TM + 2);
 
-__global__ void __launch_bounds__(kDT* kDT) derivs_kernel(Step s0) {
+template <int TM>
+__global__ void __launch_bounds__(TM * 8, TM == 32 ? 2 : 4) derivs_kernel(Step s0) {
   const Step s = at_wire(s0);
-  const int nk = s.nk, n2 = nk * nk;
-  extern __shared__ double2 dsm[];
-  const int tx = threadIdx.x % kDT, ty = threadIdx.x / kDT;
-  const int I0 = blockIdx.x * kDT, J0 = blockIdx.z * kDT;
-  const int i = I0 + ty, j = J0 + tx;
+  constexpr int MT = TM / 16, NT = TM * 8;  // 8 x 8 tiles per warp, threads
+  const int nk = s.nk, n2 = nk * nk, tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+  extern __shared__ __align__(16) double2 dsm[];
+  const int I0 = blockIdx.x * TM, J0 = blockIdx.z * TM;
   const double2* p = s.L3;
   const double2* C = s.L3 + n2;
   const double2* D = s.L3 + 2 * n2;
   const double2* Heh = s.H;
   const double2* Hee = s.H + n2;
   const double2* Hhh = s.H + 2 * n2;
-  const double2 z = make_double2(0.0, 0.0);
-  auto tile = [&](int t, int r, int c) -> double2& { return dsm[(t * kDT + r) * kDTP + c]; };
-  // tile t of matrix M: rows from block R0 (or the k chunk), columns likewise
-  auto load = [&](int t, const double2* M, int R0, int C0) {
-    const int r = R0 + ty, c = C0 + tx;
-    tile(t, ty, tx) = (r < nk && c < nk) ? M[r * nk + c] : z;
-  };
-  double2 a1 = z, a2 = z, a3 = z, a4 = z;  // dp
-  double2 b1 = z, b2 = z, b3 = z, b4 = z;  // dC
-  double2 c1 = z, c2 = z, c3 = z, c4 = z;  // dD
-  for (int k0 = 0; k0 < nk; k0 += kDT) {
-    load(T_HHH_IK, Hhh, I0, k0);
-    load(T_HHH_JK, Hhh, J0, k0);
-    load(T_HHH_KI, Hhh, k0, I0);
-    load(T_HEE_JK, Hee, J0, k0);
-    load(T_HEE_KI, Hee, k0, I0);
-    load(T_HEH_KI, Heh, k0, I0);
-    load(T_HEH_JK, Heh, J0, k0);
-    load(T_HEH_IK, Heh, I0, k0);
-    load(T_HEH_KJ, Heh, k0, J0);
-    load(T_P_KJ, p, k0, J0);
-    load(T_P_IK, p, I0, k0);
-    load(T_P_KI, p, k0, I0);
-    load(T_P_JK, p, J0, k0);
-    load(T_C_KJ, C, k0, J0);
-    load(T_C_IK, C, I0, k0);
-    load(T_D_KI, D, k0, I0);
-    load(T_D_IK, D, I0, k0);
-    load(T_D_KJ, D, k0, J0);
-    __syncthreads();
-    const int kn = min(kDT, nk - k0);
-    for (int kk = 0; kk < kn; ++kk) {
-      // dp[kh = i][ke = j]
-      a1 = ca(a1, cm(tile(T_HHH_IK, ty, kk), tile(T_P_KJ, kk, tx)));
-      a2 = ca(a2, cm(tile(T_HEE_JK, tx, kk), tile(T_P_IK, ty, kk)));
-      a3 = ca(a3, cm(tile(T_HEH_KI, kk, ty), tile(T_C_KJ, kk, tx)));
-      a4 = ca(a4, cm(tile(T_HEH_JK, tx, kk), tile(T_D_KI, kk, ty)));
-      // dC[k1 = i][k2 = j]
-      b1 = ca(b1, cm(tile(T_HEE_JK, tx, kk), tile(T_C_IK, ty, kk)));
-      b2 = ca(b2, cm(tile(T_HEE_KI, kk, ty), tile(T_C_KJ, kk, tx)));
-      b3 = ca(b3, cm(tile(T_HEH_JK, tx, kk), cconj(tile(T_P_KI, kk, ty))));
-      b4 = ca(b4, cm(cconj(tile(T_HEH_IK, ty, kk)), tile(T_P_KJ, kk, tx)));
-      // dD[k1 = i][k2 = j]
-      c1 = ca(c1, cm(tile(T_HHH_JK, tx, kk), tile(T_D_IK, ty, kk)));
-      c2 = ca(c2, cm(tile(T_HHH_KI, kk, ty), tile(T_D_KJ, kk, tx)));
-      c3 = ca(c3, cm(tile(T_HEH_KJ, kk, tx), cconj(tile(T_P_IK, ty, kk))));
-      c4 = ca(c4, cm(cconj(tile(T_HEH_KI, kk, ty)), tile(T_P_JK, tx, kk)));
+  // this thread's copies of a stage: element tid % (4 TM) of every second tile
+  auto load = [&](int st, int k0) {
+    double2* dst = dsm + st * kDStage<TM>;
+    const int half = tid / (4 * TM), el = tid % (4 * TM);
+    const int r = el >> 2, c = el & 3, kk = el / TM, cc = el % TM;
+    auto row_tile = [&](int t, const double2* M, int R0) {
+      const bool in = R0 + r < nk && k0 + c < nk;
+      cp16(dst + t * 4 * TM + el, in ? M + (R0 + r) * nk + k0 + c : M, in);
+    };
+    auto col_tile = [&](int t, const double2* M, int C0) {
+      const bool in = k0 + kk < nk && C0 + cc < nk;
+      cp16(dst + T_ROWS * 4 * TM + (t - T_ROWS) * 4 * (TM + 2) + kk * (TM + 2) + cc,
+           in ? M + (k0 + kk) * nk + C0 + cc : M, in);
+    };
+    if (half == 0) {
+      row_tile(T_HHH_IK, Hhh, I0);
+      row_tile(T_P_IK, p, I0);
+      row_tile(T_C_IK, C, I0);
+      row_tile(T_HEH_IK, Heh, I0);
+      row_tile(T_D_IK, D, I0);
+      col_tile(T_P_KJ, p, J0);
+      col_tile(T_C_KJ, C, J0);
+      col_tile(T_D_KJ, D, J0);
+      col_tile(T_HEH_KJ, Heh, J0);
+    } else {
+      row_tile(T_HEE_JK, Hee, J0);
+      row_tile(T_HEH_JK, Heh, J0);
+      row_tile(T_HHH_JK, Hhh, J0);
+      row_tile(T_P_JK, p, J0);
+      col_tile(T_HEH_KI, Heh, I0);
+      col_tile(T_D_KI, D, I0);
+      col_tile(T_HEE_KI, Hee, I0);
+      col_tile(T_P_KI, p, I0);
+      col_tile(T_HHH_KI, Hhh, I0);
     }
+  };
+  static_assert(NT == 8 * TM, "two tiles per pass of the threads");
+  const int wi = (wp & 1) * 8 * MT, wj = (wp >> 1) * 8;  // the warp's rows and columns
+  const int fr = lane >> 2, fk = lane & 3;               // fragment row (or column), k
+  CAcc dp[MT] = {}, dC[MT] = {}, dD[MT] = {};
+  const int nks = (nk + 3) / 4;
+#pragma unroll
+  for (int st = 0; st < kDStages - 1; ++st) {
+    if (st < nks) load(st, 4 * st);
+    cp_commit();
+  }
+  for (int ks = 0; ks < nks; ++ks) {
+    cp_wait<kDStages - 2>();
     __syncthreads();
+    if (ks + kDStages - 1 < nks) load((ks + kDStages - 1) % kDStages, 4 * (ks + kDStages - 1));
+    cp_commit();
+    if (J0 + wj >= nk || I0 + wi >= nk) continue;
+    const double2* sm = dsm + (ks % kDStages) * kDStage<TM>;
+    auto rowf = [&](int t, int r0) { return sm[t * 4 * TM + (r0 + fr) * 4 + fk]; };
+    auto colf = [&](int t, int c0) {
+      return sm[T_ROWS * 4 * TM + (t - T_ROWS) * 4 * (TM + 2) + fk * (TM + 2) + c0 + fr];
+    };
+    const double2 b_p = colf(T_P_KJ, wj), b_c = colf(T_C_KJ, wj), b_d = colf(T_D_KJ, wj),
+                  b_h = colf(T_HEH_KJ, wj);
+    const double2 b_ee = rowf(T_HEE_JK, wj), b_eh = rowf(T_HEH_JK, wj),
+                  b_hh = rowf(T_HHH_JK, wj), b_pt = rowf(T_P_JK, wj);
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      const int r0 = wi + 8 * m;
+      if (m > 0 && I0 + r0 >= nk) break;
+      const double2 a_pi = rowf(T_P_IK, r0), a_hki = colf(T_HEH_KI, r0);
+      cmma<false>(dp[m], rowf(T_HHH_IK, r0), b_p);
+      cmma<false>(dC[m], rowf(T_C_IK, r0), b_ee);
+      cmma<false>(dD[m], rowf(T_D_IK, r0), b_hh);
+      cmma<false>(dp[m], a_pi, b_ee);
+      cmma<false>(dC[m], neg(colf(T_HEE_KI, r0)), b_c);
+      cmma<false>(dD[m], neg(colf(T_HHH_KI, r0)), b_d);
+      cmma<false>(dp[m], neg(a_hki), b_c);
+      cmma<true>(dC[m], colf(T_P_KI, r0), b_eh);
+      cmma<true>(dD[m], a_pi, b_h);
+      cmma<false>(dp[m], neg(colf(T_D_KI, r0)), b_eh);
+      cmma<true>(dC[m], neg(rowf(T_HEH_IK, r0)), b_p);
+      cmma<true>(dD[m], neg(a_hki), b_pt);
+    }
   }
-  if (i >= nk || j >= nk) return;
-  const int e = i * nk + j;
-  const double hb = s.prm.hbar;
-  {
-    double2 r = cs(cs(ca(a1, a2), a3), a4);
-    r = ca(r, Heh[j * nk + i]);
-    // GamE[ke] + GamH[kh]: the constant rates, or CalcGammaE/H's
-    const double g = s.GamE ? s.GamE[j] + s.GamH[i] : s.prm.gam_e + s.prm.gam_h;
-    r = cs(r, cm(make_double2(0.0 * g, hb * g), p[i * nk + j]));
-    if (s.OffP) r = ca(r, s.OffP[e]);  // + OffP[kh][ke]
-    s.dX[e] = div_ih(r, hb);
-  }
-  s.dX[n2 + e] = div_ih(cs(ca(cs(b1, b2), b3), b4), hb);
-  s.dX[2 * n2 + e] = div_ih(cs(ca(cs(c1, c2), c3), c4), hb);
+  const double hb = s.prm.hbar, dt2 = 2.0 * s.prm.dt;
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int i = I0 + wi + 8 * m + fr, j = J0 + wj + 2 * fk + c;
+      if (i >= nk || j >= nk) continue;
+      const int e = i * nk + j;
+      double2 r = ca(make_double2(dp[m].re[c], dp[m].im[c]), Heh[j * nk + i]);
+      // GamE[ke] + GamH[kh]: the constant rates, or CalcGammaE/H's
+      const double g = s.GamE ? s.GamE[j] + s.GamH[i] : s.prm.gam_e + s.prm.gam_h;
+      r = cs(r, cm(make_double2(0.0 * g, hb * g), p[e]));
+      if (s.OffP) r = ca(r, s.OffP[e]);  // + OffP[kh][ke]
+      s.X3[e] = ca(s.L2[e], rs(dt2, div_ih(r, hb)));
+      s.X3[n2 + e] =
+          ca(s.L2[n2 + e], rs(dt2, div_ih(make_double2(dC[m].re[c], dC[m].im[c]), hb)));
+      s.X3[2 * n2 + e] =
+          ca(s.L2[2 * n2 + e], rs(dt2, div_ih(make_double2(dD[m].re[c], dD[m].im[c]), hb)));
+    }
 }
 
-// Leapfrog with neutrality and reshuffle (SBEs.py:5681-5718), one CTA.
+// Neutrality and reshuffle of the leapfrog (SBEs.py:5704-5718): the sums of
+// the new occupations' moduli, then every element of the three levels.
 constexpr int kLfThreads = 256;
-__global__ void __launch_bounds__(kLfThreads) leapfrog_kernel(Step s0) {
+__global__ void __launch_bounds__(kLfThreads) occ_sums_kernel(Step s0) {
   const Step s = at_wire(s0);
   const int nk = s.nk, n2 = nk * nk;
-  const double dt = s.prm.dt, small = 1e-200;
-  __shared__ double red_e[kLfThreads], red_h[kLfThreads];
-  __shared__ double fac[3];
-  auto x3_of = [&](int e) -> double2 {
-    if (s.X3) return s.X3[e];  // relaxed occupations (many-body terms)
-    return ca(s.L2[e], rs(2.0, rs(dt, s.dX[e])));  // X1 + dX dt 2
-  };
+  __shared__ double red[2][kLfThreads / 32];
   double se = 0.0, sh = 0.0;
   for (int k = threadIdx.x; k < nk; k += kLfThreads) {
-    const double2 c3 = x3_of(n2 + k * nk + k), d3 = x3_of(2 * n2 + k * nk + k);
+    const double2 c3 = s.X3[n2 + k * nk + k], d3 = s.X3[2 * n2 + k * nk + k];
     se += hypot(c3.x, c3.y);
     sh += hypot(d3.x, d3.y);
   }
-  red_e[threadIdx.x] = se;
-  red_h[threadIdx.x] = sh;
-  __syncthreads();
-  for (int o = kLfThreads / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-      red_e[threadIdx.x] += red_e[threadIdx.x + o];
-      red_h[threadIdx.x] += red_h[threadIdx.x + o];
-    }
-    __syncthreads();
+  se = warp_sum(se);
+  sh = warp_sum(sh);
+  if ((threadIdx.x & 31) == 0) {
+    red[0][threadIdx.x >> 5] = se;
+    red[1][threadIdx.x >> 5] = sh;
   }
+  __syncthreads();
   if (threadIdx.x == 0) {
-    const double total = (red_e[0] + red_h[0]) / 2.0;
-    fac[0] = total;
-    fac[1] = red_e[0] + small;
-    fac[2] = red_h[0] + small;
+    const double small = 1e-200;
+    se = sh = 0.0;
+    for (int i = 0; i < kLfThreads / 32; ++i) {
+      se += red[0][i];
+      sh += red[1][i];
+    }
+    s.fac[0] = (se + sh) / 2.0;
+    s.fac[1] = se + small;
+    s.fac[2] = sh + small;
   }
-  __syncthreads();
-  for (int e = threadIdx.x; e < 3 * n2; e += kLfThreads) {
-    const double2 x1 = s.L2[e];
-    double2 x3 = x3_of(e);
-    const int m = e / n2, r = e - m * n2;
-    if (m > 0 && r / nk == r % nk)  // occupation: |X3_kk| total / sum
-      x3 = make_double2(hypot(x3.x, x3.y) * fac[0] / fac[m], 0.0);
-    s.L1[e] = x1;
-    s.L3[e] = x3;
-    s.L2[e] = make_double2((x1.x + x3.x) / 2.0, (x1.y + x3.y) / 2.0);
-  }
+}
+
+__global__ void __launch_bounds__(kLfThreads) leapfrog_kernel(Step s0) {
+  const Step s = at_wire(s0);
+  const int nk = s.nk, n2 = nk * nk;
+  const int e = blockIdx.x * kLfThreads + threadIdx.x;
+  if (e >= 3 * n2) return;
+  const double2 x1 = s.L2[e];
+  double2 x3 = s.X3[e];
+  const int m = e / n2, r = e - m * n2;
+  if (m > 0 && r / nk == r % nk)  // occupation: |X3_kk| total / sum
+    x3 = make_double2(hypot(x3.x, x3.y) * s.fac[0] / s.fac[m], 0.0);
+  s.L1[e] = x1;
+  s.L3[e] = x3;
+  s.L2[e] = make_double2((x1.x + x3.x) / 2.0, (x1.y + x3.y) / 2.0);
 }
 
 // Wire-space sources of one level: the QWPolarization3 sums (before the
@@ -642,15 +733,6 @@ __global__ void mb_offp_kernel(MBView v0) {
   }
   // x * i * hbar
   v.OffP[e] = make_double2(-x.y * v.hbar, x.x * v.hbar);
-}
-
-// X3 = X1 + 2 dt dX, written out for the relaxation (SBEs.py:5685-5687).
-__global__ void mb_x3_kernel(Step s0, MBView v0) {
-  const Step s = at_wire(s0);
-  double2* X3 = at_wire(v0).X3;
-  const int n3 = 3 * s.nk * s.nk, e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n3) return;
-  X3[e] = ca(s.L2[e], rs(2.0, rs(s.prm.dt, s.dX[e])));
 }
 
 // In/out scattering rates of the new occupations (SBESolver._relaxation_E/H,
@@ -1155,14 +1237,37 @@ int check_mb(const PsbFullMB* mb, bool deph, bool relax, bool dct) {
   return PSB_OK;
 }
 
+// Blocks of 32 x 32 elements once they fill the GPU twice over, else of
+// 16 x 16: 64 wires of Nk 114 have 1024 blocks of 32, one wire 16 (64 of 16).
+int launch_derivs(const full::Step& s, int nw, cudaStream_t st) {
+  static std::once_flag once;
+  static cudaError_t attr = cudaSuccess;
+  constexpr size_t sm32 = (size_t)full::kDStages * full::kDStage<32> * sizeof(double2);
+  constexpr size_t sm16 = (size_t)full::kDStages * full::kDStage<16> * sizeof(double2);
+  std::call_once(once, [] {
+    attr = cudaFuncSetAttribute(full::derivs_kernel<32>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm32);
+    if (attr == cudaSuccess)
+      attr = cudaFuncSetAttribute(full::derivs_kernel<16>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm16);
+  });
+  if (attr != cudaSuccess) return set_error(PSB_ERR_CUDA, "derivs_kernel: shared memory");
+  const int n32 = (s.nk + 31) / 32, n16 = (s.nk + 15) / 16;
+  if ((int64_t)n32 * n32 * nw >= 592)
+    full::derivs_kernel<32><<<dim3(n32, nw, n32), 256, sm32, st>>>(s);
+  else
+    full::derivs_kernel<16><<<dim3(n16, nw, n16), 128, sm16, st>>>(s);
+  return PSB_OK;
+}
+
 int full_launch(const Launch& a, cudaStream_t st) {
   const int nk = a.nk, nw = a.nw, n2 = nk * nk;
   const PsbFullMB* mb = a.mb;
   const bool deph = mb && (mb->diag_dph || mb->offdiag_dph);
   const bool relax = mb && (mb->ehs || mb->phonon);
   const bool dct = mb && mb->dctrans;
-  const int rc = check_mb(mb, deph, relax, dct);
-  if (rc != PSB_OK) return rc;
+  int rc_ = check_mb(mb, deph, relax, dct);
+  if (rc_ != PSB_OK) return rc_;
   full::Step s{};
   s.nk = nk;
   s.nr = a.nr;
@@ -1176,9 +1281,10 @@ int full_launch(const Launch& a, cudaStream_t st) {
   s.L2 = reinterpret_cast<double2*>(a.L2);
   s.L3 = reinterpret_cast<double2*>(a.L3);
   double2* w = reinterpret_cast<double2*>(a.work);
-  s.Meh = w;
+  s.fac = reinterpret_cast<double*>(w);
   s.H = w + n2;
-  s.dX = w + 4 * n2;
+  s.X3 = w + 4 * n2;
+  s.st_x3 = a.st_wk;
   s.st_v3 = a.st_v3;
   s.st_e = (int64_t)3 * a.nr * 16;
   s.st_lv = (int64_t)3 * n2 * 16;
@@ -1231,16 +1337,24 @@ int full_launch(const Launch& a, cudaStream_t st) {
   }
   const int th = 128;
   const dim3 bl((n2 + th - 1) / th, nw), blk((nk + th - 1) / th, nw);
-  full::meh_kernel<<<bl, th, 0, st>>>(s);
+  if (relax || dct) {
+    // X3 goes where the relaxation and the shift find it
+    s.X3 = v.X3;
+    s.st_x3 = s.st_sc;
+  }
   {
     static std::once_flag once;
     static cudaError_t attr = cudaSuccess;
     std::call_once(once, [] {
       attr = cudaFuncSetAttribute(full::calch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  5 * PSB_MAX_NK * 16);
+                                  227 * 1024);
     });
     if (attr != cudaSuccess) return set_error(PSB_ERR_CUDA, "calch_kernel: shared memory");
-    full::calch_kernel<<<dim3(2 * nk - 1, nw), full::kHThreads, 5 * (size_t)nk * 16, st>>>(s);
+    // two CTAs per SM where that leaves several diagonals in one
+    int nd = full::kHDiags;
+    while (nd > 1 && full::h_smem(nk, nd) > 110 * 1024) nd /= 2;
+    full::calch_kernel<<<dim3((2 * nk - 1 + nd - 1) / nd, nw), 32 * nd, full::h_smem(nk, nd),
+                         st>>>(s);
   }
   // dephasing from the level the right-hand side reads (SBEs.py:5225-5232)
   if (mb && mb->diag_dph) {
@@ -1254,22 +1368,11 @@ int full_launch(const Launch& a, cudaStream_t st) {
     full::mb_offp_kernel<<<bl, th, 0, st>>>(v);
     s.OffP = v.OffP;
   }
-  {
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-      attr = cudaFuncSetAttribute(full::derivs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)full::kDerivsSmem);
-    });
-    if (attr != cudaSuccess) return set_error(PSB_ERR_CUDA, "derivs_kernel: shared memory");
-    const int nb = (nk + full::kDT - 1) / full::kDT;
-    full::derivs_kernel<<<dim3(nb, nw, nb), full::kDT * full::kDT, full::kDerivsSmem, st>>>(s);
-  }
+  rc_ = launch_derivs(s, nw, st);
+  if (rc_ != PSB_OK) return rc_;
   if (relax || dct) {
-    // X3, its occupations relaxed (SBEs.py:5688-5695) and shifted by the DC
-    // field (SBEs.py:5698-5702), then the rescale
-    const dim3 b3((3 * n2 + th - 1) / th, nw);
-    full::mb_x3_kernel<<<b3, th, 0, st>>>(s, v);
+    // X3's occupations relaxed (SBEs.py:5688-5695) and shifted by the DC field
+    // (SBEs.py:5698-5702), then the rescale
     if (relax) {
       const size_t smr = (2 * (size_t)(nk + 1) + 3 * (size_t)nk) * 8;
       full::mb_rates_kernel<<<dim3(nk, nw), full::kRateThreads, smr, st>>>(v);
@@ -1288,9 +1391,10 @@ int full_launch(const Launch& a, cudaStream_t st) {
         full::mb_shift_diag_store_kernel<<<bd, th, 0, st>>>(v);
       }
     }
-    s.X3 = v.X3;
   }
-  full::leapfrog_kernel<<<one, full::kLfThreads, 0, st>>>(s);
+  full::occ_sums_kernel<<<one, full::kLfThreads, 0, st>>>(s);
+  const dim3 b3((3 * n2 + full::kLfThreads - 1) / full::kLfThreads, nw);
+  full::leapfrog_kernel<<<b3, full::kLfThreads, 0, st>>>(s);
   return PSB_OK;
 }
 }  // namespace
