@@ -445,27 +445,135 @@ __global__ void __launch_bounds__(kLfThreads) leapfrog_kernel(Step s0) {
 //   Py, Pz likewise with dcv yw, -dcv (-1)^w,
 //   Re(r) = W(r)/(2L) sum_{k1,k2} C[k1][k2] conj(E[k1]) E[k2],
 //   Rh(r) = W(r)/(2L) sum_{k1,k2} conj(D[k1][k2]) conj(E[k1]) E[k2],
-// E[k] = exp(i kr[k] r) (qwoptics.py:56-84, 367-381).  One CTA per
-// kSrcR positions and wire (blockIdx.y of a batch: levels [nw][3][nk][nk],
-// out [nw][5][nr], yw and (-1)^w from wpar[4 w], wpar[4 w + 1] when set):
-// the phases of its positions in shared memory, threads over the column
-// (ke, k2) so the rows of p, C, D are read coalesced, each element once for
-// all kSrcR positions, then a block reduction.  The sums run in this tree
-// order, not the reference's sequential one (they agree to rounding).
-constexpr int kSrcThreads = 128, kSrcR = 4;
-__global__ void __launch_bounds__(kSrcThreads) sources_kernel(
-    int nk, int nr, const double* kr, const double* rpos, const double* window, double L,
-    double dcv, double yw, double sgnw, const double* wpar, const double2* lev, double2* out) {
-  extern __shared__ double2 ph[];  // [kSrcR][nk]
-  __shared__ double red[kSrcR][6][kSrcThreads / 32];
-  const int n2 = nk * nk, r0 = blockIdx.x * kSrcR;
+// E[k] = exp(i kr[k] r) (qwoptics.py:56-84, 367-381); blockIdx.y the wire of a
+// batch (levels [nw][3][nk][nk], out [nw][5][nr], yw and (-1)^w from wpar[4 w],
+// wpar[4 w + 1] when set).
+//
+// Polarisation.  On a uniform k grid (the reference's) conj(E[i]) E[c] =
+// exp(i (c - i) dk r) depends on c - i alone, so a CTA first sums p along its
+// diagonals, plain and with Xcv's sign, thread d over the rows (the threads of
+// a warp read neighbouring columns), and then each warp evaluates the 2 nk - 1
+// terms of one position after another, the diagonals d and -d together: nk^2 +
+// nk nr operations instead of nk^2 nr.  gridDim.x CTAs share the positions of a
+// wire; each makes its own diagonal sums.  Phases advance by a rotation of 32
+// dk r from an exact first value per lane.  Any other k grid takes the sums
+// over (i, c) as they stand, a warp per position.
+constexpr int kPolThreads = 512, kPolLanes = 128, kPolGroups = kPolThreads / kPolLanes;
+__global__ void __launch_bounds__(kPolThreads) polarisation_kernel(
+    int nk, int nr, const double* kr, const double* rpos, const double* window, double dcv,
+    double yw, double sgnw, const double* wpar, const double2* lev, double2* out, int fit) {
+  extern __shared__ __align__(16) double2 ssm[];  // [2][2 nk - 1], or [fit][nk] phases
+  const int nd = 2 * nk - 1, tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
   const int64_t w = blockIdx.y;
-  lev += w * 3 * n2;
+  const double2* p = lev + w * 3 * nk * nk;
   out += w * 5 * nr;
   if (wpar) {
     yw = wpar[4 * w];
     sgnw = wpar[4 * w + 1];
   }
+  const double k0 = kr[0], dk = (kr[nk - 1] - k0) / (nk - 1);
+  const double tol = 0x1p-47 * fmax(fabs(k0), fabs(kr[nk - 1]));
+  bool off = !(fabs(dk) > 0.0);
+  for (int k = tid; k < nk; k += kPolThreads) off |= !(fabs(kr[k] - (k0 + k * dk)) <= tol);
+  const bool uniform = !__syncthreads_or(off);
+  const int npos = (nr + gridDim.x - 1) / gridDim.x, r0 = blockIdx.x * npos,
+            r1 = min(nr, r0 + npos);
+  const double2 z = make_double2(0.0, 0.0);
+  auto store = [&](int r, double sx, double sp) {
+    const double W = window[r];
+    out[r] = make_double2(W * dcv * sx, 0.0);
+    out[nr + r] = make_double2(W * yw * dcv * sp, 0.0);
+    out[2 * nr + r] = make_double2(W * sgnw * -dcv * sp, 0.0);
+  };
+  if (!uniform) {
+    // `fit` warps have room for their position's phases
+    double2* ph = ssm + wp * nk;
+    for (int r = r0 + wp; wp < fit && r < r1; r += fit) {
+      for (int k = lane; k < nk; k += 32) {
+        double sn, cn;
+        sincos(kr[k] * rpos[r], &sn, &cn);
+        ph[k] = make_double2(cn, sn);
+      }
+      __syncwarp();
+      double sx = 0.0, sp = 0.0;
+      for (int c = lane; c < nk; c += 32)
+        for (int i = 0; i < nk; ++i) {
+          const double x = cm(cm(p[i * nk + c], ph[c]), cconj(ph[i])).x;
+          sx += ((i + 1) & 1) ? -x : x;  // conj(Xcv) / dcv at kh = i
+          sp += x;
+        }
+      sx = warp_sum(sx);
+      sp = warp_sum(sp);
+      if (lane == 0) store(r, sx, sp);
+      __syncwarp();
+    }
+    return;
+  }
+  // diagonal sums: d = c - i at d + nk - 1; row groups add up in turn
+  const int grp = tid / kPolLanes;
+  for (int d0 = 0; d0 < nd; d0 += kPolLanes) {
+    const int di = d0 + tid % kPolLanes, d = di - (nk - 1);
+    double2 fx = z, fp = z;
+    if (di < nd) {
+      const int i0 = d < 0 ? -d : 0, i1 = d < 0 ? nk : nk - d;
+#pragma unroll 4
+      for (int i = i0 + grp; i < i1; i += kPolGroups) {
+        const double2 pv = p[i * nk + i + d];
+        fx = ((i + 1) & 1) ? cs(fx, pv) : ca(fx, pv);
+        fp = ca(fp, pv);
+      }
+    }
+    for (int g = 0; g < kPolGroups; ++g) {
+      if (grp == g && di < nd) {
+        ssm[di] = g == 0 ? fx : ca(ssm[di], fx);
+        ssm[nd + di] = g == 0 ? fp : ca(ssm[nd + di], fp);
+      }
+      __syncthreads();
+    }
+  }
+  // positions: Re sum_d F[d] exp(i d phi), phi = dk r
+  for (int r = r0 + wp; r < r1; r += kPolThreads / 32) {
+    const double phi = dk * rpos[r];
+    double2 e, st;
+    sincos((double)lane * phi, &e.y, &e.x);
+    sincos(32.0 * phi, &st.y, &st.x);
+    double sx = 0.0, sp = 0.0;
+    for (int d = lane; d < nk; d += 32) {
+      const double2* f = ssm + nk - 1;
+      // Re(F[d] e + F[-d] conj(e))
+      auto term = [&](const double2* g) {
+        const double x = g[d].x * e.x - g[d].y * e.y;
+        return d == 0 ? x : x + (g[-d].x * e.x + g[-d].y * e.y);
+      };
+      sx += term(f);
+      sp += term(f + nd);
+      e = cm(e, st);
+    }
+    sx = warp_sum(sx);
+    sp = warp_sum(sp);
+    if (lane == 0) store(r, sx, sp);
+  }
+}
+
+// Densities.  A caller takes the difference of the two (Rho = RhoH - RhoE),
+// which cancels to the last digits while electrons and holes move alike, so
+// every position's two sums keep the same order and phases: one CTA per R
+// positions and wire, the phases of its positions in shared memory, threads
+// over the column k2 so the rows of C, D are read coalesced, each element once
+// for all R positions and four rows ahead, then a block reduction.  64 wires,
+// Nk 114, 230 positions: 0.29 ms (FP64 floor of these products 0.21), with the
+// polarisation 0.03 ms; 0.43 with all sums in one kernel of 4 positions.
+constexpr int kSrcThreads = 128;
+template <int kSrcR>
+__global__ void __launch_bounds__(kSrcThreads) densities_kernel(
+    int nk, int nr, const double* kr, const double* rpos, const double* window, double L,
+    const double2* lev, double2* out) {
+  extern __shared__ double2 ph[];  // [kSrcR][nk]
+  __shared__ double red[kSrcR][4][kSrcThreads / 32];
+  const int n2 = nk * nk, r0 = blockIdx.x * kSrcR;
+  const int64_t w = blockIdx.y;
+  lev += w * 3 * n2;
+  out += w * 5 * nr;
   for (int e = threadIdx.x; e < kSrcR * nk; e += kSrcThreads) {
     const int j = e / nk, k = e - j * nk;
     const int r = min(r0 + j, nr - 1);
@@ -474,40 +582,46 @@ __global__ void __launch_bounds__(kSrcThreads) sources_kernel(
     ph[e] = make_double2(cn, sn);
   }
   __syncthreads();
-  const double2* p = lev;
   const double2* C = lev + n2;
   const double2* D = lev + 2 * n2;
-  double sx[kSrcR], sp[kSrcR];
   double2 se[kSrcR], sh[kSrcR];
 #pragma unroll
-  for (int j = 0; j < kSrcR; ++j) {
-    sx[j] = sp[j] = 0.0;
-    se[j] = sh[j] = make_double2(0.0, 0.0);
-  }
+  for (int j = 0; j < kSrcR; ++j) se[j] = sh[j] = make_double2(0.0, 0.0);
   for (int c = threadIdx.x; c < nk; c += kSrcThreads) {
     double2 ec[kSrcR];
 #pragma unroll
     for (int j = 0; j < kSrcR; ++j) ec[j] = ph[j * nk + c];
-    for (int i = 0; i < nk; ++i) {
-      const double2 pv = p[i * nk + c], cv = C[i * nk + c], dv = cconj(D[i * nk + c]);
-      const double xs = ((i + 1) & 1) ? -1.0 : 1.0;  // conj(Xcv) / dcv at kh = i
+    constexpr int kAhead = 4;
+    double2 cb[kAhead], db[kAhead];
 #pragma unroll
-      for (int j = 0; j < kSrcR; ++j) {
-        const double2 ei = cconj(ph[j * nk + i]);
-        const double t = cm(cm(pv, ec[j]), ei).x;
-        sx[j] += xs * t;
-        sp[j] += t;
-        se[j] = ca(se[j], cm(cm(cv, ei), ec[j]));
-        sh[j] = ca(sh[j], cm(cm(dv, ei), ec[j]));
+    for (int u = 0; u < kAhead; ++u) {
+      const int i = min(u, nk - 1);
+      cb[u] = C[i * nk + c];
+      db[u] = D[i * nk + c];
+    }
+    for (int i0 = 0; i0 < nk; i0 += kAhead) {
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const int i = i0 + u, n = min(i + kAhead, nk - 1);
+        const double2 cv = cb[u], dv = cconj(db[u]);
+        cb[u] = C[n * nk + c];
+        db[u] = D[n * nk + c];
+        if (i >= nk) break;
+#pragma unroll
+        for (int j = 0; j < kSrcR; ++j) {
+          const double2 ei = cconj(ph[j * nk + i]);
+          se[j] = ca(se[j], cm(cm(cv, ei), ec[j]));
+          sh[j] = ca(sh[j], cm(cm(dv, ei), ec[j]));
+        }
       }
     }
   }
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
 #pragma unroll
   for (int j = 0; j < kSrcR; ++j) {
-    const double v[6] = {sx[j], sp[j], se[j].x, se[j].y, sh[j].x, sh[j].y};
+    const double v[4] = {se[j].x, se[j].y, sh[j].x, sh[j].y};
 #pragma unroll
-    for (int q = 0; q < 6; ++q) {
+    for (int q = 0; q < 4; ++q) {
       const double u = warp_sum(v[q]);
       if (lane == 0) red[j][q][wp] = u;
     }
@@ -516,17 +630,14 @@ __global__ void __launch_bounds__(kSrcThreads) sources_kernel(
   if (threadIdx.x < kSrcR) {
     const int j = threadIdx.x, r = r0 + j;
     if (r < nr) {
-      double t[6];
-      for (int q = 0; q < 6; ++q) {
+      double t[4];
+      for (int q = 0; q < 4; ++q) {
         t[q] = 0.0;
         for (int u = 0; u < kSrcThreads / 32; ++u) t[q] += red[j][q][u];
       }
       const double W = window[r], h = W / (2.0 * L);
-      out[r] = make_double2(W * dcv * t[0], 0.0);
-      out[nr + r] = make_double2(W * yw * dcv * t[1], 0.0);
-      out[2 * nr + r] = make_double2(W * sgnw * -dcv * t[1], 0.0);
-      out[3 * nr + r] = make_double2(h * t[2], h * t[3]);
-      out[4 * nr + r] = make_double2(h * t[4], h * t[5]);
+      out[3 * nr + r] = make_double2(h * t[0], h * t[1]);
+      out[4 * nr + r] = make_double2(h * t[2], h * t[3]);
     }
   }
 }
@@ -1493,18 +1604,33 @@ extern "C" int psb_full_step_batch_f64(int nw, int nk, int nr, int nq0, const do
 }
 
 namespace {
-// dynamic shared memory of sources_kernel (the phases of its positions),
-// with the opt-in above 48 KB set on first use; 0 if that fails
-size_t sources_smem(int nk) {
-  const size_t sm = (size_t)full::kSrcR * nk * 16;
-  static std::once_flag once;
-  static bool ok = true;
-  if (sm > 48 * 1024)
-    std::call_once(once, [] {
-      ok = cudaFuncSetAttribute(full::sources_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                full::kSrcR * PSB_MAX_NK * 16) == cudaSuccess;
-    });
-  return ok ? sm : 0;
+// both source kernels for nw wires; CTAs of the polarisation until the GPU has
+// about one each
+int launch_sources(int nw, int nk, int nr, const double* kr, const double* r,
+                   const double* window, double L, double dcv, double yw, double sgnw,
+                   const double* wpar, const double* lev, double* out, cudaStream_t st) {
+  // 8 positions per CTA of the densities once that leaves two CTAs per SM
+  const bool wide = (int64_t)(nr + 7) / 8 * nw >= 296;
+  const int R = wide ? 8 : 4;
+  auto dens = wide ? full::densities_kernel<8> : full::densities_kernel<4>;
+  const size_t sp = (size_t)2 * (2 * nk - 1) * 16, sd = (size_t)R * nk * 16;
+  const size_t big = sp > sd ? sp : sd;
+  if (big > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(full::polarisation_kernel,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(dens, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sd);
+    if (e != cudaSuccess)
+      return set_error(PSB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  }
+  const double2* lv = reinterpret_cast<const double2*>(lev);
+  double2* o = reinterpret_cast<double2*>(out);
+  const int fit = (int)(sp / ((size_t)nk * 16));  // 3: warps of the general sums
+  const int nb = nw >= 148 ? 1 : (148 / nw < 16 ? 148 / nw : 16);
+  dens<<<dim3((nr + R - 1) / R, nw), full::kSrcThreads, sd, st>>>(nk, nr, kr, r, window, L, lv, o);
+  full::polarisation_kernel<<<dim3(nb, nw), full::kPolThreads, sp, st>>>(
+      nk, nr, kr, r, window, dcv, yw, sgnw, wpar, lv, o, fit);
+  return check_cuda("sources kernels");
 }
 }  // namespace
 
@@ -1516,13 +1642,8 @@ extern "C" int psb_full_sources_f64(int nk, int nr, const double* d_kr, const do
     return set_error(PSB_ERR_INVALID, "psb_full_sources_f64: null pointer");
   if (nk < 2 || nk > PSB_MAX_NK || nr < 1)
     return set_error(PSB_ERR_SIZE, "psb_full_sources_f64: nk %d / nr %d out of range", nk, nr);
-  const size_t sm = sources_smem(nk);
-  if (!sm) return set_error(PSB_ERR_CUDA, "psb_full_sources_f64: shared memory");
-  full::sources_kernel<<<(nr + full::kSrcR - 1) / full::kSrcR, full::kSrcThreads, sm,
-                         (cudaStream_t)stream>>>(
-      nk, nr, d_kr, d_r, d_window, L, dcv, yw, sgnw, nullptr,
-      reinterpret_cast<const double2*>(d_level), reinterpret_cast<double2*>(d_out));
-  return check_cuda("psb_full_sources_f64");
+  return launch_sources(1, nk, nr, d_kr, d_r, d_window, L, dcv, yw, sgnw, nullptr, d_level, d_out,
+                        (cudaStream_t)stream);
 }
 
 extern "C" int psb_full_sources_batch_f64(int nw, int nk, int nr, const double* d_kr,
@@ -1534,11 +1655,6 @@ extern "C" int psb_full_sources_batch_f64(int nw, int nk, int nr, const double* 
   if (nk < 2 || nk > PSB_MAX_NK || nr < 1 || nw < 1 || nw > PSB_FULL_MAX_WIRES)
     return set_error(PSB_ERR_SIZE, "psb_full_sources_batch_f64: nw %d / nk %d / nr %d", nw, nk,
                      nr);
-  const size_t sm = sources_smem(nk);
-  if (!sm) return set_error(PSB_ERR_CUDA, "psb_full_sources_batch_f64: shared memory");
-  const dim3 bl((nr + full::kSrcR - 1) / full::kSrcR, nw);
-  full::sources_kernel<<<bl, full::kSrcThreads, sm, (cudaStream_t)stream>>>(
-      nk, nr, d_kr, d_r, d_window, L, dcv, 0.0, 0.0, d_wpar,
-      reinterpret_cast<const double2*>(d_levels), reinterpret_cast<double2*>(d_out));
-  return check_cuda("psb_full_sources_batch_f64");
+  return launch_sources(nw, nk, nr, d_kr, d_r, d_window, L, dcv, 0.0, 0.0, d_wpar, d_levels,
+                        d_out, (cudaStream_t)stream);
 }
