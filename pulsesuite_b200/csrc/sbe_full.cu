@@ -692,10 +692,13 @@ __device__ __forceinline__ MBView at_wire(MBView v) {
 }
 
 // CalcGammaE / CalcGammaH (dephasing.py:28-105): ne, nh the real parts of
-// the diagonal of C2, D2; Vxx2[q] = V(iq[q])^2; one thread per k.
-__global__ void mb_gamma_kernel(MBView v0) {
+// the diagonal of C2, D2; Vxx2[q] = V(iq[q])^2.  One warp per k, its lanes over
+// q (the index maps are read along q), four sums and a reduction: 64 wires of
+// Nk 114 take 0.013 ms, 0.12 with a thread per k.
+constexpr int kGamWarps = 4;
+__global__ void __launch_bounds__(32 * kGamWarps) mb_gamma_kernel(MBView v0) {
   const MBView v = at_wire(v0);
-  const int nk = v.nk, k = blockIdx.x * blockDim.x + threadIdx.x;
+  const int nk = v.nk, k = blockIdx.x * kGamWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (k >= nk) return;
   const int n2 = nk * nk;
   const int32_t* kpq = v.mb.maps;
@@ -711,139 +714,197 @@ __global__ void mb_gamma_kernel(MBView v0) {
   auto in = [&](int i) { return i >= 0 && i < nk; };
   const double ph = kPi / v.hbar;
   double ge = 0.0, gh = 0.0;
-  // electron-electron, then electron-hole scattering of electrons
-  for (int q = 0; q < nk; ++q) {
-    const int a = kpq[k * nk + q];
+  for (int q = lane; q < nk; q += 32) {
+    const int e = k * nk + q, iq = v.mb.iq[q];
+    const double veh = v.V3[iq], vee = v.V3[nk + iq], vhh = v.V3[2 * nk + iq];
+    const double xe = fabs(v.mb.xe[q]), xh = fabs(v.mb.xh[q]);
+    // electron-electron and hole-hole scattering
+    const int a = kpq[e], c = kmq[e];
     if (in(a)) {
-      const double vv = v.V3[nk + v.mb.iq[q]];
-      ge = ge + ph * (vv * vv) * ne(a) * (1.0 - ne(a)) * fabs(v.mb.xe[q]);
+      ge = ge + ph * (vee * vee) * ne(a) * (1.0 - ne(a)) * xe;
+      gh = gh + ph * (vhh * vhh) * nh(a) * (1.0 - nh(a)) * xh;
+    }
+    // electron-hole scattering of electrons, of holes
+    if (in(c)) {
+      const int a1 = k1pmq[e], b1 = k1p[e], a2 = k1mq[e], b2 = k1[e];
+      if (in(a1) && in(b1))
+        ge = ge + ph * (veh * veh) *
+                      (nh(a1) * (1.0 - nh(b1)) * ne(c) + (1.0 - nh(a1)) * nh(b1) * (1.0 - ne(c))) *
+                      xh;
+      if (in(a2) && in(b2))
+        gh = gh + ph * (veh * veh) *
+                      (ne(a2) * (1.0 - ne(b2)) * nh(c) + (1.0 - ne(a2)) * ne(b2) * (1.0 - nh(c))) *
+                      xe;
     }
   }
-  for (int q = 0; q < nk; ++q) {
-    const int a = k1pmq[k * nk + q], b = k1p[k * nk + q], c = kmq[k * nk + q];
-    if (in(a) && in(b) && in(c)) {
-      const double vv = v.V3[v.mb.iq[q]];
-      ge = ge + ph * (vv * vv) *
-                    (nh(a) * (1.0 - nh(b)) * ne(c) + (1.0 - nh(a)) * nh(b) * (1.0 - ne(c))) *
-                    fabs(v.mb.xh[q]);
-    }
+  ge = warp_sum(ge);
+  gh = warp_sum(gh);
+  if (lane == 0) {
+    v.GamE[k] = ge;
+    v.GamH[k] = gh;
   }
-  // hole-hole, then electron-hole scattering of holes
-  for (int q = 0; q < nk; ++q) {
-    const int a = kpq[k * nk + q];
-    if (in(a)) {
-      const double vv = v.V3[2 * nk + v.mb.iq[q]];
-      gh = gh + ph * (vv * vv) * nh(a) * (1.0 - nh(a)) * fabs(v.mb.xh[q]);
-    }
-  }
-  for (int q = 0; q < nk; ++q) {
-    const int a = k1mq[k * nk + q], b = k1[k * nk + q], c = kmq[k * nk + q];
-    if (in(a) && in(b) && in(c)) {
-      const double vv = v.V3[v.mb.iq[q]];
-      gh = gh + ph * (vv * vv) *
-                    (ne(a) * (1.0 - ne(b)) * nh(c) + (1.0 - ne(a)) * ne(b) * (1.0 - nh(c))) *
-                    fabs(v.mb.xe[q]);
-    }
-  }
-  v.GamE[k] = ge;
-  v.GamH[k] = gh;
 }
 
-__device__ __forceinline__ double lrtz(double a, double b) { return (b / kPi) / (a * a + b * b); }
+// (b / pi) / (x^2 + b^2) and (c / pi) / (y^2 + c^2) with one division
+__device__ __forceinline__ void lrtz2(double x, double b, double y, double c, double& lx,
+                                      double& ly) {
+  const double dx = fma(x, x, __dmul_rn(b, b)), dy = fma(y, y, __dmul_rn(c, c));
+  const double r = (1.0 / kPi) / __dmul_rn(dx, dy);
+  lx = __dmul_rn(__dmul_rn(b, r), dy);
+  ly = __dmul_rn(__dmul_rn(c, r), dx);
+}
 
 // CalcOffDiagDeph_E2 / _H2 (dephasing.py:226-318): De[q + nk][k] and
 // Dh[q + nk][k] for q in [-nk, nk], with |C_kk|, |D_kk| as occupations and
-// Vsq(q) = V(|q|)^2 for 0 < |q| < nk; one thread per (q, k), the partner
-// momentum p in the reference's order, then the factor pi / hbar.  The
-// occupations and band energies are staged in shared memory per CTA.
-__global__ void mb_offd_kernel(MBView v0) {
-  const MBView v = at_wire(v0);
-  const int nk = v.nk, n2 = nk * nk;
-  extern __shared__ double osm[];  // [4][nk]: |C_kk|, |D_kk|, Ee, Eh
+// Vsq(q) = V(|q|)^2 for 0 < |q| < nk, times pi / hbar: one thread per (q, k),
+// the sums over the partner momentum p.  The Lorentzians of the energy
+// differences (most of the work, a division each) do not depend on the wire,
+// so a CTA takes W wires of the batch: 64 wires of Nk 114 take 0.18 ms with W
+// = 8, 0.76 with one wire per CTA.  A wire's own operations and their order do
+// not depend on W.
+template <int W>
+__global__ void __launch_bounds__(128) mb_offd_kernel(MBView v0, int nw) {
+  const int nk = v0.nk, n2 = nk * nk, wv0 = blockIdx.y * W;
+  extern __shared__ double osm[];  // Ee, Eh [nk]; [2][nk][W]: |C_kk|, |D_kk|
+  double* Ee = osm;
+  double* Eh = osm + nk;
+  double* occ = osm + 2 * nk;
   for (int i = threadIdx.x; i < nk; i += blockDim.x) {
-    const double2 c = v.L[n2 + i * nk + i], d = v.L[2 * n2 + i * nk + i];
-    osm[i] = hypot(c.x, c.y);
-    osm[nk + i] = hypot(d.x, d.y);
-    osm[2 * nk + i] = v.Ee[i];
-    osm[3 * nk + i] = v.Eh[i];
+    Ee[i] = v0.Ee[i];
+    Eh[i] = v0.Eh[i];
+  }
+  for (int i = threadIdx.x; i < nk * W; i += blockDim.x) {
+    const int w = min(wv0 + i / nk, nw - 1), k = i % nk;
+    const double2* L = bump(v0.L, w * v0.st_lv);
+    const double2 c = L[n2 + k * nk + k], d = L[2 * n2 + k * nk + k];
+    occ[k * W + i / nk] = hypot(c.x, c.y);
+    occ[(nk + k) * W + i / nk] = hypot(d.x, d.y);
   }
   __syncthreads();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= (2 * nk + 1) * nk) return;
-  const int qi = e / nk, k = e - qi * nk, q = qi - nk;
-  const double* Ee = osm + 2 * nk;
-  const double* Eh = osm + 3 * nk;
-  auto ne = [&](int i) { return osm[i]; };
-  auto nh = [&](int i) { return osm[nk + i]; };
+  const int qi = e / nk, k = e - qi * nk, q = qi - nk, kq = k + q;
   const int aq = q < 0 ? -q : q;
-  auto vsq = [&](int t) {
-    const double x = (aq > 0 && aq < nk) ? v.V3[t * nk + aq] : 0.0;
-    return x * x;
+  const double* ne = occ;
+  const double* nh = occ + nk * W;
+  const double hb = v0.hbar;
+  const double b_ee = hb * v0.mb.gam_eh, b_eh = hb * v0.mb.gam_h;  // De: gee = g[0], geh = g[2]
+  const double b_hh = hb * v0.mb.gam_e;                             // Dh: ghh = g[1], geh = g[2]
+  // sums of L n n: same-band (ee, hh), electron-hole (eh, he), per wire
+  double see[W], shh[W], seh[W], she[W];
+#pragma unroll
+  for (int w = 0; w < W; ++w) see[w] = shh[w] = seh[w] = she[w] = 0.0;
+  // a (1 - b)(1 - c) + (1 - a) b c, c the occupation at k, as
+  // (a - a b) + c (b - a)
+  auto add = [&](double& s, double L, double a, double b, double c) {
+    s = fma(L, fma(c, b - a, fma(-a, b, a)), s);
   };
-  const double hb = v.hbar;
-  const double b_ee = hb * v.mb.gam_eh, b_eh = hb * v.mb.gam_h;  // De: gee = g[0], geh = g[2]
-  const double b_hh = hb * v.mb.gam_e;                            // Dh: ghh = g[1], geh = g[2]
-  double de = 0.0, dh = 0.0;
-  const int kq = k + q;
-  const bool kin = kq >= 0 && kq < nk;
-  // same-band scattering: q in [max(p - nk, -k), min(p - 1, nk - k - 1)]
-  for (int p = 0; p < nk && kin; ++p) {
-    const int pm = p - q;
-    if (q < max(p - nk, -k) || q > min(p - 1, nk - k - 1) || pm < 0 || pm >= nk) continue;
-    const double Ed = ((Ee[kq] + Ee[pm]) - Ee[p]) - Ee[k];
-    de = de + vsq(1) * lrtz(Ed, b_ee) *
-                  (ne(pm) * (1.0 - ne(p)) * (1.0 - ne(k)) + (1.0 - ne(pm)) * ne(p) * ne(k));
+  if (kq >= 0 && kq < nk) {
+    const double ek = Ee[k], hk = Eh[k], ekq = Ee[kq], hkq = Eh[kq];
+    // same-band scattering: partners p and p - q in [1, nk - 1]
+    for (int p = max(0, q + 1); p <= min(nk - 1, nk - 1 + q); ++p) {
+      const int pm = p - q;
+      double le, lh;
+      lrtz2(((ekq + Ee[pm]) - Ee[p]) - ek, b_ee, ((hkq + Eh[pm]) - Eh[p]) - hk, b_hh, le, lh);
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        add(see[w], le, ne[pm * W + w], ne[p * W + w], ne[k * W + w]);
+        add(shh[w], lh, nh[pm * W + w], nh[p * W + w], nh[k * W + w]);
+      }
+    }
+    // electron-hole scattering: partners p and p + q
+    for (int p = max(0, -q); p <= min(nk - 1, nk - 1 - q); ++p) {
+      const int pp = p + q;
+      double le, lh;
+      lrtz2(((ekq + Eh[pp]) - Eh[p]) - ek, b_eh, ((hkq + Ee[pp]) - Ee[p]) - hk, b_eh, le, lh);
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        add(seh[w], le, nh[pp * W + w], nh[p * W + w], ne[k * W + w]);
+        add(she[w], lh, ne[pp * W + w], ne[p * W + w], nh[k * W + w]);
+      }
+    }
   }
-  // electron-hole scattering: q in [max(-p, -k), min(nk - p - 1, nk - k - 1)]
-  for (int p = 0; p < nk && kin; ++p) {
-    const int pp = p + q;
-    if (q < max(-p, -k) || q > min(nk - p - 1, nk - k - 1) || pp < 0 || pp >= nk) continue;
-    const double Ed = ((Ee[kq] + Eh[pp]) - Eh[p]) - Ee[k];
-    de = de + vsq(0) * lrtz(Ed, b_eh) *
-                  (nh(pp) * (1.0 - nh(p)) * (1.0 - ne(k)) + (1.0 - nh(pp)) * nh(p) * ne(k));
+#pragma unroll
+  for (int w = 0; w < W; ++w) {
+    const int wv = wv0 + w;
+    if (wv >= nw) break;
+    const double* V3 = bump(v0.V3, wv * v0.st_v3);
+    double vs[3];
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+      const double x = (aq > 0 && aq < nk) ? V3[t * nk + aq] : 0.0;
+      vs[t] = __dmul_rn(x, x);
+    }
+    const double f = kPi / hb;
+    bump(v0.De, wv * v0.st_sc)[e] = fma(vs[1], see[w], __dmul_rn(vs[0], seh[w])) * f;
+    bump(v0.Dh, wv * v0.st_sc)[e] = fma(vs[2], shh[w], __dmul_rn(vs[0], she[w])) * f;
   }
-  for (int p = 0; p < nk && kin; ++p) {
-    const int pm = p - q;
-    if (q < max(p - nk, -k) || q > min(p - 1, nk - k - 1) || pm < 0 || pm >= nk) continue;
-    const double Ed = ((Eh[kq] + Eh[pm]) - Eh[p]) - Eh[k];
-    dh = dh + vsq(2) * lrtz(Ed, b_hh) *
-                  (nh(pm) * (1.0 - nh(p)) * (1.0 - nh(k)) + (1.0 - nh(pm)) * nh(p) * nh(k));
-  }
-  for (int p = 0; p < nk && kin; ++p) {
-    const int pp = p + q;
-    if (q < max(-p, -k) || q > min(nk - p - 1, nk - k - 1) || pp < 0 || pp >= nk) continue;
-    const double Ed = ((Eh[kq] + Ee[pp]) - Ee[p]) - Eh[k];
-    dh = dh + vsq(0) * lrtz(Ed, b_eh) *
-                  (ne(pp) * (1.0 - ne(p)) * (1.0 - nh(k)) + (1.0 - ne(pp)) * ne(p) * nh(k));
-  }
-  v.De[e] = de * kPi / hb;
-  v.Dh[e] = dh * kPi / hb;
 }
 
 // OffDiagDephasing2 (dephasing.py:320-359): x[kh][ke] = i hbar (sum_q
-// Dh[q][kh] p[kh + q][ke] + sum_q De[q][ke] p[kh][ke + q]), q != 0; one
-// thread per (kh, ke).
-__global__ void mb_offp_kernel(MBView v0) {
+// Dh[q][kh] p[kh + q][ke] + sum_q De[q][ke] p[kh][ke + q]), q != 0: two
+// products of p with the real matrices MH[kh][k'] = Dh[k' - kh][kh] and
+// ME[k'][ke] = De[k' - ke][ke] (zero for k' = kh, ke) on the FP64 matrix
+// instructions.  One CTA per 32 x 32 block, a warp per 16 x 8 of it; per 8
+// values of k' the four operand tiles come through shared memory, read one
+// step ahead.  64 wires of Nk 114: 0.04 ms, 0.23 with a thread per element.
+constexpr int kOT = 32, kOK = 8;
+__global__ void __launch_bounds__(256) mb_offp_kernel(MBView v0) {
   const MBView v = at_wire(v0);
-  const int nk = v.nk, e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nk * nk) return;
-  const int kh = e / nk, ke = e - kh * nk;
+  const int nk = v.nk, nb = (nk + kOT - 1) / kOT, tid = threadIdx.x;
+  const int I0 = (blockIdx.x / nb) * kOT, J0 = (blockIdx.x % nb) * kOT;
+  const int lane = tid & 31, wp = tid >> 5, fr = lane >> 2, fk = lane & 3;
+  // [row][k'] with rows of kOK + 4, [k'][column] with rows of kOT + 2 (p) and
+  // + 4 (ME): no bank conflicts in the fragments
+  __shared__ double mh[kOT][kOK + 4], me[kOK][kOT + 4];
+  __shared__ double2 pi[kOT][kOK + 4], pj[kOK][kOT + 2];
   const double2* p = v.L;
-  double2 x = make_double2(0.0, 0.0);
-  for (int q = -kh; q <= nk - kh - 1; ++q) {
-    const double u = q == 0 ? 0.0 : 1.0;  // undel
-    const double d = v.Dh[(q + nk) * nk + kh];
-    const double2 pv = p[(kh + q) * nk + ke];
-    x = ca(x, make_double2(d * pv.x * u, d * pv.y * u));
+  const double2 z = make_double2(0.0, 0.0);
+  const int lr = tid >> 3, lk = tid & 7, ck = tid >> 5, cc = tid & 31;
+  double nh, ne;
+  double2 npi, npj;
+  auto fetch = [&](int k0) {
+    const int kh = I0 + lr, kr = k0 + lk, kc = k0 + ck, ke = J0 + cc;
+    const bool inr = kh < nk && kr < nk, inc = kc < nk && ke < nk;
+    nh = inr && kr != kh ? v.Dh[(kr - kh + nk) * nk + kh] : 0.0;
+    npi = inr ? p[kh * nk + kr] : z;
+    ne = inc && kc != ke ? v.De[(kc - ke + nk) * nk + ke] : 0.0;
+    npj = inc ? p[kc * nk + ke] : z;
+  };
+  const int wi = (wp & 1) * 16, wj = (wp >> 1) * 8;
+  CAcc acc[2] = {};
+  fetch(0);
+  for (int k0 = 0; k0 < nk; k0 += kOK) {
+    __syncthreads();
+    mh[lr][lk] = nh;
+    pi[lr][lk] = npi;
+    me[ck][cc] = ne;
+    pj[ck][cc] = npj;
+    __syncthreads();
+    if (k0 + kOK < nk) fetch(k0 + kOK);
+#pragma unroll
+    for (int s = 0; s < kOK; s += 4) {
+      const double2 bp = pj[s + fk][wj + fr];
+      const double be = me[s + fk][wj + fr];
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const double ah = mh[wi + 8 * m + fr][s + fk];
+        const double2 ap = pi[wi + 8 * m + fr][s + fk];
+        dmma(acc[m].re, ah, bp.x);
+        dmma(acc[m].im, ah, bp.y);
+        dmma(acc[m].re, ap.x, be);
+        dmma(acc[m].im, ap.y, be);
+      }
+    }
   }
-  for (int q = -ke; q <= nk - ke - 1; ++q) {
-    const double u = q == 0 ? 0.0 : 1.0;
-    const double d = v.De[(q + nk) * nk + ke];
-    const double2 pv = p[kh * nk + ke + q];  // p^T[ke + q][kh]
-    x = ca(x, make_double2(d * pv.x * u, d * pv.y * u));
-  }
-  // x * i * hbar
-  v.OffP[e] = make_double2(-x.y * v.hbar, x.x * v.hbar);
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int kh = I0 + wi + 8 * m + fr, ke = J0 + wj + 2 * fk + c;
+      if (kh < nk && ke < nk)  // x * i * hbar
+        v.OffP[kh * nk + ke] = make_double2(-acc[m].im[c] * v.hbar, acc[m].re[c] * v.hbar);
+    }
 }
 
 // In/out scattering rates of the new occupations (SBESolver._relaxation_E/H,
@@ -1371,6 +1432,22 @@ int launch_derivs(const full::Step& s, int nw, cudaStream_t st) {
   return PSB_OK;
 }
 
+// mb_offd_kernel with 8 wires per CTA where the batch has them
+int launch_offd(const full::MBView& v, int nk, int nw, cudaStream_t st) {
+  const int W = nw >= 4 ? 8 : 1, th = 128;
+  auto kern = W == 8 ? full::mb_offd_kernel<8> : full::mb_offd_kernel<1>;
+  const size_t sm = (size_t)nk * (2 + 2 * W) * 8;
+  if (sm > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(
+        kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess)
+      return set_error(PSB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  }
+  const int nd = (2 * nk + 1) * nk;
+  kern<<<dim3((nd + th - 1) / th, (nw + W - 1) / W), th, sm, st>>>(v, nw);
+  return PSB_OK;
+}
+
 int full_launch(const Launch& a, cudaStream_t st) {
   const int nk = a.nk, nw = a.nw, n2 = nk * nk;
   const PsbFullMB* mb = a.mb;
@@ -1469,14 +1546,16 @@ int full_launch(const Launch& a, cudaStream_t st) {
   }
   // dephasing from the level the right-hand side reads (SBEs.py:5225-5232)
   if (mb && mb->diag_dph) {
-    full::mb_gamma_kernel<<<blk, th, 0, st>>>(v);
+    full::mb_gamma_kernel<<<dim3((nk + full::kGamWarps - 1) / full::kGamWarps, nw),
+                            32 * full::kGamWarps, 0, st>>>(v);
     s.GamE = v.GamE;
     s.GamH = v.GamH;
   }
   if (mb && mb->offdiag_dph) {
-    const int nd = (2 * nk + 1) * nk;
-    full::mb_offd_kernel<<<dim3((nd + th - 1) / th, nw), th, 4 * (size_t)nk * 8, st>>>(v);
-    full::mb_offp_kernel<<<bl, th, 0, st>>>(v);
+    rc_ = launch_offd(v, nk, nw, st);
+    if (rc_ != PSB_OK) return rc_;
+    const int nb = (nk + full::kOT - 1) / full::kOT;
+    full::mb_offp_kernel<<<dim3(nb * nb, nw), 256, 0, st>>>(v);
     s.OffP = v.OffP;
   }
   rc_ = launch_derivs(s, nw, st);
