@@ -661,8 +661,9 @@ struct MBView {
   double2* OffP;
   double2* X3;         // [3][nk][nk]
   double* rates;       // [5][nk]: WinE, WoutE, WinH, WoutH, Rsp
-  double2* shift;      // [nk]: circulant kernel of the DC shift
-  double2* tr;         // [3][nk][nk]: DC-shift intermediate
+  double2* shift;      // [nk]: circulant kernel of the DC shift; before it [2][nk] occupations
+  double2* tr;         // [3][nk][nk]: DC-shift intermediate; before it R1, R2, R4, R3 of
+                       // the scattering rates (5 nk^2 doubles at most)
   double gap;          // J
   int lf;
   // a batch of wires (blockIdx.y): byte strides of V3, the levels, the
@@ -908,14 +909,103 @@ __global__ void __launch_bounds__(256) mb_offp_kernel(MBView v0) {
 }
 
 // In/out scattering rates of the new occupations (SBESolver._relaxation_E/H,
-// SBEs.py:5248-5291): MBCE / MBCH (coulomb.py:957-1071) with |Re n| on the
-// 1-based grid, k3(a, b, c) = a + b - c (1-based, 0 when outside), and the
-// reference's C arrays read at [k - 1][..][..]; then MBPE / MBPH
-// (phonons.py:140-271) with Re n; with recomb also SpontEmission's Rsp.
-// One CTA per (k, wire): the occupations and V^2 in shared memory, threads
-// over the inner index of each double sum (so C[k][q1][q2] is read along
-// q2), block reductions.  The sums run in this tree order, not the
-// reference's sequential one (they agree to rounding).
+// SBEs.py:5248-5291): MBCE / MBCH (coulomb.py:957-1071) with |Re n|, k3(a, b,
+// c) = a + b - c, and the reference's C arrays read at [k - 1][..][..] (its
+// 1-based grid; row 0 of an array is zero); then MBPE / MBPH (phonons.py:
+// 140-271) with Re n; with recomb also SpontEmission's Rsp.
+//
+// The eight double sums are built from four families of single sums,
+//   R1[k][k1] = sum_kp Ceh[k][kp][k1] (1 - nh[kp]) nh[kp + k1 - k]
+//   R2[k][k4] = sum_k2 Cee[k][k2][k4] (1 - ne[k2]) ne[k2 + k - k4]
+//   R4 as R2 with Chh and nh
+//   R3[kp][d] = sum_kk Ceh[kk][kp][kk + d] (1 - ne[kk]) ne[kk + d]
+// e.g. electrons in: sum_k1 Veh^2(k - k1) ne[k1] R1[k][k1] + ..., electrons out:
+// sum_k1 Veh^2(k - k1) (1 - ne[k1]) R1[k1][k] + ....  For a fixed difference d
+// (k1 - k or k4 - k) each family is one matrix product: the slice of C with
+// that difference, the same for every wire, times the occupation products of
+// the batch's wires.  mb_scatter_kernel does these on the FP64 matrix
+// instructions, one CTA per (d, family) and 8 NT wires; mb_rates_kernel adds
+// up per (k, wire).  A wire's column does not depend on the others.  64 wires
+// of Nk 114: 0.14 ms, bound by the strided reads of the slices of C (L2); 1.15
+// with the double sums per (k, wire), which read C once per wire.
+__global__ void mb_occ_kernel(MBView v0) {
+  const MBView v = at_wire(v0);
+  const int nk = v.nk, i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nk) return;
+  double* occ = reinterpret_cast<double*>(v.shift);  // [2][nk], free until the DC shift
+  occ[i] = fabs(v.X3[nk * nk + i * nk + i].x);
+  occ[nk + i] = fabs(v.X3[2 * nk * nk + i * nk + i].x);
+}
+
+constexpr int kScWarps = 8, kScK = 128;  // k values of the occupation products at a time
+// rows of the occupation products: 8 NT wires + 4 (no bank conflicts)
+__host__ __device__ constexpr int sc_ld(int nt) { return 8 * nt + 4; }
+
+template <int NT>
+__global__ void __launch_bounds__(32 * kScWarps) mb_scatter_kernel(MBView v0, int nw) {
+  const int nk = v0.nk, n2 = nk * nk, N1 = nk + 1;
+  const int d = (int)blockIdx.x - (nk - 1), fam = blockIdx.y, w0 = blockIdx.z * 8 * NT;
+  const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5, fr = lane >> 2, fk = lane & 3;
+  extern __shared__ double gsm[];  // [kScK][sc_ld(NT)]
+  const int lo = d < 0 ? -d : 0, hi = d < 0 ? nk : nk - d;  // i with i and i + d on the grid
+  const size_t cs3 = (size_t)N1 * N1 * N1;
+  // families 0, 1, 2: rows k of [lo, hi), summed over all kp; 3: rows kp, over kk
+  const double* C = v0.mb.C + (fam == 1 ? cs3 : (fam == 2 ? 2 * cs3 : 0)) + d;
+  const bool by_row = fam < 3;
+  const int row_lo = by_row ? lo : 0, row_hi = by_row ? hi : nk;
+  const int sum_lo = by_row ? 0 : lo, sum_hi = by_row ? nk : hi;
+  const size_t row_st = by_row ? (size_t)N1 * N1 + 1 : N1;
+  const size_t sum_st = by_row ? N1 : (size_t)N1 * N1 + 1;
+  // partner of i in the occupation products, the occupations it takes
+  const int pd = fam == 1 || fam == 2 ? -d : d, band = fam == 0 || fam == 2 ? 1 : 0;
+  const int tiles = (row_hi - row_lo + 7) / 8, chunks = (sum_hi - sum_lo + kScK - 1) / kScK;
+  for (int t0 = 0; t0 < tiles; t0 += kScWarps) {
+    const int row = row_lo + 8 * (t0 + wp) + fr;
+    double acc[NT][2];
+#pragma unroll
+    for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = 0.0;
+    for (int c = 0; c < chunks; ++c) {
+      const int s0 = sum_lo + c * kScK, sn = min(kScK, sum_hi - s0);
+      if (t0 == 0 || chunks > 1) {
+        __syncthreads();
+        for (int e = tid; e < kScK * 8 * NT; e += 32 * kScWarps) {
+          const int w = e / kScK, i = e % kScK, k = s0 + i, r = k + pd;
+          double g = 0.0;
+          if (i < sn && r >= 0 && r < nk && w0 + w < nw) {
+            const double* o = reinterpret_cast<const double*>(
+                                  bump(v0.shift, (int64_t)(w0 + w) * v0.st_sc)) + band * nk;
+            g = (1.0 - o[k]) * o[r];
+          }
+          gsm[i * sc_ld(NT) + w] = g;
+        }
+        __syncthreads();
+      }
+      if (t0 + wp >= tiles) continue;
+      const double* a = C + (size_t)row * row_st + (size_t)(s0 + fk) * sum_st;
+      const bool in = row < row_hi;
+#pragma unroll 8
+      for (int k = 0; k < sn; k += 4) {
+        const double x = in && k + fk < sn ? a[(size_t)k * sum_st] : 0.0;
+        const double* b = gsm + (k + fk) * sc_ld(NT) + fr;
+#pragma unroll
+        for (int n = 0; n < NT; ++n) dmma(acc[n], x, b[8 * n]);
+      }
+    }
+    if (row >= row_hi || t0 + wp >= tiles) continue;
+    // families 0, 1, 2 at [k][k + d], family 3 at [kp][d + nk - 1]
+    const size_t o = (size_t)fam * n2 +
+                     (by_row ? (size_t)row * nk + row + d : (size_t)row * (2 * nk - 1) + blockIdx.x);
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int w = w0 + 8 * n + 2 * fk + u;
+        if (w < nw)
+          reinterpret_cast<double*>(bump(v0.tr, (int64_t)w * v0.st_sc))[o] = acc[n][u];
+      }
+  }
+}
+
 constexpr int kRateThreads = 128;
 
 // sum of K values over the CTA (kRateThreads threads); every thread gets them
@@ -940,82 +1030,29 @@ __device__ __forceinline__ void rate_block_sum(double (&v)[K], double (*red)[kRa
 __global__ void __launch_bounds__(kRateThreads) mb_rates_kernel(MBView v0) {
   const MBView v = at_wire(v0);
   const int nk = v.nk, k0 = blockIdx.x;
-  const int n2 = nk * nk, N1 = nk + 1;
-  extern __shared__ double sm[];
-  double* ne1 = sm;             // [nk + 1] |Re n_e|, 1-based, [0] = 0
-  double* nh1 = ne1 + N1;       // [nk + 1]
-  double* v2 = nh1 + N1;        // [3][nk] V(q)^2
-  __shared__ double red[5][kRateThreads / 32];
+  const int n2 = nk * nk;
+  __shared__ double red[4][kRateThreads / 32];
   const double2* C3 = v.X3 + n2;
   const double2* D3 = v.X3 + 2 * n2;
-  for (int i = threadIdx.x; i <= nk; i += kRateThreads) {
-    ne1[i] = i == 0 ? 0.0 : fabs(C3[(i - 1) * nk + i - 1].x);
-    nh1[i] = i == 0 ? 0.0 : fabs(D3[(i - 1) * nk + i - 1].x);
-  }
-  for (int i = threadIdx.x; i < 3 * nk; i += kRateThreads) {
-    const double x = v.V3[i];
-    v2[i] = x * x;
-  }
-  __syncthreads();
-  auto k3 = [&](int a, int b, int c) {  // 0-based arguments, 1-based result
-    const int r = (a + 1) + (b + 1) - (c + 1);
-    return (r < 1 || r > nk) ? 0 : r;
-  };
-  auto vv2 = [&](int t, int a, int b) { return v2[t * nk + (a > b ? a - b : b - a)]; };
-  const size_t cs3 = (size_t)N1 * N1 * N1;
-  const double* Ceh = v.mb.C;
-  const double* Cee = Ceh + cs3;
-  const double* Chh = Ceh + 2 * cs3;
-  auto cix = [&](int a, int b, int c) { return ((size_t)a * N1 + b) * N1 + c; };
   double acc[4] = {0.0, 0.0, 0.0, 0.0};  // WinE, WoutE, WinH, WoutH
   if (v.mb.ehs) {
-    const int k = k0 + 1;  // MBCE: k; MBCH: kp
-    // two q1 per iteration keep twice the C reads in flight (each
-    // accumulator still adds in q1 order)
-#pragma unroll 2
-    for (int q1 = 1; q1 <= nk; ++q1) {
-      for (int q2 = threadIdx.x + 1; q2 <= nk; q2 += kRateThreads) {
-        {  // electrons (MBCE)
-          const int kp = q1, k1 = q2;
-          int r = k3(kp - 1, k1 - 1, k - 1);
-          if (r > 0)
-            acc[0] += vv2(0, k - 1, k1 - 1) * (1.0 - nh1[kp]) * nh1[r] * ne1[k1] *
-                      Ceh[cix(k - 1, kp - 1, k1 - 1)];
-          r = k3(kp - 1, k - 1, k1 - 1);
-          if (r > 0)
-            acc[1] += vv2(0, k1 - 1, k - 1) * (1.0 - ne1[k1]) * (1.0 - nh1[kp]) * nh1[r] *
-                      Ceh[cix(k1 - 1, kp - 1, k - 1)];
-          const int k2 = q1, k4 = q2;
-          r = k3(k - 1, k2 - 1, k4 - 1);
-          if (r > 0)
-            acc[0] += vv2(1, k - 1, k4 - 1) * (1.0 - ne1[k2]) * ne1[r] * ne1[k4] *
-                      Cee[cix(k - 1, k2 - 1, k4 - 1)];
-          r = k3(k4 - 1, k2 - 1, k - 1);
-          if (r > 0)
-            acc[1] += vv2(1, k4 - 1, k - 1) * (1.0 - ne1[k4]) * (1.0 - ne1[k2]) * ne1[r] *
-                      Cee[cix(k4 - 1, k2 - 1, k - 1)];
-        }
-        {  // holes (MBCH): kp is this CTA's momentum
-          const int kp = k, kk = q1, k1 = q2;
-          int r = k3(kp - 1, k1 - 1, kk - 1);
-          if (r > 0)
-            acc[2] += vv2(0, kk - 1, k1 - 1) * (1.0 - ne1[kk]) * nh1[r] * ne1[k1] *
-                      Ceh[cix(kk - 1, kp - 1, k1 - 1)];
-          r = k3(kp - 1, kk - 1, k1 - 1);
-          if (r > 0)
-            acc[3] += vv2(0, k1 - 1, kk - 1) * (1.0 - ne1[kk]) * (1.0 - nh1[r]) * ne1[k1] *
-                      Ceh[cix(kk - 1, r - 1, k1 - 1)];
-          const int k2p = q1, k4p = q2;
-          r = k3(kp - 1, k2p - 1, k4p - 1);
-          if (r > 0)
-            acc[2] += vv2(2, kp - 1, k4p - 1) * (1.0 - nh1[k2p]) * nh1[r] * nh1[k4p] *
-                      Chh[cix(kp - 1, k2p - 1, k4p - 1)];
-          r = k3(k4p - 1, k2p - 1, kp - 1);
-          if (r > 0)
-            acc[3] += vv2(2, k4p - 1, kp - 1) * (1.0 - nh1[k4p]) * (1.0 - nh1[k2p]) * nh1[r] *
-                      Chh[cix(k4p - 1, k2p - 1, kp - 1)];
-        }
-      }
+    const double* R1 = reinterpret_cast<const double*>(v.tr);
+    const double* R2 = R1 + n2;
+    const double* R4 = R2 + n2;
+    const double* R3 = R4 + n2;
+    const double* ne = reinterpret_cast<const double*>(v.shift);
+    const double* nh = ne + nk;
+    for (int i = threadIdx.x; i < nk; i += kRateThreads) {
+      const int q = i > k0 ? i - k0 : k0 - i;
+      const double veh = v.V3[q], vee = v.V3[nk + q], vhh = v.V3[2 * nk + q];
+      const double eh2 = veh * veh, ee2 = vee * vee, hh2 = vhh * vhh;
+      const int a = k0 * nk + i, b = i * nk + k0;
+      // MBCE: from i into k0, from k0 into i
+      acc[0] += ne[i] * (eh2 * R1[a] + ee2 * R2[a]);
+      acc[1] += (1.0 - ne[i]) * (eh2 * R1[b] + ee2 * R2[b]);
+      // MBCH: the partner hole at i = kp + d, and at i = kp - d
+      acc[2] += nh[i] * (eh2 * R3[k0 * (2 * nk - 1) + i - k0 + nk - 1] + hh2 * R4[a]);
+      acc[3] += (1.0 - nh[i]) * (eh2 * R3[i * (2 * nk - 1) + k0 - i + nk - 1] + hh2 * R4[b]);
     }
   }
   rate_block_sum<4>(acc, red);
@@ -1448,6 +1485,27 @@ int launch_offd(const full::MBView& v, int nk, int nw, cudaStream_t st) {
   return PSB_OK;
 }
 
+// mb_scatter_kernel for batches of up to 64 wires a CTA
+template <int NT>
+int launch_scatter_nt(const full::MBView& v, int nk, int nw, cudaStream_t st) {
+  const size_t sm = (size_t)full::kScK * full::sc_ld(NT) * 8;
+  if (sm > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(
+        full::mb_scatter_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess)
+      return set_error(PSB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  }
+  full::mb_scatter_kernel<NT>
+      <<<dim3(2 * nk - 1, 4, (nw + 8 * NT - 1) / (8 * NT)), 32 * full::kScWarps, sm, st>>>(v, nw);
+  return PSB_OK;
+}
+int launch_scatter(const full::MBView& v, int nk, int nw, cudaStream_t st) {
+  if (nw <= 8) return launch_scatter_nt<1>(v, nk, nw, st);
+  if (nw <= 16) return launch_scatter_nt<2>(v, nk, nw, st);
+  if (nw <= 32) return launch_scatter_nt<4>(v, nk, nw, st);
+  return launch_scatter_nt<8>(v, nk, nw, st);
+}
+
 int full_launch(const Launch& a, cudaStream_t st) {
   const int nk = a.nk, nw = a.nw, n2 = nk * nk;
   const PsbFullMB* mb = a.mb;
@@ -1564,8 +1622,12 @@ int full_launch(const Launch& a, cudaStream_t st) {
     // X3's occupations relaxed (SBEs.py:5688-5695) and shifted by the DC field
     // (SBEs.py:5698-5702), then the rescale
     if (relax) {
-      const size_t smr = (2 * (size_t)(nk + 1) + 3 * (size_t)nk) * 8;
-      full::mb_rates_kernel<<<dim3(nk, nw), full::kRateThreads, smr, st>>>(v);
+      if (mb->ehs) {
+        full::mb_occ_kernel<<<blk, th, 0, st>>>(v);
+        rc_ = launch_scatter(v, nk, nw, st);
+        if (rc_ != PSB_OK) return rc_;
+      }
+      full::mb_rates_kernel<<<dim3(nk, nw), full::kRateThreads, 0, st>>>(v);
       full::mb_relax_kernel<<<blk, th, 0, st>>>(v, a.params->dt);
     }
     if (dct) {
