@@ -249,8 +249,9 @@ class WireBatch:
 
     def rhs(self, stream=None):
         dy = torch.empty_like(self.y)
+        flags = self.tab_flags | (abi.PSB_TAB_ONE_CLASS if len(self.classes) == 1 else 0)
         _lib.call("psb_rhs_f64", *self._common(), device.ptr(self.y), device.ptr(dy),
-                  self.n_state, self.nkmax, self.tab_flags, abi.as_ptr(self.model),
+                  self.n_state, self.nkmax, flags, abi.as_ptr(self.model),
                   device.stream_ptr(stream))
         return dy
 

@@ -396,30 +396,28 @@ constexpr int kLfThreads = 256;
 __global__ void __launch_bounds__(kLfThreads) occ_sums_kernel(Step s0) {
   const Step s = at_wire(s0);
   const int nk = s.nk, n2 = nk * nk;
-  __shared__ double red[2][kLfThreads / 32];
+  __shared__ double red_e[kLfThreads], red_h[kLfThreads];
   double se = 0.0, sh = 0.0;
   for (int k = threadIdx.x; k < nk; k += kLfThreads) {
     const double2 c3 = s.X3[n2 + k * nk + k], d3 = s.X3[2 * n2 + k * nk + k];
     se += hypot(c3.x, c3.y);
     sh += hypot(d3.x, d3.y);
   }
-  se = warp_sum(se);
-  sh = warp_sum(sh);
-  if ((threadIdx.x & 31) == 0) {
-    red[0][threadIdx.x >> 5] = se;
-    red[1][threadIdx.x >> 5] = sh;
-  }
+  red_e[threadIdx.x] = se;
+  red_h[threadIdx.x] = sh;
   __syncthreads();
+  for (int o = kLfThreads / 2; o > 0; o >>= 1) {
+    if (threadIdx.x < o) {
+      red_e[threadIdx.x] += red_e[threadIdx.x + o];
+      red_h[threadIdx.x] += red_h[threadIdx.x + o];
+    }
+    __syncthreads();
+  }
   if (threadIdx.x == 0) {
     const double small = 1e-200;
-    se = sh = 0.0;
-    for (int i = 0; i < kLfThreads / 32; ++i) {
-      se += red[0][i];
-      sh += red[1][i];
-    }
-    s.fac[0] = (se + sh) / 2.0;
-    s.fac[1] = se + small;
-    s.fac[2] = sh + small;
+    s.fac[0] = (red_e[0] + red_h[0]) / 2.0;
+    s.fac[1] = red_e[0] + small;
+    s.fac[2] = red_h[0] + small;
   }
 }
 
@@ -1158,85 +1156,99 @@ __global__ void mb_relax_kernel(MBView v0, double dt) {
 // (dcfield.py:1169-1211), i.e. a circular convolution with
 //   s[d] = (1/nk) sum_m exp(-i Y_m dk) exp(2 pi i m d / nk),
 // applied along both indices of each matrix (lf) or to its diagonal.
-__global__ void mb_shift_kernel(MBView v0) {
+// One CTA per wire: the phases exp(-i Y_m dk) and the roots of nk in shared
+// memory, thread d sums over m (64 wires of Nk 114: 0.01 ms; 0.06 with both
+// evaluated per (m, d)).
+constexpr int kShThreads = 128;
+__global__ void __launch_bounds__(kShThreads) mb_shift_kernel(MBView v0) {
   const MBView v = at_wire(v0);
-  const int nk = v.nk, d = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d >= nk) return;
-  double re = 0.0, im = 0.0;
-  for (int m = 0; m < nk; ++m) {
-    double sy, cy, sw, cw;
-    sincos(-v.mb.Y[m] * v.mb.dc_dk, &sy, &cy);
-    const int r = (int)(((long long)m * d) % nk);
-    sincospi(2.0 * r / nk, &sw, &cw);
-    re += cy * cw - sy * sw;
-    im += cy * sw + sy * cw;
+  const int nk = v.nk;
+  extern __shared__ double2 shs[];  // [nk] phases, [nk] roots
+  for (int i = threadIdx.x; i < nk; i += kShThreads) {
+    sincos(-v.mb.Y[i] * v.mb.dc_dk, &shs[i].y, &shs[i].x);
+    sincospi(2.0 * i / nk, &shs[nk + i].y, &shs[nk + i].x);
   }
-  v.shift[d] = make_double2(re / nk, im / nk);
+  __syncthreads();
+  for (int d = threadIdx.x; d < nk; d += kShThreads) {
+    double re = 0.0, im = 0.0;
+    int r = 0;  // m d mod nk
+    for (int m = 0; m < nk; ++m) {
+      const double cy = shs[m].x, sy = shs[m].y, cw = shs[nk + r].x, sw = shs[nk + r].y;
+      re += fma(cy, cw, -__dmul_rn(sy, sw));  // (rounding: see cm_rn)
+      im += fma(cy, sw, __dmul_rn(sy, cw));
+      r += d;
+      if (r >= nk) r -= nk;
+    }
+    v.shift[d] = make_double2(re / nk, im / nk);
+  }
 }
 
-// The two circulant products of the shift, tiled: one CTA per kST x kST
-// block of one matrix (x) of one wire; per chunk of kST summation indices
-// the block's operand tile and the 2 kST - 1 coefficients s[(j - b) mod nk]
-// it needs sit in shared memory.  Each element sums in the old order (the
-// summation index ascending).
-constexpr int kST = 16;
+// The complex product with its rounding spelled out: a caller's charge density
+// is the difference of two densities of the shifted C and D and cancels to the
+// last digits, so their bits stay.
+__device__ __forceinline__ double2 cm_rn(double2 a, double2 b) {
+  return make_double2(fma(a.x, b.x, -__dmul_rn(a.y, b.y)), fma(a.y, b.x, __dmul_rn(a.x, b.y)));
+}
 
-// T[x][a][j] = sum_b X3[x][a][b] s[(j - b) mod nk]
-__global__ void __launch_bounds__(kST* kST) mb_shift_rows_kernel(MBView v0) {
+// The two circulant products of the shift, tiled: one CTA per 32 x 32 block of
+// one matrix (x) of one wire, a warp per 8 rows, a lane per column; per chunk
+// of kST summation indices the block's operand tile and the coefficients s[(j -
+// b) mod nk] it needs sit in shared memory, and a lane's eight sums share the
+// operand that varies along the columns (the other is a broadcast).  Bound by
+// the FP64 pipe.  Each element sums with the summation index ascending.
+// 64 wires of Nk 114: 0.12 ms each, 0.23 with one element per thread.
+constexpr int kST = 16, kSB = 32, kSR = 8, kSThreads = kSB / kSR * 32;
+
+// ROWS: T[x][a][j] = sum_b X3[x][a][b] s[(j - b) mod nk], into tr;
+// else X3[x][i][j] = sum_a s[(i - a) mod nk] T[x][a][j], into X3
+template <bool ROWS>
+__global__ void __launch_bounds__(kSThreads) mb_shift_mat_kernel(MBView v0) {
   const MBView v = at_wire(v0);
-  const int nk = v.nk, n2 = nk * nk, nb = (nk + kST - 1) / kST;
+  const int nk = v.nk, n2 = nk * nk, nb = (nk + kSB - 1) / kSB;
   const int x = blockIdx.x / (nb * nb), t = blockIdx.x % (nb * nb);
-  const int A0 = (t / nb) * kST, J0 = (t % nb) * kST;
-  const int tx = threadIdx.x % kST, ty = threadIdx.x / kST;
-  __shared__ double2 xt[kST][kST + 1];
-  __shared__ double2 sv[2 * kST - 1];
-  const double2* X = v.X3 + (size_t)x * n2;
-  const int a = A0 + ty, j = J0 + tx;
-  double2 acc = make_double2(0.0, 0.0);
+  const int I0 = (t / nb) * kSB, J0 = (t % nb) * kSB;
+  const int tid = threadIdx.x, lane = tid & 31, r0 = (tid >> 5) * kSR;
+  __shared__ double2 xt[ROWS ? kSB : kST][ROWS ? kST + 1 : kSB + 1];
+  __shared__ double2 sv[kSB + kST - 1];
+  const double2* X = (ROWS ? v.X3 : v.tr) + (size_t)x * n2;
+  double2 acc[kSR];
+#pragma unroll
+  for (int r = 0; r < kSR; ++r) acc[r] = make_double2(0.0, 0.0);
+  const int S0 = ROWS ? J0 : I0;  // output index the coefficients run over
   for (int b0 = 0; b0 < nk; b0 += kST) {
-    const int r = A0 + ty, c = b0 + tx;
-    xt[ty][tx] = (r < nk && c < nk) ? X[r * nk + c] : make_double2(0.0, 0.0);
-    if (threadIdx.x < 2 * kST - 1) {
-      // sv[u] = s[(J0 - b0 - (kST - 1) + u) mod nk]
-      int d = (J0 - b0 - (kST - 1) + (int)threadIdx.x) % nk;
+    for (int e = tid; e < kSB * kST; e += kSThreads) {
+      const int er = ROWS ? e / kST : e / kSB, ec = ROWS ? e % kST : e % kSB;
+      const int r = (ROWS ? I0 : b0) + er, c = (ROWS ? b0 : J0) + ec;
+      xt[er][ec] = (r < nk && c < nk) ? X[r * nk + c] : make_double2(0.0, 0.0);
+    }
+    for (int u = tid; u < kSB + kST - 1; u += kSThreads) {
+      // sv[u] = s[(S0 - b0 - (kST - 1) + u) mod nk]
+      int d = (S0 - b0 - (kST - 1) + u) % nk;
       if (d < 0) d += nk;
-      sv[threadIdx.x] = v.shift[d];
+      sv[u] = v.shift[d];
     }
     __syncthreads();
     const int bn = min(kST, nk - b0);
-    for (int bb = 0; bb < bn; ++bb) acc = ca(acc, cm(xt[ty][bb], sv[tx - bb + kST - 1]));
+    if (I0 + r0 < nk)
+      for (int bb = 0; bb < bn; ++bb) {
+        if (ROWS) {
+          const double2 c = sv[lane - bb + kST - 1];
+#pragma unroll
+          for (int r = 0; r < kSR; ++r) acc[r] = ca(acc[r], cm_rn(xt[r0 + r][bb], c));
+        } else {
+          const double2 c = xt[bb][lane];
+#pragma unroll
+          for (int r = 0; r < kSR; ++r) acc[r] = ca(acc[r], cm_rn(sv[r0 + r - bb + kST - 1], c));
+        }
+      }
     __syncthreads();
   }
-  if (a < nk && j < nk) v.tr[(size_t)x * n2 + a * nk + j] = acc;
-}
-
-// X3[x][i][j] = sum_a s[(i - a) mod nk] T[x][a][j]
-__global__ void __launch_bounds__(kST* kST) mb_shift_cols_kernel(MBView v0) {
-  const MBView v = at_wire(v0);
-  const int nk = v.nk, n2 = nk * nk, nb = (nk + kST - 1) / kST;
-  const int x = blockIdx.x / (nb * nb), t = blockIdx.x % (nb * nb);
-  const int I0 = (t / nb) * kST, J0 = (t % nb) * kST;
-  const int tx = threadIdx.x % kST, ty = threadIdx.x / kST;
-  __shared__ double2 tt[kST][kST + 1];
-  __shared__ double2 sv[2 * kST - 1];
-  const double2* T = v.tr + (size_t)x * n2;
-  const int i = I0 + ty, j = J0 + tx;
-  double2 acc = make_double2(0.0, 0.0);
-  for (int a0 = 0; a0 < nk; a0 += kST) {
-    const int r = a0 + ty, c = J0 + tx;
-    tt[ty][tx] = (r < nk && c < nk) ? T[r * nk + c] : make_double2(0.0, 0.0);
-    if (threadIdx.x < 2 * kST - 1) {
-      // sv[u] = s[(I0 - a0 - (kST - 1) + u) mod nk]
-      int d = (I0 - a0 - (kST - 1) + (int)threadIdx.x) % nk;
-      if (d < 0) d += nk;
-      sv[threadIdx.x] = v.shift[d];
-    }
-    __syncthreads();
-    const int an = min(kST, nk - a0);
-    for (int aa = 0; aa < an; ++aa) acc = ca(acc, cm(sv[ty - aa + kST - 1], tt[aa][tx]));
-    __syncthreads();
+  double2* out = (ROWS ? v.tr : v.X3) + (size_t)x * n2;
+#pragma unroll
+  for (int r = 0; r < kSR; ++r) {
+    const int i = I0 + r0 + r, j = J0 + lane;
+    if (i < nk && j < nk) out[i * nk + j] = acc[r];
   }
-  if (i < nk && j < nk) v.X3[(size_t)x * n2 + i * nk + j] = acc;
 }
 
 // without lf only the diagonals move: T[x][a] = sum_n s[(a - n) mod nk] X3[x][n][n]
@@ -1631,12 +1643,12 @@ int full_launch(const Launch& a, cudaStream_t st) {
       full::mb_relax_kernel<<<blk, th, 0, st>>>(v, a.params->dt);
     }
     if (dct) {
-      full::mb_shift_kernel<<<blk, th, 0, st>>>(v);
+      full::mb_shift_kernel<<<one, full::kShThreads, (size_t)2 * nk * 16, st>>>(v);
       if (a.params->lf) {
-        const int nb = (nk + full::kST - 1) / full::kST;
+        const int nb = (nk + full::kSB - 1) / full::kSB;
         const dim3 bt(3 * nb * nb, nw);
-        full::mb_shift_rows_kernel<<<bt, full::kST * full::kST, 0, st>>>(v);
-        full::mb_shift_cols_kernel<<<bt, full::kST * full::kST, 0, st>>>(v);
+        full::mb_shift_mat_kernel<true><<<bt, full::kSThreads, 0, st>>>(v);
+        full::mb_shift_mat_kernel<false><<<bt, full::kSThreads, 0, st>>>(v);
       } else {
         const dim3 bd((3 * nk + th - 1) / th, nw);
         full::mb_shift_diag_kernel<<<bd, th, 0, st>>>(v);
