@@ -79,9 +79,7 @@ __device__ __forceinline__ uint32_t x_off(int k, int col, uint32_t sbo) {
   return (uint32_t)((col >> 3) * sbo + (k >> 4) * 128 + (col & 7) * 16 + (k & 15));
 }
 
-// MMA-issuing warps: one thread issues a tcgen05.mma only every ~100-120
-// cycles whatever N is (measured on B200, M = 128, K = 32 int8, N <= 128),
-// so a group of 4 wires (N = 16, the narrowest MMAs) splits the K slices of
+// MMA-issuing warps: a group of 4 wires (N = 16, the narrowest MMAs) splits the K slices of
 // every row tile between two issuing warps, each into its own partial
 // accumulators, which the epilogue adds (exact int32 sums).  Wider groups
 // keep one issuer: their accumulators leave no tensor memory for a second
@@ -511,12 +509,14 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsLow));
     if (warp < kMmaWarp + NI) {
     // ---- MMA issuers ----------------------------------------------------------
-    // The whole warp polls the barriers (uniform control flow) and lane 0
-    // alone issues the MMAs and commits.  One thread issues every MMA, and
-    // these narrow MMAs are short, so the issuing thread's own instructions
-    // between them set the rate: a barrier poll whose result it branches on
-    // stalls the issue for ~150-180 cycles (measured), about the time of
-    // three MMAs.  So the MMAs of a row tile (persistent A) or of a group of
+    // One thread polls the barriers, issues every MMA and commits.  It is
+    // chosen by elect.sync, inside whose branch the compiler knows that one
+    // lane is active: it keeps descriptors and TMEM addresses in uniform
+    // registers.  (Behind a lane == 0 test it converted them at each MMA and
+    // the issue took ~100-120 cycles; per stage, W = 8: Nk 1024 50.9 -> 42.6
+    // us, Nk 512 18.5 -> 17.9, Nk 256 6.3 -> 6.05; W = 4, Nk 512: 11.3 ->
+    // 10.2.)  A barrier poll stalls the issue for about the time of three
+    // MMAs, so the MMAs of a row tile (persistent A) or of a group of
     // streamed slots go out in one unbroken sequence, with one poll before
     // it; descriptors and TMEM addresses advance incrementally.
     // With NI = 2 issuer ik takes the slices kj = ik (mod 2) of every row
@@ -524,29 +524,19 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
     // group (and both release it), so the generators keep filling one
     // buffer while the issuers read the other.
     const int ik = warp - kMmaWarp;
-    const bool issuer = lane == 0;
-    uint32_t it = 0;  // row tiles issued
-    int gb = 0;       // streamed group buffer of the next slices (two of G slots)
-    uint32_t gph = 0; // parity of that buffer's current fill
     const int G = nslot / 2;
-    auto warp_wait = [&](uint64_t* bar, uint32_t parity) -> bool {
-      const bool got = mbar_wait(bar, parity, abort, a.spin_limit);
-      return __all_sync(0xffffffffu, got);
-    };
-    // (an abort is seen through the stage-end snapshot and inside every
-    // wait, so the stage start needs no vote of its own)
+    const int ng = (nK + G - 1) / G;  // streamed groups of a row tile
     for (int s = 0; s < total_stages; ++s) {
-      {
-        bool ok = !(s == 0 && persist) || warp_wait(&afull[0], 0);
+      if (elect_one()) {
+        bool ok = !(s == 0 && persist) || mbar_wait(&afull[0], 0, abort, a.spin_limit);
         tc_fence_after();
         // B descriptor of X[s & 1] at k' = 0; +32 per 64-wide slice, +16 per
         // K step (start address in 16-byte units: 256 B per 32 k')
         const uint64_t bdesc0 = smem_desc(smem_u32(xbase + (s & 1) * L.xbuf), 128, xsbo);
-        for (int mi = 0; ok && mi < nM; ++mi, ++it) {
+        for (int mi = 0; ok && mi < nM; ++mi) {
+          const uint32_t it = (uint32_t)s * nM + mi;  // row tiles issued before this one
           const int b = it & 1;
-          // every lane polls; the vote on the outcome comes at the tile end
-          if (it >= 2 && !mbar_wait(&dfree[b], ((it >> 1) - 1) & 1, abort, a.spin_limit))
-            ok = false;
+          if (it >= 2 && !mbar_wait(&dfree[b], ((it >> 1) - 1) & 1, abort, a.spin_limit)) break;
           tc_fence_after();
           const uint32_t d2 = tmem + (uint32_t)(3 * N * (b * NI + ik));
           const uint32_t d3 = d2 + (uint32_t)N;
@@ -561,51 +551,32 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
             umma_i8(d3, a1 + kPlaneCols + 8, bd + 16, idesc2, 1);
             umma_i8(d4, a1 + 2 * kPlaneCols + 8, bd + 16, idesc1, 1);
           };
-          uint64_t bd = bdesc0;
           if (persist) {
             // persistent slot of slice kj is 2 mi - kj + nK - 1
-            if (issuer && ok) {
-              uint32_t a1 = tmem + acol0 + (uint32_t)((2 * mi + nK - 1 - ik) * kTileCols);
-              bd += 32 * ik;
-              for (int kj = ik; kj < nK; kj += NI, a1 -= NI * kTileCols, bd += 32 * NI)
-                slice(a1, bd, kj != ik);
-            }
+            uint32_t a1 = tmem + acol0 + (uint32_t)((2 * mi + nK - 1 - ik) * kTileCols);
+            uint64_t bd = bdesc0 + 32 * ik;
+            for (int kj = ik; kj < nK; kj += NI, a1 -= NI * kTileCols, bd += 32 * NI)
+              slice(a1, bd, kj != ik);
           } else {
-            // streamed: slices k0 .. k0 + gn - 1 sit in slots gb G .. gb G + gn - 1.
-            // Every lane polls the group and the warp reconverges after it
-            // (so no lane can fall a buffer cycle behind and test a parity
-            // that has come round again), but it votes on the outcome only
-            // once per row tile: a vote costs the issuing lane about as much
-            // as the poll.
-            bool first = true;  // this issuer's first slice of the row tile
-            for (int k0 = 0; ok && k0 < nK; k0 += G, bd += 32 * G) {
+            // streamed: group g's slices k0 .. k0 + gn - 1 sit in the slots
+            // of buffer gb, filled for the (gi >> 1)-th time
+            uint32_t gi = it * (uint32_t)ng;
+            for (int k0 = 0; k0 < nK; k0 += G, ++gi) {
+              const int gb = gi & 1;
               const int gn = min(G, nK - k0);
-              if (!mbar_wait(&afull[gb], gph, abort, a.spin_limit)) {
-                ok = false;
-                break;
-              }
+              ok = mbar_wait(&afull[gb], (gi >> 1) & 1u, abort, a.spin_limit);
+              if (!ok) break;
               tc_fence_after();
-              if (issuer) {
-                uint32_t a1 = tmem + acol0 + (uint32_t)(gb * G * kTileCols);
-                uint64_t bj = bd;
-                for (int j = 0; j < gn; ++j, a1 += kTileCols, bj += 32) {
-                  if (((k0 + j) & (NI - 1)) != ik) continue;
-                  slice(a1, bj, !first);
-                  first = false;
-                }
-                umma_commit(&afree[gb]);  // the group's slots are reusable once these finish
-              }
-              __syncwarp();
-              if (++gb == 2) {
-                gb = 0;
-                gph ^= 1u;
-              }
+              const int j0 = NI == 1 ? 0 : ((ik - k0) & (NI - 1));
+              uint32_t a1 = tmem + acol0 + (uint32_t)((gb * G + j0) * kTileCols);
+              uint64_t bj = bdesc0 + 32 * (uint64_t)(k0 + j0);
+              for (int j = j0; j < gn; j += NI, a1 += NI * kTileCols, bj += 32 * NI)
+                slice(a1, bj, k0 + j != ik);
+              umma_commit(&afree[gb]);  // the group's slots are reusable once these finish
             }
+            if (!ok) break;
           }
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-          if (issuer) umma_commit(&dfull[b]);  // the row tile is ready to drain
-          __syncwarp();
+          umma_commit(&dfull[b]);  // the row tile is ready to drain
         }
       }
       __syncwarp();
@@ -901,7 +872,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
 
   // ---- teardown -----------------------------------------------------------------
   // every MMA of every issuer has completed before TMEM is released
-  if (warp >= kMmaWarp && warp < kMmaWarp + NI && lane == 0) umma_commit(final_bar);
+  if (warp >= kMmaWarp && warp < kMmaWarp + NI && elect_one()) umma_commit(final_bar);
   if (warp == kMmaWarp && lane == 0) {
     bool done = false;
     for (uint32_t i = 0; i < kSpinLimit && !done; ++i) done = mbar_try_wait(final_bar, 0);

@@ -511,37 +511,34 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
     // (mod 4) of every (row tile, k' slice) pair of a tile: two K steps,
     // three digit planes per pair, into that row tile's own accumulator.
     // Every issuer commits each group (afree) and each item (dfull), so
-    // those barriers expect kIssuers arrivals.  Lane 0 issues.
+    // those barriers expect kIssuers arrivals.  One elected lane issues (see split_rk4_kernel).
     const int ik = warp - kMmaWarp;
-    const bool issuer = lane == 0;
-    uint32_t it = 0;
-    int gb = 0;
-    uint32_t gph = 0;
-    bool go = true;
     const uint64_t bdesc0 = smem_desc(smem_u32(xbase), kSeqBlock, 128);
-    for (int s = 0; s < total_stages && go; ++s) {
-      for (int j = 0; j < nw && go; ++j, ++it) {
-        const int b = it & 1;
-        bool w8 = true;
-        if (s >= 1) w8 = mbar_wait_sleep(&xfull[j], (s - 1) & 1, abort, lim);
-        if (w8 && it >= 2) w8 = mbar_wait_sleep(&dfree[b], ((it >> 1) - 1) & 1, abort, lim);
-        go = __all_sync(0xffffffffu, w8);
-        if (!go) break;
-        tc_fence_after();
-        const uint32_t dbase = tmem + (uint32_t)b * dstride;
-        // descriptor start addresses count 16-byte units
-        const uint64_t bwire = bdesc0 + (uint64_t)(((uint32_t)(j * NT) * L.seq) >> 4);
-        for (int d0 = dmin; d0 <= dmax; d0 += G) {
-          const int gn = min(G, dmax - d0 + 1);
-          go = __all_sync(0xffffffffu, mbar_wait_sleep(&afull[gb], gph, abort, lim));
+    if (elect_one()) {
+      uint32_t it = 0;  // items issued
+      uint32_t gi = 0;  // groups issued: buffer gi & 1, filled for the (gi >> 1)-th time
+      bool go = true;
+      for (int s = 0; s < total_stages && go; ++s) {
+        for (int j = 0; j < nw && go; ++j, ++it) {
+          const int b = it & 1;
+          if (s >= 1) go = mbar_wait_sleep(&xfull[j], (s - 1) & 1, abort, lim);
+          if (go && it >= 2) go = mbar_wait_sleep(&dfree[b], ((it >> 1) - 1) & 1, abort, lim);
           if (!go) break;
           tc_fence_after();
-          if (issuer) {
+          const uint32_t dbase = tmem + (uint32_t)b * dstride;
+          // descriptor start addresses count 16-byte units
+          const uint64_t bwire = bdesc0 + (uint64_t)(((uint32_t)(j * NT) * L.seq) >> 4);
+          for (int d0 = dmin; d0 <= dmax; d0 += G, ++gi) {
+            const int gb = gi & 1;
+            const int gn = min(G, dmax - d0 + 1);
+            go = mbar_wait_sleep(&afull[gb], (gi >> 1) & 1u, abort, lim);
+            if (!go) break;
+            tc_fence_after();
             for (int jj = 0; jj < gn; ++jj) {
               const int d = d0 + jj;
               const int mlo = max(0, (d + 1) >> 1), mhi = min(nM - 1, (d + nK - 1) >> 1);
               // first row tile >= mlo of this issuer
-              const int m0 = mlo + ((ik - mlo) % kIssuers + kIssuers) % kIssuers;
+              const int m0 = mlo + ((ik - mlo) & (kIssuers - 1));
               const uint32_t aslot = tmem + acol0 + (uint32_t)((gb * G + jj) * NT * kTileCols);
 #pragma unroll
               for (int t = 0; t < NT; ++t) {
@@ -567,17 +564,12 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
             }
             umma_commit(&afree[gb]);  // the group's slots are free once these finish
           }
-          __syncwarp();
-          if (++gb == 2) {
-            gb = 0;
-            gph ^= 1u;
-          }
+          if (!go) break;
+          umma_commit(&dfull[b]);  // this issuer's accumulators are complete
         }
-        if (!go) break;
-        if (issuer) umma_commit(&dfull[b]);  // this issuer's accumulators are complete
-        __syncwarp();
       }
     }
+    __syncwarp();
   } else if (warp >= kGenWarp0) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsLow));
     // ---- A-tile generators: row r = 32 gq + lane of tile d is a(64 d + r - c),
@@ -886,7 +878,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
 
   // ---- teardown -----------------------------------------------------------------
   // every MMA of every issuer has completed before TMEM is released
-  if (warp >= kMmaWarp && lane == 0) umma_commit(final_bar);
+  if (warp >= kMmaWarp && elect_one()) umma_commit(final_bar);
   if (warp == kMmaWarp && lane == 0) {
     bool done = false;
     for (uint32_t i = 0; i < kSpinLimit && !done; ++i) done = mbar_try_wait(final_bar, 0);
