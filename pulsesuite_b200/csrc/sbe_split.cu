@@ -39,38 +39,81 @@
 //     X[s & 1] while its epilogue writes the digits of the next stage point
 //     into X[(s+1) & 1], with each column's scale taken from the previous
 //     stage's column maximum and one bit of headroom; a column whose values
-//     outgrow that headroom is re-digitised with its exact scale at the end
-//     of the stage;
+//     outgrow that headroom is re-digitised with its exact scale before the
+//     next stage's MMAs;
 //   * T is Toeplitz and never stored as a matrix: each 128 x 64 tile of the
 //     A operand (three digit planes) is generated straight into tensor
 //     memory by four generator warps from tables of digit quads
 //     (a(d), a(d-1), a(d-2), a(d-3)) in shared memory -- one 32-bit lookup
 //     per TMEM cell.  A tile depends only on 2 mi - kj (mi the row tile, kj
 //     the 64-wide k' slice); when all distinct tiles fit in tensor memory
-//     they are generated once per call, else they stream through a double
-//     buffer;
-//   * one thread issues tcgen05.mma (M = 128, N = 4W, K = 32), six digit
-//     products per K step, into the three accumulators of a row tile; the
-//     accumulators are double buffered per row tile, so the epilogue of
-//     tile mi overlaps the MMAs of tile mi + 1;
-//   * eight drain/epilogue warps read a finished tile's accumulators and
+//     they are generated once per call, else each is generated once per
+//     stage and used for all its (mi, kj) pairs when every row tile can have
+//     its accumulators, else they stream row tile by row tile (Feed);
+//   * one thread issues tcgen05.mma (M = 128, N = 4W .. 12W, K = 32), six
+//     digit products per K step, into the three accumulators of a row tile,
+//     so the epilogue of tile mi overlaps the MMAs of later tiles;
+//   * sixteen drain/epilogue warps read a finished tile's accumulators and
 //     evaluate the diagonal SBE right-hand side and the RK4 stage
-//     combination (stage order of libpulsesuite/integrator.py:143-157);
+//     combination (stage order of libpulsesuite/integrator.py:143-157); one
+//     warp evaluates the wires' drives a stage ahead;
 //   * the per-element state (y FP64, FP32 copy of y, stage point and
 //     accumulator FP32) stays
 //     in shared memory for the whole call when it fits (psb_split_max_nk_
 //     resident), else in the caller's workspace.
+// What bounds it (B200, full waves of CTAs): the epilogue's instructions
+// (~250 an element and warp, half of a stage at Nk 256, W = 8) and the serial
+// chain of a stage: its last digits -> barrier -> first row tile's MMAs ->
+// drain, ~1.5 us; at Nk > 512 the generation of the tiles (~550 cycles
+// each).  The tensor cores run ~15 % of the time.  us per stage of a CTA,
+// before (8 epilogue warps, MMAs issued behind a lane test, two issuers at
+// W = 4, streamed tiles by row, drive and scales inside the stage's chain)
+// and now:
+//   Nk        64    128    256    512   1024
+//   W = 4   2.09   2.41   3.92  11.32   35.1
+//           1.70   1.96   3.15   7.55   21.0
+//   W = 8   3.16   3.76   6.27  18.52   50.9
+//           2.52   2.94   5.15  14.54   40.6
+//   W = 16  6.30   6.69  16.87  37.41
+//           4.03   4.70  12.11  26.00
+// Tried and slower: 8 epilogue warps with twice the registers (Nk 256, W = 8:
+// 5.9), column maxima by redux.sync (~32 cycles each: Nk 64, W = 16 4.07 to
+// 4.58) or by votes against the last exponent (+4 %), band energies loaded at
+// the row tile's start (Nk 256 +2 %).
 // Every mbarrier wait is bounded; on a timeout the CTA records
 // PSB_ERR_TIMEOUT in its wires' status, waits for its MMAs, frees TMEM and
 // returns.
 #include <math.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "split_common.cuh"
 
 namespace psb {
 namespace split {
+
+constexpr int kEpiWarps = 16;   // warps 0..15: drain + epilogue (warpgroups 0..3)
+constexpr int kGenWarp0 = 16;   // warps 16..19: A-tile generators
+constexpr int kGenWarps = 4;
+constexpr int kMmaWarp = 20;    // warp 20: TMEM owner + MMA issuer
+constexpr int kDriveWarp = 21;  // warp 21: the wires' drives of the next stage
+                                // (22, 23 only complete that warpgroup)
+constexpr int kThreadsS = 32 * 24;
+constexpr int kEpiThreads = 32 * kEpiWarps;
+constexpr int kStageThreads = kEpiThreads + 64;  // epilogue, issuer and drive warps
+// Registers per thread: 80 at launch (65536 / 768 threads, a multiple of 8);
+// after the set-up the generator and MMA warpgroups give theirs down to
+// kRegsGen and kRegsMma and the four epilogue warpgroups take them, no more
+// in all than the launch holds, so the increase always finds its registers.
+// (The generators want 32 words in flight: 56 against 48 registers is Nk
+// 1024, W = 8 46.8 -> 40.6 us per stage; 88 for the epilogue costs W = 16 7 %.)
+constexpr int kRegsLaunch = 80;
+constexpr int kRegsGen = 56;
+constexpr int kRegsMma = 40;
+constexpr int kRegsHigh = 96;
+static_assert(kEpiWarps * kRegsHigh + 4 * kRegsGen + 4 * kRegsMma <= 24 * kRegsLaunch,
+              "register split exceeds the launch allocation");
 
 // Byte offset of element (k, col) in one digit plane of X (K-major: 16 k of
 // a column contiguous in a core-matrix row, 8 columns per core matrix; core
@@ -79,33 +122,39 @@ __device__ __forceinline__ uint32_t x_off(int k, int col, uint32_t sbo) {
   return (uint32_t)((col >> 3) * sbo + (k >> 4) * 128 + (col & 7) * 16 + (k & 15));
 }
 
-// MMA-issuing warps: a group of 4 wires (N = 16, the narrowest MMAs) splits the K slices of
-// every row tile between two issuing warps, each into its own partial
-// accumulators, which the epilogue adds (exact int32 sums).  Wider groups
-// keep one issuer: their accumulators leave no tensor memory for a second
-// set.
-__host__ __device__ constexpr int issuers_of(int n) { return n == 16 ? 2 : 1; }
-// TMEM columns: two row-tile buffers of issuers_of(n) accumulator sets
-// (D2, D3, D4: 3 N each), then the A slots (3 digit planes): all distinct
-// tiles when they fit (persistent), else streamed slots in the remaining
-// columns (up to kMaxSlots), used as two buffers of nslot / 2 slots: the
-// generators fill one group while the MMAs read the other.
+// TMEM columns: accumulator sets of a row tile (D2, D3, D4: 3 N columns), then
+// the A slots (3 digit planes each), in one of three arrangements:
+//   kAll     every distinct tile has its slot, written once per call; two
+//            accumulator sets, so a row tile's drain overlaps the next one's
+//            MMAs;
+//   kByTile  the distinct tiles stream through the slots, each generated
+//            once per stage and used for all the (row tile, slice) pairs it
+//            serves; every row tile has its accumulator set;
+//   kByRow   what is too large for that: the tiles of each row tile stream
+//            through the slots; two accumulator sets.
+// Streamed slots are two buffers of nslot / 2: the generators fill one group
+// while the MMAs read the other.
 constexpr int kMaxSlots = 8;
-__host__ __device__ inline int acc_cols(int n) { return 6 * n * issuers_of(n); }
-__host__ __device__ inline bool persistent_tiles(int nk, int n) {
-  return acc_cols(n) + kTileCols * ntiles_of(nk) <= kTmemCols;
+enum class Feed { kAll, kByTile, kByRow };
+__host__ __device__ inline Feed feed_of(int nk, int n) {
+  if (6 * n + kTileCols * ntiles_of(nk) <= kTmemCols) return Feed::kAll;
+  return 3 * n * mtiles_of(nk) + 2 * kTileCols <= kTmemCols ? Feed::kByTile : Feed::kByRow;
 }
-__host__ __device__ inline int ring_slots(int n) {
-  const int r = (kTmemCols - acc_cols(n)) / kTileCols;
+__host__ __device__ inline int acc_cols(int nk, int n) {
+  return feed_of(nk, n) == Feed::kByTile ? 3 * n * mtiles_of(nk) : 6 * n;
+}
+__host__ __device__ inline int ring_slots(int nk, int n) {
+  const int r = (kTmemCols - acc_cols(nk, n)) / kTileCols;
   return r < kMaxSlots ? r : kMaxSlots;
 }
 __host__ __device__ inline int tmem_cols(int nk, int n) {
-  const int slots = persistent_tiles(nk, n) ? ntiles_of(nk) : ring_slots(n);
-  const int need = acc_cols(n) + kTileCols * slots;
+  const int slots = feed_of(nk, n) == Feed::kAll ? ntiles_of(nk) : ring_slots(nk, n);
+  const int need = acc_cols(nk, n) + kTileCols * slots;
   int c = 32;
   while (c < need) c <<= 1;
   return c;
 }
+constexpr int kMaxAcc = PSB_MAX_NK / kTileRows;  // accumulator sets
 
 struct Args {
   const PsbTable* tables;
@@ -149,13 +198,13 @@ struct Layout {
     ntab_words = kTileRows * nM + kpad;
     bars = tab + kDigits * 4 * (uint32_t)ntab_words;  // digit-quad tables
     bars = (bars + 15) & ~15u;
-    misc = bars + 8 * 24;  // afull[8], afree[8], dfull[2], dfree[2], final
+    misc = bars + 8 * 28;  // afull[8], afree[8], dfull[8], dfree[2], final
     // misc: tmem base (16 B), abort + snapshots (16 B), pulse constants
     // double[W][2][4], wire params double4[W], t double[W], off int64[W],
     // P partials double[2][4][W], X column decode factors float[2][N],
     // column maxima float[4][N], column write scales float[N], column
     // overflow flags int[2][N], gap/hbar double[W]
-    total = misc + 32 + 328 * W + 16;  // + any-overflow flags int[2]
+    total = misc + 32 + 344 * W + 16;  // drive float2[2][W]; any-overflow flags int[2]
   }
 };
 
@@ -165,8 +214,7 @@ struct Layout {
 template <int W, bool RES>
 __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
   constexpr int N = 4 * W;
-  constexpr int NI = issuers_of(N);  // MMA-issuing warps (kMmaWarp ..)
-  constexpr int WH = W / 2;  // wires per drain/epilogue warp
+  constexpr int WH = W / 4;  // wires per drain/epilogue warp
   extern __shared__ __align__(1024) uint8_t smem[];
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
@@ -195,8 +243,8 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
   }
   const int nk = tb.nk, kpad = kpad_of(nk), nM = mtiles_of(nk), nK = kpad / kTileK;
   const Layout<W, RES> L(nk);
-  const bool persist = persistent_tiles(nk, N);
-  const int nslot = ring_slots(N);  // streamed A slots
+  const Feed feed = feed_of(nk, N);
+  const int nslot = ring_slots(nk, N);  // streamed A slots
   const int ntile = ntiles_of(nk);
   uint8_t* xbase = smem;  // X[b] digit plane p at xbase + b xbuf + p plane
   double4* s_y = reinterpret_cast<double4*>(smem + L.st);
@@ -207,7 +255,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
   uint64_t* afull = reinterpret_cast<uint64_t*>(smem + L.bars);
   uint64_t* afree = afull + kMaxSlots;
   uint64_t* dfull = afree + kMaxSlots;
-  uint64_t* dfree = dfull + 2;
+  uint64_t* dfree = dfull + kMaxAcc;
   uint64_t* final_bar = dfree + 2;  // teardown: all MMAs of this CTA done
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L.misc);
   volatile int* abort = reinterpret_cast<volatile int*>(smem + L.misc + 16);
@@ -224,7 +272,8 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
   float* scw = reinterpret_cast<float*>(smem + L.misc + 32 + 272 * W);     // [N]
   int* ovf = reinterpret_cast<int*>(smem + L.misc + 32 + 288 * W);         // [2][N]
   double* gaph = reinterpret_cast<double*>(smem + L.misc + 32 + 320 * W);  // [W]
-  volatile int* ovf_any = reinterpret_cast<volatile int*>(smem + L.misc + 32 + 328 * W);  // [2]
+  volatile int* ovf_any = reinterpret_cast<volatile int*>(smem + L.misc + 32 + 344 * W);  // [2]
+  float2* drv = reinterpret_cast<float2*>(smem + L.misc + 32 + 328 * W);  // [2][W] M(t)/hbar
   const double inv_hbar = 1.0 / a.hbar;
   const uint32_t xsbo = (uint32_t)kpad * 8;
   const double* blk = a.tabdata + tb.off;
@@ -244,13 +293,11 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
   if (tid == 0) {
     for (int b = 0; b < kMaxSlots; ++b) {
       mbar_init(&afull[b], kGenWarps);
-      mbar_init(&afree[b], NI);
+      mbar_init(&afree[b], 1);
     }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&dfull[b], NI);
-      mbar_init(&dfree[b], kEpiWarps);
-    }
-    mbar_init(final_bar, NI);
+    for (int b = 0; b < kMaxAcc; ++b) mbar_init(&dfull[b], 1);
+    for (int b = 0; b < 2; ++b) mbar_init(&dfree[b], kEpiWarps);
+    mbar_init(final_bar, 1);
     *abort = 0;
     snap[0] = 0;
     snap[1] = 0;
@@ -299,7 +346,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
   const uint32_t tmem = *tmem_slot;
   // TMEM column map: accumulator set b at 3 N b (D2, D3, D4 at +0, +N,
   // +2N); A slot i at acol0 + kTileCols i (digit plane p at + kPlaneCols p).
-  const uint32_t acol0 = (uint32_t)acc_cols(N);
+  const uint32_t acol0 = (uint32_t)acc_cols(nk, N);
   double vmax = 0.0;
 #pragma unroll
   for (int i = 0; i < kThreadsS / 32; ++i) vmax = fmax(vmax, vmax_w[i]);
@@ -339,42 +386,35 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
   // warp (q, hh): rows 128 mi + 32 q + lane (q = TMEM lane quarter), wires
   // w0 .. w0 + WH - 1.
   const int q = warp & 3;
-  const int hh = (warp >> 2) & 1;
+  const int hh = (warp >> 2) & 3;
   const int w0 = hh * WH;
   double4* g_y = reinterpret_cast<double4*>(a.y);
-  // Largest |value| of each of this warp's X columns, per lane quarter q.
-  // Halving butterfly (colmax_halve): the 4 WH columns need 4 WH shuffles
-  // in all, not 5 per column; afterwards lane L holds column
-  // (L >> (5 - m)) & (4 WH - 1), m = log2(4 WH).
-  auto publish_colmax = [&](const float* cm) {
-    constexpr int C = 4 * WH;  // 8, 16 or 32
-    static_assert(C == 8 || C == 16 || C == 32, "column count of a drain warp");
-    float v[C];
+  // Values of C columns combined over the warp's lanes by halving (C / 2 + C / 4
+  // + .. exchanges, then one a level): lane L ends with column L / (32 / C).
+  auto halve = [&](auto* v, auto C_, auto op) {
+    constexpr int C = decltype(C_)::value;
 #pragma unroll
-    for (int c = 0; c < C; ++c) v[c] = cm[c];
-    if constexpr (C == 32) {
-      // five halvings leave lane L with column L
-      colmax_halve<32>(v, 16, lane);
-      colmax_halve<16>(v, 8, lane);
-      colmax_halve<8>(v, 4, lane);
-      colmax_halve<4>(v, 2, lane);
-      colmax_halve<2>(v, 1, lane);
-      colmax[q * N + 4 * w0 + lane] = v[0];
-    } else if constexpr (C == 16) {
-      colmax_halve<16>(v, 16, lane);
-      colmax_halve<8>(v, 8, lane);
-      colmax_halve<4>(v, 4, lane);
-      colmax_halve<2>(v, 2, lane);
-      v[0] = fmaxf(v[0], __shfl_xor_sync(0xffffffffu, v[0], 1));
-      if ((lane & 1) == 0) colmax[q * N + 4 * w0 + ((lane >> 1) & 15)] = v[0];
-    } else {
-      colmax_halve<8>(v, 16, lane);
-      colmax_halve<4>(v, 8, lane);
-      colmax_halve<2>(v, 4, lane);
-      v[0] = fmaxf(v[0], __shfl_xor_sync(0xffffffffu, v[0], 2));
-      v[0] = fmaxf(v[0], __shfl_xor_sync(0xffffffffu, v[0], 1));
-      if ((lane & 3) == 0) colmax[q * N + 4 * w0 + ((lane >> 2) & 7)] = v[0];
+    for (int o = 16, n = C; o > 0; o >>= 1) {
+      if (n > 1) {
+        n >>= 1;
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < C / 2; ++i) {
+          if (i >= n) break;
+          const auto send = up ? v[i] : v[i + n];
+          const auto keep = up ? v[i + n] : v[i];
+          v[i] = op(keep, __shfl_xor_sync(0xffffffffu, send, o));
+        }
+      } else {
+        v[0] = op(v[0], __shfl_xor_sync(0xffffffffu, v[0], o));
+      }
     }
+  };
+  // Largest |value| of each of this warp's X columns, per lane quarter q.
+  auto publish_colmax = [&](float* cm) {
+    constexpr int C = 4 * WH;
+    halve(cm, std::integral_constant<int, C>{}, [](float x, float y) { return fmaxf(x, y); });
+    if (lane % (32 / C) == 0) colmax[q * N + 4 * w0 + lane / (32 / C)] = cm[0];
   };
   auto track = [&](float* cm, int j, float4 v) {
     cm[4 * j + 0] = fmaxf(cm[4 * j + 0], fabsf(v.x));
@@ -411,11 +451,12 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
     return min(max(-1 - e2, -120), 120);
   };
   auto sexp_lag = [](float m) -> int {
-    int e2 = 0;
     if (!(m > 0.f) || !isfinite(m)) return -2;
-    frexpf(m, &e2);
+    // m < 2^e2; a subnormal's smaller exponent meets the same clamp
+    const int e2 = (int)(__float_as_uint(m) >> 23) - 126;
     return min(max(-2 - e2, -120), 120);
   };
+  auto pow2 = [](int e) { return __uint_as_float((uint32_t)(127 + e) << 23); };  // |e| <= 120
   // Decode factor of a column digitised with scale 2^sexp: exchange sum / hbar
   // = VS / (hbar 254^2) 2^-sexp (D2 + (D3 + D4/254)/254).
   const double dec0 = VS * inv_hbar / (kBase * kBase);
@@ -459,8 +500,8 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
   auto set_write_scales = [&](int b) {
     if (tid < N) {
       const int sexp = sexp_lag(col_max(tid));
-      scw[tid] = ldexpf(1.f, sexp);
-      xfach[b * N + tid] = ldexpf(dec0f, -sexp);
+      scw[tid] = pow2(sexp);
+      xfach[b * N + tid] = dec0f * pow2(-sexp);
     }
   };
 
@@ -492,101 +533,151 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
     publish_colmax(cm0);
     named_sync(2, kEpiThreads);
     x_pass(0, false);
-    set_write_scales(1);
     fence_async_smem();
   }
+  // Drive of a stage as M/hbar, by one warp: lane 2w + j evaluates pulse j of
+  // wire w at that stage's time, the two added in order.
+  const double h = a.dt;
+  double tj = warp == kDriveWarp && lane < 2 * W ? wt[lane >> 1] : 0.0;
+  auto drive = [&](int s) {
+    const int stg = s & 3;
+    const double t = tj + (stg == 0 ? 0.0 : (stg == 3 ? h : h / 2.0));
+    const double* pc = pulse + (lane < 2 * W ? 4 * lane : 0);
+    const double u = t - pc[0];
+    const double env = exp(pc[1] * u * u);
+    double mr = 0.0, mim = 0.0;
+    if ((lane & 1) == 0) {
+      mr = __fma_rn(pc[2], env, mr);
+      mim = __fma_rn(pc[3], env, mim);
+    }
+    mr = __shfl_sync(0xffffffffu, mr, lane & 30);
+    mim = __shfl_sync(0xffffffffu, mim, lane & 30);
+    if ((lane & 1) && lane < 2 * W) {
+      mr = __fma_rn(pc[2], env, mr);
+      mim = __fma_rn(pc[3], env, mim);
+      drv[(s & 1) * W + (lane >> 1)] =
+          make_float2((float)(mr * inv_hbar), (float)(mim * inv_hbar));
+    }
+  };
+  if (warp == kDriveWarp) drive(0);
   __syncthreads();
 
   static_assert(3 * N <= 256, "stacked MMA width 3N must be <= 256");
   const uint32_t idesc1 = idesc_i8(N), idesc2 = idesc_i8(2 * N), idesc3 = idesc_i8(3 * N);
   const int total_stages = a.nsteps * 4;
-  const double h = a.dt;
 
   // Roles.  Each warpgroup changes its register allocation once, at the top
-  // of its branch (all four warps at the same instruction): warpgroups 2
-  // and 3 down to kRegsLow, the epilogue warpgroups 0 and 1 up to kRegsHigh.
+  // of its branch (all four warps at the same instruction): warpgroups 4
+  // and 5 down to kRegsGen and kRegsMma, the epilogue's 0 to 3 up to
+  // kRegsHigh.
   if (warp >= kMmaWarp) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsLow));
-    if (warp < kMmaWarp + NI) {
-    // ---- MMA issuers ----------------------------------------------------------
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsMma));
+    if (warp == kMmaWarp) {
+    // ---- MMA issuer -----------------------------------------------------------
     // One thread polls the barriers, issues every MMA and commits.  It is
     // chosen by elect.sync, inside whose branch the compiler knows that one
     // lane is active: it keeps descriptors and TMEM addresses in uniform
-    // registers.  (Behind a lane == 0 test it converted them at each MMA and
-    // the issue took ~100-120 cycles; per stage, W = 8: Nk 1024 50.9 -> 42.6
-    // us, Nk 512 18.5 -> 17.9, Nk 256 6.3 -> 6.05; W = 4, Nk 512: 11.3 ->
-    // 10.2.)  A barrier poll stalls the issue for about the time of three
-    // MMAs, so the MMAs of a row tile (persistent A) or of a group of
-    // streamed slots go out in one unbroken sequence, with one poll before
-    // it; descriptors and TMEM addresses advance incrementally.
-    // With NI = 2 issuer ik takes the slices kj = ik (mod 2) of every row
-    // tile into accumulator set ik; with streamed A both issuers read every
-    // group (and both release it), so the generators keep filling one
-    // buffer while the issuers read the other.
-    const int ik = warp - kMmaWarp;
+    // registers and the MMAs go out at the tensor cores' rate (N = 32: 32
+    // cycles a piece of a slice; behind a lane == 0 test it converted them at
+    // each MMA, 54 cycles and more).  A barrier poll stalls the issue for
+    // about the time of three MMAs, so the MMAs of a row tile (kAll) or of a
+    // group of streamed slots go out in one unbroken sequence, with one poll
+    // before it.
     const int G = nslot / 2;
-    const int ng = (nK + G - 1) / G;  // streamed groups of a row tile
+    const int ng = feed == Feed::kByTile ? (ntile + G - 1) / G : (nK + G - 1) / G;
     for (int s = 0; s < total_stages; ++s) {
+      // the last stage's digits outgrew a scale: wait for the epilogue's
+      // second pass
+      if (s > 0 && ovf_any[s & 1]) named_sync(3, kEpiThreads + 32);
       if (elect_one()) {
-        bool ok = !(s == 0 && persist) || mbar_wait(&afull[0], 0, abort, a.spin_limit);
-        tc_fence_after();
         // B descriptor of X[s & 1] at k' = 0; +32 per 64-wide slice, +16 per
         // K step (start address in 16-byte units: 256 B per 32 k')
         const uint64_t bdesc0 = smem_desc(smem_u32(xbase + (s & 1) * L.xbuf), 128, xsbo);
-        for (int mi = 0; ok && mi < nM; ++mi) {
-          const uint32_t it = (uint32_t)s * nM + mi;  // row tiles issued before this one
-          const int b = it & 1;
-          if (it >= 2 && !mbar_wait(&dfree[b], ((it >> 1) - 1) & 1, abort, a.spin_limit)) break;
-          tc_fence_after();
-          const uint32_t d2 = tmem + (uint32_t)(3 * N * (b * NI + ik));
-          const uint32_t d3 = d2 + (uint32_t)N;
-          const uint32_t d4 = d2 + (uint32_t)(2 * N);
-          // one 64-wide K slice: K step 0 (the tile's first slice overwrites
-          // its accumulators), then K step 1
-          auto slice = [&](uint32_t a1, uint64_t bd, bool acc) {
-            umma_i8(d2, a1, bd, idesc3, acc);                // T1 [X1|X2|X3] -> D2|D3|D4
-            umma_i8(d3, a1 + kPlaneCols, bd, idesc2, 1);     // T2 [X1|X2] -> D3|D4
-            umma_i8(d4, a1 + 2 * kPlaneCols, bd, idesc1, 1); // T3 X1 -> D4
-            umma_i8(d2, a1 + 8, bd + 16, idesc3, 1);
-            umma_i8(d3, a1 + kPlaneCols + 8, bd + 16, idesc2, 1);
-            umma_i8(d4, a1 + 2 * kPlaneCols + 8, bd + 16, idesc1, 1);
-          };
-          if (persist) {
-            // persistent slot of slice kj is 2 mi - kj + nK - 1
-            uint32_t a1 = tmem + acol0 + (uint32_t)((2 * mi + nK - 1 - ik) * kTileCols);
-            uint64_t bd = bdesc0 + 32 * ik;
-            for (int kj = ik; kj < nK; kj += NI, a1 -= NI * kTileCols, bd += 32 * NI)
-              slice(a1, bd, kj != ik);
-          } else {
-            // streamed: group g's slices k0 .. k0 + gn - 1 sit in the slots
-            // of buffer gb, filled for the (gi >> 1)-th time
-            uint32_t gi = it * (uint32_t)ng;
-            for (int k0 = 0; k0 < nK; k0 += G, ++gi) {
-              const int gb = gi & 1;
-              const int gn = min(G, nK - k0);
-              ok = mbar_wait(&afull[gb], (gi >> 1) & 1u, abort, a.spin_limit);
-              if (!ok) break;
-              tc_fence_after();
-              const int j0 = NI == 1 ? 0 : ((ik - k0) & (NI - 1));
-              uint32_t a1 = tmem + acol0 + (uint32_t)((gb * G + j0) * kTileCols);
-              uint64_t bj = bdesc0 + 32 * (uint64_t)(k0 + j0);
-              for (int j = j0; j < gn; j += NI, a1 += NI * kTileCols, bj += 32 * NI)
-                slice(a1, bj, k0 + j != ik);
-              umma_commit(&afree[gb]);  // the group's slots are reusable once these finish
+        // one 64-wide K slice into the accumulator set at d2: K step 0 (the
+        // row tile's first slice overwrites its accumulators), then K step 1
+        auto slice = [&](uint32_t d2, uint32_t a1, uint64_t bd, bool acc) {
+          const uint32_t d3 = d2 + (uint32_t)N, d4 = d2 + (uint32_t)(2 * N);
+          umma_i8(d2, a1, bd, idesc3, acc);                // T1 [X1|X2|X3] -> D2|D3|D4
+          umma_i8(d3, a1 + kPlaneCols, bd, idesc2, 1);     // T2 [X1|X2] -> D3|D4
+          umma_i8(d4, a1 + 2 * kPlaneCols, bd, idesc1, 1); // T3 X1 -> D4
+          umma_i8(d2, a1 + 8, bd + 16, idesc3, 1);
+          umma_i8(d3, a1 + kPlaneCols + 8, bd + 16, idesc2, 1);
+          umma_i8(d4, a1 + 2 * kPlaneCols + 8, bd + 16, idesc1, 1);
+        };
+        auto slot = [&](int i) { return tmem + acol0 + (uint32_t)(i * kTileCols); };
+        tc_fence_after();
+        if (feed == Feed::kByTile) {
+          // tiles dl = 2 mi - kj upwards: row tile mi's slices come in the
+          // order kj = nK - 1 .. 0, so it is complete after tile 2 mi (the
+          // accumulators were drained before the last stage end)
+          uint32_t gi = (uint32_t)s * ng;  // groups before this one
+          for (int i0 = 0; i0 < ntile; i0 += G, ++gi) {
+            const int gb = gi & 1;
+            const int gn = min(G, ntile - i0);
+            if (!mbar_wait(&afull[gb], (gi >> 1) & 1u, abort, a.spin_limit)) break;
+            tc_fence_after();
+            for (int j = 0; j < gn; ++j) {
+              const int dl = i0 + j - (nK - 1);
+              const int m0 = max(0, (dl + 1) >> 1), m1 = min(nM - 1, (dl + nK - 1) >> 1);
+              const uint32_t a1 = slot(gb * G + j);
+              uint32_t d2 = tmem + (uint32_t)(3 * N * m0);
+              uint64_t bd = bdesc0 + 32 * (uint64_t)(2 * m0 - dl);
+              for (int kj = 2 * m0 - dl; kj <= 2 * m1 - dl; kj += 2, d2 += 3 * N, bd += 64)
+                slice(d2, a1, bd, kj != nK - 1);
+              if (dl >= 0 && (dl & 1) == 0) umma_commit(&dfull[dl >> 1]);
             }
-            if (!ok) break;
+            umma_commit(&afree[gb]);  // the group's slots are reusable once these finish
           }
-          umma_commit(&dfull[b]);  // the row tile is ready to drain
+        } else {
+          bool ok = feed != Feed::kAll || s > 0 || mbar_wait(&afull[0], 0, abort, a.spin_limit);
+          tc_fence_after();
+          for (int mi = 0; ok && mi < nM; ++mi) {
+            const uint32_t it = (uint32_t)s * nM + mi;  // row tiles before this one
+            const int b = it & 1;
+            // (what the last stage left was drained before its end)
+            if (mi >= 2 && !mbar_wait(&dfree[b], ((it >> 1) - 1) & 1, abort, a.spin_limit)) break;
+            tc_fence_after();
+            const uint32_t d2 = tmem + (uint32_t)(3 * N * b);
+            if (feed == Feed::kAll) {
+              // the slot of slice kj is 2 mi - kj + nK - 1
+              for (int kj = 0; kj < nK; ++kj)
+                slice(d2, slot(2 * mi + nK - 1 - kj), bdesc0 + 32 * (uint64_t)kj, kj != 0);
+            } else {
+              // group g's slices k0 .. k0 + gn - 1 sit in the slots of buffer
+              // gb, filled for the (gi >> 1)-th time
+              uint32_t gi = it * (uint32_t)ng;
+              for (int k0 = 0; k0 < nK; k0 += G, ++gi) {
+                const int gb = gi & 1;
+                const int gn = min(G, nK - k0);
+                ok = mbar_wait(&afull[gb], (gi >> 1) & 1u, abort, a.spin_limit);
+                if (!ok) break;
+                tc_fence_after();
+                for (int j = 0; j < gn; ++j)
+                  slice(d2, slot(gb * G + j), bdesc0 + 32 * (uint64_t)(k0 + j), k0 + j != 0);
+                umma_commit(&afree[gb]);
+              }
+              if (!ok) break;
+            }
+            umma_commit(&dfull[b]);  // the row tile is ready to drain
+          }
         }
       }
       __syncwarp();
       // wait for the epilogue to publish the next stage's X
-      named_sync(1, kEpiThreads + 32 * NI);
+      named_sync(1, kStageThreads);
       if (snap[s & 1]) break;
     }
+    } else if (warp == kDriveWarp) {
+      for (int s = 0; s < total_stages; ++s) {
+        if ((s & 3) == 3) tj = tj + h;
+        if (s + 1 < total_stages) drive(s + 1);
+        named_sync(1, kStageThreads);
+        if (snap[s & 1]) break;
+      }
+      if (lane < 2 * W && (lane & 1) == 0 && !*abort) wt[lane >> 1] = tj;
     }
   } else if (warp >= kGenWarp0) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsLow));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsGen));
     // ---- A-tile generators ------------------------------------------------------
     // Row r = 32 gq + lane of the tile for 2 mi - kj = dl is a(d0 - c),
     // c = 0..63, d0 = 64 dl + r; TMEM column j of a digit plane holds
@@ -596,36 +687,46 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
       const int base = 64 * dl + 32 * gq + lane - dlo;
       const uint32_t ta = tmem + ((uint32_t)(32 * gq) << 16) + acol0 +
                           (uint32_t)(slot * kTileCols);
+      // (two planes' words in flight)
+      uint32_t r0[16], r1[16];
+      auto load = [&](int p, uint32_t* r) {
+        const uint32_t* t = tabq + p * L.ntab_words + base;
 #pragma unroll
-      for (int p = 0; p < kDigits; ++p) {
-        uint32_t r[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) r[j] = tabq[p * L.ntab_words + base - 4 * j];
-        tmem_st16(ta + p * kPlaneCols, r);
-      }
+        for (int j = 0; j < 16; ++j) r[j] = t[-4 * j];
+      };
+      load(0, r0);
+      load(1, r1);
+      tmem_st16(ta, r0);
+      load(2, r0);
+      tmem_st16(ta + kPlaneCols, r1);
+      tmem_st16(ta + 2 * kPlaneCols, r0);
     };
-    if (persist) {
+    if (feed == Feed::kAll) {
       for (int sl = 0; sl < ntile; ++sl) gen_tile(sl - (nK - 1), sl);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&afull[0]);
     } else {
-      // the issuer's group sequence: per row tile, slices in groups of at
-      // most G, alternating between two buffers of G slots
+      // the issuer's group sequence: the distinct tiles of a stage (kByTile)
+      // or the slices of each of its row tiles, in groups of at most G,
+      // alternating between two buffers of G slots
       const int G = nslot / 2;
+      const int nrow = feed == Feed::kByTile ? 1 : nM;
+      const int nsl = feed == Feed::kByTile ? ntile : nK;
       int gb = 0;           // group buffer of the next group
       uint32_t gph = 0;     // parity of that buffer's current fill
       bool first = true;    // first pass over both buffers: nothing to wait for
       for (int s = 0; s < total_stages && !*abort; ++s) {
-        for (int mi = 0; mi < nM && !*abort; ++mi) {
-          for (int k0 = 0; k0 < nK; k0 += G) {
-            const int gn = min(G, nK - k0);
+        for (int mi = 0; mi < nrow && !*abort; ++mi) {
+          for (int k0 = 0; k0 < nsl; k0 += G) {
+            const int gn = min(G, nsl - k0);
             bool got = first || mbar_wait(&afree[gb], gph ^ 1u, abort, a.spin_limit);
             got = __all_sync(0xffffffffu, got);
             if (!got) break;
             tc_fence_after();
-            for (int j = 0; j < gn; ++j) gen_tile(2 * mi - (k0 + j), gb * G + j);
+            for (int j = 0; j < gn; ++j)
+              gen_tile(feed == Feed::kByTile ? k0 + j - (nK - 1) : 2 * mi - (k0 + j), gb * G + j);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             tc_fence_before();
             __syncwarp();
@@ -646,30 +747,73 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
     const uint32_t lrow = tmem + ((uint32_t)(32 * q) << 16);
     const float inv_base = 1.f / 254.f;
     const float hf = (float)h, h2f = (float)(h / 2.0), h6f = (float)(h / 6.0);
-    // lane j < WH keeps the time of wire w0 + j
-    double tj = (lane < WH) ? wt[w0 + lane] : 0.0;
+    bool done = true;
+    double ee = 0.0, eh = 0.0;  // Ee, Eh of this lane's row in the next row tile
+    auto band = [&](int mi) {
+      const int k = mi * kTileRows + 32 * q + lane;
+      if (k < nk) {
+        ee = Ee[k];
+        eh = Eh[k];
+      }
+    };
+    band(0);
+    // sums of p over this warp's rows at the end of a step: per wire re, im
+    double pp[2 * WH];
+#pragma unroll
+    for (int c = 0; c < 2 * WH; ++c) pp[c] = 0.0;
+    auto sum_p = [&]() {
+      constexpr int C = 2 * WH;
+      halve(pp, std::integral_constant<int, C>{}, [](double x, double y) { return x + y; });
+      if (lane % (32 / C) == 0) {
+        const int c = lane / (32 / C);
+        ppart[((c & 1) * 4 + q) * W + w0 + (c >> 1)] = pp[0];
+      }
+#pragma unroll
+      for (int c = 0; c < C; ++c) pp[c] = 0.0;
+    };
+    // P(t) = pscale sum_k p_k of the step that sum_p closed, from the warps'
+    // partial sums: one lane per wire, which counts the steps to its next
+    // sample and knows where that goes
+    const bool p_lane = q == 0 && lane < WH && w0 + lane < grp.nw && a.P && a.p_stride > 0;
+    const int64_t p_off = p_lane ? a.wires[grp.wire[w0 + lane]].p_off : -1;
+    int p_left = a.p_stride, p_row = 0;
+    auto put_p = [&]() {
+      if (!p_lane || --p_left > 0) return;
+      p_left = a.p_stride;
+      const int r = p_row++;
+      if (r < a.p_cap && p_off >= 0 && p_off + r < a.n_P) {
+        const int w = w0 + lane;
+        double sr = 0.0, si = 0.0;
+        for (int qq = 0; qq < 4; ++qq) {
+          sr += ppart[(0 * 4 + qq) * W + w];
+          si += ppart[(1 * 4 + qq) * W + w];
+        }
+        a.P[2 * (p_off + r)] = wpar[w].w * sr;
+        a.P[2 * (p_off + r) + 1] = wpar[w].w * si;
+      }
+    };
     for (int s = 0; s < total_stages; ++s) {
       const int stg = s & 3;
       const int bn = (s + 1) & 1;  // X buffer this stage's epilogue writes
-      // drive of this stage as M/hbar: lane j < WH evaluates wire w0 + j
-      float Mr = 0.f, Mi = 0.f;
-      if (lane < WH) {
-        const double t = tj + (stg == 0 ? 0.0 : (stg == 3 ? h : h / 2.0));
-        const double* pc = pulse + (w0 + lane) * 8;
-        double mr = 0.0, mim = 0.0;
-#pragma unroll
-        for (int jj = 0; jj < 2; ++jj) {
-          const double u = t - pc[4 * jj + 0];
-          const double env = exp(pc[4 * jj + 1] * u * u);
-          mr += pc[4 * jj + 2] * env;
-          mim += pc[4 * jj + 3] * env;
-        }
-        Mr = (float)(mr * inv_hbar);
-        Mi = (float)(mim * inv_hbar);
+      // What the stage end leaves to its successor, so that the MMAs run
+      // meanwhile: columns whose values outgrew their scale are re-digitised
+      // (rare, and the issuer waits for it), the write scales of this
+      // stage's digits follow from the last stage's column maxima, and a
+      // finished step's P is written.  X[bn]'s flags were read a stage ago.
+      if (s > 0 && ovf_any[s & 1]) {
+        x_pass(s & 1, true);
+        fence_async_smem();
+        named_sync(3, kEpiThreads + 32);
       }
-      double pr[WH], pim[WH];
-#pragma unroll
-      for (int jj = 0; jj < WH; ++jj) pr[jj] = pim[jj] = 0.0;
+      set_write_scales(bn);
+      if (tid < N) ovf[bn * N + tid] = 0;
+      if (tid == 0) ovf_any[bn] = 0;
+      if (s > 1) {
+        if (stg == 0) sum_p();
+        if (stg == 1) put_p();
+      }
+      named_sync(2, kEpiThreads);
+      const float2* dr = drv + (s & 1) * W;
       float cm[4 * WH];
 #pragma unroll
       for (int c = 0; c < 4 * WH; ++c) cm[c] = 0.f;
@@ -678,65 +822,60 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
       int* ovn = ovf + bn * N;
       for (int mi = 0; mi < nM; ++mi, ++it) {
         const int k = mi * kTileRows + 32 * q + lane;
-        const int b = it & 1;
-        // band energies of this row: loaded before the wait, which hides them
-        const double ekh = k < nk ? (Ee[k] + Eh[k]) * inv_hbar : 0.0;
-        bool got = mbar_wait(&dfull[b], (it >> 1) & 1, abort, a.spin_limit);
+        // accumulator set of this row tile and the parity of its completion
+        const int b = feed == Feed::kByTile ? mi : (int)(it & 1);
+        const uint32_t full = feed == Feed::kByTile ? (uint32_t)(s & 1) : (it >> 1) & 1u;
+        const double ekh = (ee + eh) * inv_hbar;  // band energies of this row
+        bool got = mbar_wait_sleep(&dfull[b], full, abort, a.spin_limit);
         got = __all_sync(0xffffffffu, got);
         if (got) tc_fence_after();
+        band(mi + 1 < nM ? mi + 1 : 0);  // the next row's, used a tile later
         // this lane's row takes part in this tile (abort read once per tile)
         const bool live = got && k < nk && !*abort;
         const uint32_t kofs = (uint32_t)(k >> 4) * 128 + (uint32_t)(k & 15);
+        constexpr int JW = WH < 2 ? WH : 2;  // wires of one TMEM read
 #pragma unroll
-        for (int jp = 0; jp < WH; jp += 2) {
-          // accumulators of wires w0+jp, w0+jp+1 (8 columns each)
-          uint32_t r2[8], r3[8], r4[8];
+        for (int jp = 0; jp < WH; jp += JW) {
+          // accumulators of wires w0+jp .. w0+jp+JW-1 (4 JW columns each)
+          uint32_t r2[4 * JW], r3[4 * JW], r4[4 * JW];
+          auto ld = [](uint32_t col, uint32_t* r) {
+            if constexpr (JW == 2)
+              tmem_ld8(col, r);
+            else
+              tmem_ld4(col, r);
+          };
           if (got) {
-            const uint32_t col = lrow + (uint32_t)(3 * N * b * NI + 4 * (w0 + jp));
-            tmem_ld8(col, r2);
-            tmem_ld8(col + N, r3);
-            tmem_ld8(col + 2 * N, r4);
-            if (NI == 2 && nK > 1) {
-              // the second issuer's partial sums (every row tile has slices
-              // of both issuers when nK > 1)
-              uint32_t s2[8], s3[8], s4[8];
-              tmem_ld8(col + 3 * N, s2);
-              tmem_ld8(col + 4 * N, s3);
-              tmem_ld8(col + 5 * N, s4);
-              tmem_ld_wait();
-#pragma unroll
-              for (int c = 0; c < 8; ++c) {
-                r2[c] += s2[c];
-                r3[c] += s3[c];
-                r4[c] += s4[c];
-              }
-            }
+            const uint32_t col = lrow + (uint32_t)(3 * N * b + 4 * (w0 + jp));
+            ld(col, r2);
+            ld(col + N, r3);
+            ld(col + 2 * N, r4);
             tmem_ld_wait();
           }
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
+          for (int u = 0; u < JW; ++u) {
             const int j = jp + u;
             const int w = w0 + j;
-            const float Mjr = __shfl_sync(0xffffffffu, Mr, j);
-            const float Mji = __shfl_sync(0xffffffffu, Mi, j);
             if (!live || w >= grp.nw) continue;
+            const float2 Mj = dr[w];
             // exchange sums / hbar (SBEs.py:896-921) from the exact digit
             // products, rounded once to FP32
+            const float4 fxw = *reinterpret_cast<const float4*>(fx + 4 * w);
+            const float fxv[4] = {fxw.x, fxw.y, fxw.z, fxw.w};
             float exh[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
               const int cc = 4 * u + c;
               const float e = (float)(int)r2[cc] +
                               ((float)(int)r3[cc] + (float)(int)r4[cc] * inv_base) * inv_base;
-              exh[c] = e * fx[4 * w + c];
+              exh[c] = e * fxv[c];
             }
             float4* ysp; float4* accp; float4* yfp;
             ws_ptrs(w, k, ysp, accp, yfp);
             const float4 ysf = *ysp;
             // diagonal RHS (SBEs.py:1962-1975, 2325-2337, 2623-2636) / hbar:
             // phase and dephasing terms in FP64, Rabi terms in FP32
-            const float omr = Mjr + exh[0];
-            const float omi = Mji + exh[1];
+            const float omr = Mj.x + exh[0];
+            const float omi = Mj.y + exh[1];
             const double sumh = (ekh + gaph[w]) - (double)(exh[2] + exh[3]);
             const float nn = ysf.z + ysf.w - 1.f;
             const double prd = ysf.x, pid = ysf.y;
@@ -763,8 +902,8 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
               *yp = yv;
               nxt = make_float4((float)yv.x, (float)yv.y, (float)yv.z, (float)yv.w);
               *yfp = nxt;
-              pr[j] += yv.x;
-              pim[j] += yv.y;
+              pp[2 * j] += yv.x;
+              pp[2 * j + 1] += yv.y;
             } else {
               const float4 af = *accp;
               *accp = make_float4(af.x + 2.f * f0, af.y + 2.f * f1, af.z + 2.f * f2,
@@ -788,73 +927,38 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
               xn[o] = (uint8_t)d1;
               xn[L.plane + o] = (uint8_t)d2;
               xn[2 * L.plane + o] = (uint8_t)d3;
-              if (!(fabsf(xv[c]) < 0.5f)) {
-                ovn[4 * w + c] = 1;
-                ovf_any[bn] = 1;
-              }
+            }
+            // a value outside its lagged scale (or not a number): rare
+            if (!(fabsf(xv[0]) < 0.5f && fabsf(xv[1]) < 0.5f && fabsf(xv[2]) < 0.5f &&
+                  fabsf(xv[3]) < 0.5f)) {
+#pragma unroll
+              for (int c = 0; c < 4; ++c)
+                if (!(fabsf(xv[c]) < 0.5f)) ovn[4 * w + c] = 1;
+              ovf_any[bn] = 1;
             }
           }
         }
         // accumulators of this row tile are free again
         tc_fence_before();
         __syncwarp();
-        if (lane == 0 && got) mbar_arrive(&dfree[b]);
+        if (lane == 0 && got && feed != Feed::kByTile) mbar_arrive(&dfree[b]);
       }
       publish_colmax(cm);
-      if (stg == 3) {
-        // P(t) = pscale * sum_k p_k, reduced in a fixed order
-#pragma unroll
-        for (int jj = 0; jj < WH; ++jj) {
-          double sr = pr[jj], si = pim[jj];
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) {
-            sr += __shfl_xor_sync(0xffffffffu, sr, o);
-            si += __shfl_xor_sync(0xffffffffu, si, o);
-          }
-          if (lane == 0) {
-            ppart[(0 * 4 + q) * W + w0 + jj] = sr;
-            ppart[(1 * 4 + q) * W + w0 + jj] = si;
-          }
-        }
-      }
-      named_sync(2, kEpiThreads);
-      if (!*abort) {
-        // columns whose values outgrew the lagged scale: exact re-digitising
-        if (ovf_any[bn]) x_pass(bn, true);
-        // flags of X[s & 1] were consumed at the end of the previous stage
-        if (tid < N) ovf[(s & 1) * N + tid] = 0;
-        if (tid == 0) ovf_any[s & 1] = 0;
-        // write scales of the next stage (digits into X[s & 1])
-        set_write_scales(s & 1);
-      }
-      if (stg == 3) {
-        if (q == 0 && lane < WH && w0 + lane < grp.nw) {
-          const int w = w0 + lane;
-          const int step = s >> 2;
-          if (a.P && a.p_stride > 0 && (step + 1) % a.p_stride == 0) {
-            const int r = (step + 1) / a.p_stride - 1;
-            const PsbWire& wd = a.wires[grp.wire[w]];
-            if (r < a.p_cap && wd.p_off >= 0 && wd.p_off + r < a.n_P) {
-              double sr = 0.0, si = 0.0;
-              for (int qq = 0; qq < 4; ++qq) {
-                sr += ppart[(0 * 4 + qq) * W + w];
-                si += ppart[(1 * 4 + qq) * W + w];
-              }
-              a.P[2 * (wd.p_off + r)] = wpar[w].w * sr;
-              a.P[2 * (wd.p_off + r) + 1] = wpar[w].w * si;
-            }
-          }
-        }
-        tj = tj + h;
-      }
       // this thread's digit stores become visible to the tensor cores
       fence_async_smem();
       if (warp == 0 && lane == 0) snap[s & 1] = *abort;
-      named_sync(1, kEpiThreads + 32 * NI);
-      if (snap[s & 1]) break;
+      named_sync(1, kStageThreads);
+      if (snap[s & 1]) {
+        done = false;
+        break;
+      }
+    }
+    if (done) {  // (every warp read the same snapshot)
+      sum_p();
+      named_sync(2, kEpiThreads);
+      put_p();
     }
     if (!*abort) {
-      if (q == 0 && lane < WH) wt[w0 + lane] = tj;
       // resident state back to the caller's y
       if (RES) {
         for (int mi = 0; mi < nM; ++mi) {
@@ -872,7 +976,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
 
   // ---- teardown -----------------------------------------------------------------
   // every MMA of every issuer has completed before TMEM is released
-  if (warp >= kMmaWarp && warp < kMmaWarp + NI && elect_one()) umma_commit(final_bar);
+  if (warp == kMmaWarp && elect_one()) umma_commit(final_bar);
   if (warp == kMmaWarp && lane == 0) {
     bool done = false;
     for (uint32_t i = 0; i < kSpinLimit && !done; ++i) done = mbar_try_wait(final_bar, 0);

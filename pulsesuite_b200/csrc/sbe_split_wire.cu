@@ -70,6 +70,24 @@ namespace splitw {
 
 using namespace psb::split;
 
+constexpr int kEpiWarps = 8;    // warps 0..7: drain + epilogue (warpgroups 0, 1)
+constexpr int kGenWarp0 = 8;    // warps 8..11: A-tile generators (warpgroup 2)
+constexpr int kGenWarps = 4;
+constexpr int kMmaWarp = 12;    // warp 12: TMEM owner + MMA issuer (warpgroup 3;
+                                // warps 13..15 only complete that warpgroup)
+constexpr int kThreadsS = 32 * 16;
+constexpr int kEpiThreads = 32 * kEpiWarps;
+// Registers per thread: 128 at launch (65536 / 512 threads); after the
+// set-up the generator and MMA warpgroups give theirs down to kRegsLow and
+// the two epilogue warpgroups take them: 256 kRegsHigh + 256 kRegsLow =
+// 512 * kRegsLaunch, so the increase always finds its registers.
+constexpr int kRegsLaunch = 128;
+constexpr int kRegsLow = 64;
+constexpr int kRegsHigh = 2 * kRegsLaunch - kRegsLow;  // 192
+static_assert(kEpiWarps * 32 * kRegsHigh + (kThreadsS - kEpiWarps * 32) * kRegsLow <=
+                  kThreadsS * kRegsLaunch,
+              "register split exceeds the launch allocation");
+
 constexpr int kIssuers = 4;  // warps 12..15 issue MMAs (row tiles mi = k mod 4)
 constexpr int kMaxW = PSB_SPLIT_WMAX;
 constexpr int kSeqRows = 24;                // N rows of a sequence per 16-k block

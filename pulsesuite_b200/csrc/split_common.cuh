@@ -11,23 +11,6 @@
 namespace psb {
 namespace split {
 
-constexpr int kEpiWarps = 8;    // warps 0..7: drain + epilogue (warpgroups 0, 1)
-constexpr int kGenWarp0 = 8;    // warps 8..11: A-tile generators (warpgroup 2)
-constexpr int kGenWarps = 4;
-constexpr int kMmaWarp = 12;    // warp 12: TMEM owner + MMA issuer (warpgroup 3;
-                                // warps 13..15 only complete that warpgroup)
-constexpr int kThreadsS = 32 * 16;
-constexpr int kEpiThreads = 32 * kEpiWarps;
-// Registers per thread: 128 at launch (65536 / 512 threads); after the
-// set-up the generator and MMA warpgroups give theirs down to kRegsLow and
-// the two epilogue warpgroups take them: 256 kRegsHigh + 256 kRegsLow =
-// 512 * kRegsLaunch, so the increase always finds its registers.
-constexpr int kRegsLaunch = 128;
-constexpr int kRegsLow = 64;
-constexpr int kRegsHigh = 2 * kRegsLaunch - kRegsLow;  // 192
-static_assert(kEpiWarps * 32 * kRegsHigh + (kThreadsS - kEpiWarps * 32) * kRegsLow <=
-                  kThreadsS * kRegsLaunch,
-              "register split exceeds the launch allocation");
 constexpr int kTileRows = 128;  // M of one MMA
 constexpr int kTileK = 64;      // k' per A tile
 constexpr int kDigits = 3;
@@ -151,17 +134,24 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
         "=r"(r[7])
       : "r"(taddr));
 }
+// 4 consecutive TMEM columns of this thread's lane (no wait)
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr));
+}
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+// 16 columns of this thread's lane (no wait).  No memory clobber: the next
+// columns' words may be loaded ahead of it.
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
       "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
       "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
       "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]),
-      "r"(r[15])
-      : "memory");
+      "r"(r[15]));
 }
 
 // Three balanced base-254 digits of v, |v| < 1/2 (so |254 v| < 127): each
@@ -182,20 +172,6 @@ __device__ __forceinline__ void digits3(float v, int& d1, int& d2, int& d3) {
   d1 = __float_as_int(t1) - kMagicBits;
   d2 = __float_as_int(t2) - kMagicBits;
   d3 = __float_as_int(t3) - kMagicBits;
-}
-
-// One step of a halving max-butterfly over a warp: each lane holds C
-// values, sends half of them to the lane `o` apart and keeps the maxima of
-// the other half (the lane with bit o set keeps the upper half).
-template <int C>
-__device__ __forceinline__ void colmax_halve(float* v, int o, int lane) {
-  const bool up = (lane & o) != 0;
-#pragma unroll
-  for (int i = 0; i < C / 2; ++i) {
-    const float send = up ? v[i] : v[i + C / 2];
-    const float keep = up ? v[i + C / 2] : v[i];
-    v[i] = fmaxf(keep, __shfl_xor_sync(0xffffffffu, send, o));
-  }
 }
 
 // Shared-memory matrix descriptor, no swizzle (canonical layout of 8-row x
