@@ -825,7 +825,8 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
         // accumulator set of this row tile and the parity of its completion
         const int b = feed == Feed::kByTile ? mi : (int)(it & 1);
         const uint32_t full = feed == Feed::kByTile ? (uint32_t)(s & 1) : (it >> 1) & 1u;
-        const double ekh = (ee + eh) * inv_hbar;  // band energies of this row
+        // band energies of this row (not fused into the sum with the gap)
+        const double ekh = __dmul_rn(ee + eh, inv_hbar);
         bool got = mbar_wait_sleep(&dfull[b], full, abort, a.spin_limit);
         got = __all_sync(0xffffffffu, got);
         if (got) tc_fence_after();
