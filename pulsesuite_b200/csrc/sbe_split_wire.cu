@@ -42,21 +42,27 @@
 // buffered between consecutive wires).
 //
 // One CTA owns a group of up to 16 wires (one grid) for all steps and
-// visits them round robin, stage by stage.  Roles (16 warps):
-//   warps 0..7   drain + epilogue: the whole wire per item (8 warps share
-//                its row tiles), FP64 right-hand side and RK4 stage
-//                combination, then the exact column scales and the digits
-//                of the next stage point, the n1D and P(t) sums; for
+// visits them round robin, stage by stage.  Roles (24 warps):
+//   warps 0..15  drain + epilogue in two teams of 8, team t the wires j = t
+//                (mod 2) with accumulator buffer t: the whole wire per item
+//                (8 warps share its row tiles), FP64 right-hand side and RK4
+//                stage combination, then the exact column scales and the
+//                digits of the next stage point, the n1D and P(t) sums; for
 //                screened tables, then n1D -> eps(q) (coulomb.py:1172-1193)
 //                -> V/eps and VS of the wire's next stage;
-//   warps 8..11  A-tile generators; for a screened wire they first write
+//   warps 16..19 A-tile generators; for a screened wire they first write
 //                the digits of its V/eps / VS into its byte arrays;
-//   warps 12..15 MMA issuers, one per row tile mi (mod 4); warp 12 owns
-//                TMEM.  One thread issues a tcgen05.mma about every 100-120
-//                cycles whatever N is (measured on B200 for M = 128, K = 32
-//                int8, N <= 128), while four issuing warps reach about four
-//                times that rate, so the narrow per-wire MMAs are spread
-//                over four issuers with disjoint accumulators.
+//   warps 20..23 MMA issuers (one elected lane each), one per row tile mi
+//                (mod 4); warp 20 owns TMEM.
+// What bounds it: up to Nk 256 the epilogue, a chain of ~8000 cycles a wire
+// (loads, RHS, two reductions, digits, two FP64 logarithms and the divisions
+// of eps) that the second team hides; from Nk 512 the generators (~500
+// cycles a tile, 14 tiles a wire and stage).  us per wire-stage of a screened
+// CTA, one team of 8 epilogue warps -> now: Nk 64 4.1 -> 2.2, 128 4.0 ->
+// 2.3, 256 4.5 -> 2.9, 512 6.5 -> 5.0, 1024 15.6 -> 11.7; distinct screened
+// matrices, Nk 300: 9.9 -> 8.5.  Tried and slower: eight generator warps (72
+// registers at launch: Nk 128 +7 %, Nk 512 -2 %), two digit planes in flight
+// per generator (Nk 512 +4 %).
 // While one wire's epilogue and table run, the tensor cores work on the
 // other wires of the group.  Every mbarrier wait is bounded (as in
 // sbe_split.cu); a CTA that runs out records PSB_ERR_TIMEOUT in its wires'
@@ -70,30 +76,30 @@ namespace splitw {
 
 using namespace psb::split;
 
-constexpr int kEpiWarps = 8;    // warps 0..7: drain + epilogue (warpgroups 0, 1)
-constexpr int kGenWarp0 = 8;    // warps 8..11: A-tile generators (warpgroup 2)
+constexpr int kTeams = 2;       // epilogue teams: team t takes the wires j = t (mod 2)
+constexpr int kTeamWarps = 8;   // warps 0..7 and 8..15 (warpgroups 0, 1 and 2, 3)
+constexpr int kTeamThreads = 32 * kTeamWarps;
+constexpr int kGenWarp0 = 16;   // warps 16..19: A-tile generators
 constexpr int kGenWarps = 4;
-constexpr int kMmaWarp = 12;    // warp 12: TMEM owner + MMA issuer (warpgroup 3;
-                                // warps 13..15 only complete that warpgroup)
-constexpr int kThreadsS = 32 * 16;
-constexpr int kEpiThreads = 32 * kEpiWarps;
-// Registers per thread: 128 at launch (65536 / 512 threads); after the
-// set-up the generator and MMA warpgroups give theirs down to kRegsLow and
-// the two epilogue warpgroups take them: 256 kRegsHigh + 256 kRegsLow =
-// 512 * kRegsLaunch, so the increase always finds its registers.
-constexpr int kRegsLaunch = 128;
-constexpr int kRegsLow = 64;
-constexpr int kRegsHigh = 2 * kRegsLaunch - kRegsLow;  // 192
-static_assert(kEpiWarps * 32 * kRegsHigh + (kThreadsS - kEpiWarps * 32) * kRegsLow <=
-                  kThreadsS * kRegsLaunch,
+constexpr int kMmaWarp = 20;    // warps 20..23: MMA issuers, 20 the TMEM owner
+constexpr int kThreadsS = 32 * 24;
+constexpr int kSetupThreads = 512;  // threads that sum a wire's initial n1D
+// Registers per thread: 80 at launch (65536 / 768 threads, a multiple of 8);
+// after the set-up the generator and MMA warpgroups give theirs down to
+// kRegsGen and kRegsMma and the four epilogue warpgroups take them, no more
+// in all than the launch holds, so the increase always finds its registers.
+constexpr int kRegsLaunch = 80;
+constexpr int kRegsGen = 56;
+constexpr int kRegsMma = 40;
+constexpr int kRegsHigh = 96;
+static_assert(kTeams * kTeamWarps * kRegsHigh + 4 * kRegsGen + 4 * kRegsMma <= 24 * kRegsLaunch,
               "register split exceeds the launch allocation");
 
-constexpr int kIssuers = 4;  // warps 12..15 issue MMAs (row tiles mi = k mod 4)
+constexpr int kIssuers = 4;  // warps 20..23 issue MMAs (row tiles mi = k mod 4)
 constexpr int kMaxW = PSB_SPLIT_WMAX;
 constexpr int kSeqRows = 24;                // N rows of a sequence per 16-k block
 constexpr int kSeqBlock = kSeqRows * 16;    // bytes per 16-k block (K-direction stride)
-constexpr int kMaxTilesPerWarp = 4;         // row tiles per epilogue warp (nk <= 1024)
-constexpr int kMaxNkW = 2 * kMaxTilesPerWarp * kTileRows;  // 1024
+constexpr int kMaxNkW = PSB_MAX_NK;
 constexpr int kMaxSlotsW = 8;
 
 // Fixed part of the shared-memory map (bytes from `misc`).
@@ -104,10 +110,13 @@ constexpr uint32_t kOffGaph = kOffWpar + 32 * kMaxW;       // double[16]
 constexpr uint32_t kOffWt = kOffGaph + 8 * kMaxW;          // double[16][2]
 constexpr uint32_t kOffWoff = kOffWt + 16 * kMaxW;         // int64[16]
 constexpr uint32_t kOffVs = kOffWoff + 8 * kMaxW;          // double[16][3]
-constexpr uint32_t kOffSx = kOffVs + 24 * kMaxW;           // int[8 warps][16][4]
-constexpr uint32_t kOffRed = kOffSx + 16 * kEpiWarps * kMaxW;  // [2][8 warps] x 48 B
-constexpr uint32_t kOffSred = kOffRed + 2 * kEpiWarps * 48;    // double[16][4]
-constexpr uint32_t kMiscBytes = kOffSred + 8 * 4 * 16;
+constexpr uint32_t kOffSx = kOffVs + 24 * kMaxW;           // int[16][4]
+constexpr uint32_t kOffRed = kOffSx + 16 * kMaxW;  // [team][2][8 warps] x 48 B
+constexpr uint32_t kOffSred = kOffRed + 2 * kTeams * kTeamWarps * 48;    // double[16][4]
+constexpr uint32_t kMiscEnd = kOffSred + 8 * 4 * 16;
+// (the largest groups, psb_split_wire_max_group, follow from this size)
+constexpr uint32_t kMiscBytes = kOffSx + 3328;
+static_assert(kMiscEnd <= kMiscBytes, "shared-memory map");
 constexpr int kNumBars = 2 * kMaxSlotsW + 5 + 3 * kMaxW;
 
 struct Args {
@@ -287,7 +296,8 @@ __device__ void table_digits(const double* sv, const double* vs, int nk, int c0,
   }
 }
 
-template <int NT>
+// MT: row tiles of an epilogue warp (2: nk <= 512, 4: nk <= 1024).
+template <int NT, int MT>
 __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const int tid = threadIdx.x;
@@ -301,7 +311,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
   PsbTable tb{};
   if (ok) {
     tb = a.tables[grp.table];
-    ok = tb.nk >= 2 && tb.nk <= kMaxNkW && tb.off >= 0 &&
+    ok = tb.nk >= 2 && tb.nk <= 2 * MT * kTileRows && tb.off >= 0 &&
          tb.off + 9 * (int64_t)tb.nk <= a.n_tabdata && (tb.flags & PSB_TAB_EXCITONS) &&
          (NT == 3 || (tb.flags & PSB_TAB_SHARED_V)) &&
          (((tb.flags & PSB_TAB_SCREENED) != 0) == scr) &&
@@ -342,15 +352,15 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
   uint8_t* misc = smem + L.misc;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(misc);
   volatile int* abort = reinterpret_cast<volatile int*>(misc + kOffAbort);
-  volatile int* snap = reinterpret_cast<volatile int*>(misc + kOffSnap);  // [2]
+  volatile int* snap = reinterpret_cast<volatile int*>(misc + kOffSnap);  // [team][2]
   double* pulse = reinterpret_cast<double*>(misc + kOffPulse);
   double4* wpar = reinterpret_cast<double4*>(misc + kOffWpar);
   double* gaph = reinterpret_cast<double*>(misc + kOffGaph);
   double* wtb = reinterpret_cast<double*>(misc + kOffWt);  // [W][2] by step parity
   int64_t* woff = reinterpret_cast<int64_t*>(misc + kOffWoff);
   double* vsw = reinterpret_cast<double*>(misc + kOffVs);  // [W][3] (unscreened: row 0)
-  int* sx = reinterpret_cast<int*>(misc + kOffSx);  // [epilogue warp][W][4] column scales
-  uint8_t* red = misc + kOffRed;                      // [2][8] {float cm[4], double n1, pr, pi}
+  int* sx = reinterpret_cast<int*>(misc + kOffSx);  // [W][4] column scales
+  uint8_t* red = misc + kOffRed;                      // [team][2][8] {float cm[4], double n1, pr, pi}
   double* sred = reinterpret_cast<double*>(misc + kOffSred);
   const double inv_hbar = 1.0 / a.hbar;
   const double* blk = a.tabdata + tb.off;
@@ -367,11 +377,11 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&dfull[b], kIssuers);
-      mbar_init(&dfree[b], kEpiWarps);
+      mbar_init(&dfree[b], kTeamWarps);
     }
     mbar_init(final_bar, kIssuers);
     for (int j = 0; j < kMaxW; ++j) {
-      mbar_init(&xfull[j], kEpiWarps);
+      mbar_init(&xfull[j], kTeamWarps);
       mbar_init(&svfull[j], 1);
       mbar_init(&gdone[j], kGenWarps);
     }
@@ -430,7 +440,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
   for (int j = 0; j < nw; ++j) {
     float cm[4] = {0.f, 0.f, 0.f, 0.f};
     double sn = 0.0;
-    for (int k = tid; k < nk; k += kThreadsS) {
+    for (int k = tid; tid < kSetupThreads && k < nk; k += kSetupThreads) {
       const double4 yv = g_y[woff[j] + k];
       const float4 yf = make_float4((float)yv.x, (float)yv.y, (float)yv.z, (float)yv.w);
       a.ws_ys[woff[j] + k] = yf;
@@ -447,7 +457,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
 #pragma unroll
       for (int v = 0; v < 4; ++v) cm[v] = fmaxf(cm[v], __shfl_xor_sync(0xffffffffu, cm[v], o));
     }
-    if (lane == 0) {
+    if (lane == 0 && tid < kSetupThreads) {
       sred[warp * 4 + 0] = sn;
       float* f = reinterpret_cast<float*>(sred + warp * 4 + 1);
       for (int v = 0; v < 4; ++v) f[v] = cm[v];
@@ -455,7 +465,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
     __syncthreads();
     double tot = 0.0;
     float cma[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int i = 0; i < kThreadsS / 32; ++i) {
+    for (int i = 0; i < kSetupThreads / 32; ++i) {
       tot += sred[i * 4 + 0];
       const float* f = reinterpret_cast<const float*>(sred + i * 4 + 1);
       for (int v = 0; v < 4; ++v) cma[v] = fmaxf(cma[v], f[v]);
@@ -465,7 +475,8 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
       double n1d = tot / 2.0 / tb.L;
       n1d = n1d < tb.dens_max ? n1d : tb.dens_max;
       double* svj = svb + (uint32_t)j * (L.svsz / 8);
-      table_scaled<NT>(qcs, vts, nk, true, n1d, svj, vsw + 3 * j, sred, 0, kThreadsS, 0);
+      if (tid < kSetupThreads)
+        table_scaled<NT>(qcs, vts, nk, true, n1d, svj, vsw + 3 * j, sred, 0, kSetupThreads, 1);
       __syncthreads();
       table_digits<NT>(svj, vsw + 3 * j, nk, (int)c0, tabq + (uint32_t)(j * NT) * L.tabsz,
                        L.plane, 0, kThreadsS);
@@ -497,10 +508,11 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
         xq[16 * 16] = (uint8_t)d3;
       }
     }
-    if (tid < 4 * kEpiWarps) sx[((tid >> 2) * kMaxW + j) * 4 + (tid & 3)] = se[tid & 3];
+    if (tid < 4) sx[4 * j + tid] = se[tid];
   }
   if (!scr) {
-    table_scaled<NT>(qcs, vts, nk, false, 0.0, svb, vsw, sred, 0, kThreadsS, 0);
+    if (tid < kSetupThreads)
+      table_scaled<NT>(qcs, vts, nk, false, 0.0, svb, vsw, sred, 0, kSetupThreads, 1);
     __syncthreads();
     table_digits<NT>(svb, vsw, nk, (int)c0, tabq, L.plane, 0, kThreadsS);
   }
@@ -521,9 +533,15 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
   const uint32_t idesc16 = idesc_i8(16);
   const int total_stages = a.nsteps * 4;
   const double h = a.dt;
+  // Accumulator buffer b = j & 1 serves the wires of team b in (stage, wire)
+  // order; how often it was filled before stage s of wire j:
+  auto pow2 = [](int e) { return __uint_as_float((uint32_t)(127 + e) << 23); };  // |e| <= 120
+  auto fill = [&](int s, int j) -> uint32_t {
+    return (uint32_t)s * (uint32_t)((nw + 1 - (j & 1)) >> 1) + (uint32_t)(j >> 1);
+  };
 
   if (warp >= kMmaWarp) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsLow));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsMma));
     // ---- MMA issuers: items (stage, wire) in order; per item the distinct
     // tiles d in groups of G slots; issuer k takes the row tiles mi = k
     // (mod 4) of every (row tile, k' slice) pair of a tile: two K steps,
@@ -533,14 +551,14 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
     const int ik = warp - kMmaWarp;
     const uint64_t bdesc0 = smem_desc(smem_u32(xbase), kSeqBlock, 128);
     if (elect_one()) {
-      uint32_t it = 0;  // items issued
       uint32_t gi = 0;  // groups issued: buffer gi & 1, filled for the (gi >> 1)-th time
       bool go = true;
       for (int s = 0; s < total_stages && go; ++s) {
-        for (int j = 0; j < nw && go; ++j, ++it) {
-          const int b = it & 1;
+        for (int j = 0; j < nw && go; ++j) {
+          const int b = j & 1;
+          const uint32_t use = fill(s, j);
           if (s >= 1) go = mbar_wait_sleep(&xfull[j], (s - 1) & 1, abort, lim);
-          if (go && it >= 2) go = mbar_wait_sleep(&dfree[b], ((it >> 1) - 1) & 1, abort, lim);
+          if (go && use > 0) go = mbar_wait_sleep(&dfree[b], (use - 1) & 1, abort, lim);
           if (!go) break;
           tc_fence_after();
           const uint32_t dbase = tmem + (uint32_t)b * dstride;
@@ -589,7 +607,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
     }
     __syncwarp();
   } else if (warp >= kGenWarp0) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsLow));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsGen));
     // ---- A-tile generators: row r = 32 gq + lane of tile d is a(64 d + r - c),
     // c = 0..63; TMEM column jc of a digit plane holds c = 4 jc .. 4 jc + 3,
     // the four bytes from R[c0 - 64 d - r + 4 jc]: 17 aligned words and a
@@ -661,7 +679,9 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsHigh));
     // ---- drain / epilogue: warp (q, hh) takes rows 128 mi + 32 q + lane of
     // the row tiles mi = hh, hh + 2, ... of the current wire.
-    const int q = warp & 3, hh = warp >> 2;
+    const int q = warp & 3, hh = (warp >> 2) & 1;
+    const int team = warp / kTeamWarps, ew = warp % kTeamWarps;
+    const int ttid = tid - team * kTeamThreads;
     const uint32_t lrow = tmem + ((uint32_t)(32 * q) << 16);
     const float inv_base = 1.f / 254.f;
     const float hf = (float)h, h2f = (float)(h / 2.0), h6f = (float)(h / 6.0);
@@ -670,8 +690,8 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
     bool go = true;
     for (int s = 0; s < total_stages && go; ++s) {
       const int stg = s & 3, step = s >> 2;
-      for (int j = 0; j < nw; ++j, ++it) {
-        const int b = it & 1;
+      for (int j = team; j < nw; j += kTeams, ++it) {
+        const int b = team;
         bool got = true;
         // decode factors VS_t / (hbar 254^2) 2^-sexp (VS of a screened wire's
         // stage was set by these warps when they built its table); scaling a
@@ -680,7 +700,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
 #pragma unroll
         for (int v = 0; v < 4; ++v)
           fac[v] = (float)(vsw[(scr ? 3 * j : 0) + mat_of<NT>(v)] * dec_hb) *
-                   ldexpf(1.f, -sx[(warp * kMaxW + j) * 4 + v]);
+                   pow2(-sx[4 * j + v]);
         // drive M(t)/hbar of this stage: lane 0 evaluates pulse 0, lane 1
         // pulse 1, summed in that order
         double mr = 0.0, mim = 0.0;
@@ -700,29 +720,34 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
         const double gw = wpar[j].y, gj = gaph[j];
         const int64_t wo = woff[j];
         // this thread's elements: loads issued before the accumulator wait
-        float4 ysv[kMaxTilesPerWarp], accv[kMaxTilesPerWarp], yfv[kMaxTilesPerWarp];
-        double ekh[kMaxTilesPerWarp];
-#pragma unroll
-        for (int i = 0; i < kMaxTilesPerWarp; ++i) {
+        // (for four row tiles they would not fit in its registers)
+        float4 ysv[MT], accv[MT], yfv[MT];
+        double ekh[MT];
+        auto load = [&](int i) {
           const int k = (hh + 2 * i) * kTileRows + 32 * q + lane;
           if (k < nk) {
             ysv[i] = a.ws_ys[wo + k];
-            accv[i] = a.ws_acc[wo + k];
-            yfv[i] = a.ws_yf[wo + k];
+            if (stg != 0) accv[i] = a.ws_acc[wo + k];
+            if (stg == 1 || stg == 2) yfv[i] = a.ws_yf[wo + k];
             ekh[i] = (Ee[k] + Eh[k]) * inv_hbar;
           }
+        };
+        if (MT == 2) {
+#pragma unroll
+          for (int i = 0; i < MT; ++i) load(i);
         }
-        if (got) got = mbar_wait(&dfull[b], (it >> 1) & 1, abort, lim);
+        if (got) got = mbar_wait_sleep(&dfull[b], fill(s, j) & 1, abort, lim);
         got = __all_sync(0xffffffffu, got);
         if (got) tc_fence_after();
         float cm[4] = {0.f, 0.f, 0.f, 0.f};
         double n1 = 0.0, pr = 0.0, pim = 0.0;
-        float4 nx[kMaxTilesPerWarp];
+        float4 nx[MT];
 #pragma unroll
-        for (int i = 0; i < kMaxTilesPerWarp; ++i) {
+        for (int i = 0; i < MT; ++i) {
           const int mi = hh + 2 * i;
           nx[i] = make_float4(0.f, 0.f, 0.f, 0.f);
           if (mi >= nM) break;
+          if (MT != 2) load(i);
           uint32_t r[16];
           if (got) {
             const uint32_t col = lrow + (uint32_t)b * dstride + 16u * (uint32_t)mi;
@@ -791,55 +816,69 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
         tc_fence_before();
         __syncwarp();
         if (lane == 0 && got) mbar_arrive(&dfree[b]);
+        // over the warp: the four maxima by halving (lane 8v ends with column
+        // v), n1D's sum for screened tables, P's at a step's end
+        {
+          const bool u16 = (lane & 16) != 0, u8 = (lane & 8) != 0;
+          float m0 = fmaxf(u16 ? cm[2] : cm[0],
+                           __shfl_xor_sync(0xffffffffu, u16 ? cm[0] : cm[2], 16));
+          float m1 = fmaxf(u16 ? cm[3] : cm[1],
+                           __shfl_xor_sync(0xffffffffu, u16 ? cm[1] : cm[3], 16));
+          m0 = fmaxf(u8 ? m1 : m0, __shfl_xor_sync(0xffffffffu, u8 ? m0 : m1, 8));
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-          for (int v = 0; v < 4; ++v) cm[v] = fmaxf(cm[v], __shfl_xor_sync(0xffffffffu, cm[v], o));
-          n1 += __shfl_xor_sync(0xffffffffu, n1, o);
-          pr += __shfl_xor_sync(0xffffffffu, pr, o);
-          pim += __shfl_xor_sync(0xffffffffu, pim, o);
+          for (int o = 4; o > 0; o >>= 1) m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, o));
+          cm[0] = m0;
         }
-        uint8_t* rb = red + ((it & 1) * kEpiWarps) * 48;
+        if (scr) {
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) n1 += __shfl_xor_sync(0xffffffffu, n1, o);
+        }
+        if (stg == 3) {
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) {
+            pr += __shfl_xor_sync(0xffffffffu, pr, o);
+            pim += __shfl_xor_sync(0xffffffffu, pim, o);
+          }
+        }
+        uint8_t* rb = red + (2 * team + (it & 1)) * kTeamWarps * 48;
+        if ((lane & 7) == 0) reinterpret_cast<float*>(rb + ew * 48)[lane >> 3] = cm[0];
         if (lane == 0) {
-          float* rf = reinterpret_cast<float*>(rb + warp * 48);
-          double* rd = reinterpret_cast<double*>(rb + warp * 48 + 16);
-          rf[0] = cm[0];
-          rf[1] = cm[1];
-          rf[2] = cm[2];
-          rf[3] = cm[3];
+          double* rd = reinterpret_cast<double*>(rb + ew * 48 + 16);
           rd[0] = n1;
           rd[1] = pr;
           rd[2] = pim;
         }
-        if (stg == 3 && tid == 0) wtb[2 * j + ((step + 1) & 1)] = wtb[2 * j + (step & 1)] + h;
-        if (tid == 0) snap[it & 1] = *abort;
-        named_sync(1, kEpiThreads);
-        if (snap[it & 1]) {
+        if (stg == 3 && ttid == 0) wtb[2 * j + ((step + 1) & 1)] = wtb[2 * j + (step & 1)] + h;
+        if (ttid == 0) snap[2 * team + (it & 1)] = *abort;
+        named_sync(1 + team, kTeamThreads);
+        if (snap[2 * team + (it & 1)]) {
           go = false;
           break;
         }
         // exact column scales of the next stage point (largest |x| in [1/4, 1/2))
         float cma[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int wq = 0; wq < kEpiWarps; ++wq) {
-          const float* rf = reinterpret_cast<const float*>(rb + wq * 48);
-#pragma unroll
-          for (int v = 0; v < 4; ++v) cma[v] = fmaxf(cma[v], rf[v]);
+        for (int wq = 0; wq < kTeamWarps; ++wq) {
+          const float4 rf = *reinterpret_cast<const float4*>(rb + wq * 48);
+          cma[0] = fmaxf(cma[0], rf.x);
+          cma[1] = fmaxf(cma[1], rf.y);
+          cma[2] = fmaxf(cma[2], rf.z);
+          cma[3] = fmaxf(cma[3], rf.w);
         }
         int se[4];
         float sc[4];
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
-          int e2 = 0;
           se[v] = 0;
           if (cma[v] > 0.f && isfinite(cma[v])) {
-            frexpf(cma[v], &e2);
+            // max |x| < 2^e2; a subnormal's smaller exponent meets the same clamp
+            const int e2 = (int)(__float_as_uint(cma[v]) >> 23) - 126;
             se[v] = min(max(-1 - e2, -120), 120);
           }
-          sc[v] = ldexpf(1.f, se[v]);
+          sc[v] = pow2(se[v]);
         }
         if (s + 1 < total_stages) {
 #pragma unroll
-          for (int i = 0; i < kMaxTilesPerWarp; ++i) {
+          for (int i = 0; i < MT; ++i) {
             const int k = (hh + 2 * i) * kTileRows + 32 * q + lane;
             if (k >= nk) continue;
             const float xv[4] = {nx[i].x * sc[0], nx[i].y * sc[1], nx[i].z * sc[2],
@@ -857,38 +896,39 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
           }
           if (lane < 4) {
             const int sv = lane == 0 ? se[0] : (lane == 1 ? se[1] : (lane == 2 ? se[2] : se[3]));
-            sx[(warp * kMaxW + j) * 4 + lane] = sv;
+            sx[4 * j + lane] = sv;  // (the same from every warp of the team)
           }
           // digit stores become visible to the tensor cores
           fence_async_smem();
           __syncwarp();
           if (lane == 0) mbar_arrive(&xfull[j]);
         }
-        double n1t = 0.0, prt = 0.0, pit = 0.0;
-        for (int wq = 0; wq < kEpiWarps; ++wq) {
-          const double* rd = reinterpret_cast<const double*>(rb + wq * 48 + 16);
-          n1t += rd[0];
-          prt += rd[1];
-          pit += rd[2];
-        }
-        if (tid == 0) {
-          if (stg == 3 && a.P && a.p_stride > 0 && (step + 1) % a.p_stride == 0) {
-            const int rr = (step + 1) / a.p_stride - 1;
-            const PsbWire& wd = a.wires[grp.wire[j]];
-            if (rr < a.p_cap && wd.p_off >= 0 && wd.p_off + rr < a.n_P) {
-              a.P[2 * (wd.p_off + rr)] = wpar[j].w * prt;
-              a.P[2 * (wd.p_off + rr) + 1] = wpar[j].w * pit;
-            }
+        if (ttid == 0 && stg == 3 && a.P && a.p_stride > 0 && (step + 1) % a.p_stride == 0) {
+          double prt = 0.0, pit = 0.0;
+          for (int wq = 0; wq < kTeamWarps; ++wq) {
+            const double* rd = reinterpret_cast<const double*>(rb + wq * 48 + 16);
+            prt += rd[1];
+            pit += rd[2];
+          }
+          const int rr = (step + 1) / a.p_stride - 1;
+          const PsbWire& wd = a.wires[grp.wire[j]];
+          if (rr < a.p_cap && wd.p_off >= 0 && wd.p_off + rr < a.n_P) {
+            a.P[2 * (wd.p_off + rr)] = wpar[j].w * prt;
+            a.P[2 * (wd.p_off + rr) + 1] = wpar[j].w * pit;
           }
         }
         // screened: this wire's table for its next stage, from the n1D of the
         // stage point just written (CalcScreenedArrays, coulomb.py:1218-1223)
         if (scr && s + 1 < total_stages) {
+          double n1t = 0.0;
+          for (int wq = 0; wq < kTeamWarps; ++wq)
+            n1t += *reinterpret_cast<const double*>(rb + wq * 48 + 16);
           double n1d = n1t / 2.0 / tb.L;
           n1d = n1d < tb.dens_max ? n1d : tb.dens_max;
           table_scaled<NT>(qcs, vts, nk, true, n1d, svb + (uint32_t)j * (L.svsz / 8), vsw + 3 * j,
-                           sred, 0, kEpiThreads, 1);
-          if (tid == 0) mbar_arrive(&svfull[j]);
+                           sred + 4 * kTeamWarps * team, team * kTeamThreads, kTeamThreads,
+                           1 + team);
+          if (ttid == 0) mbar_arrive(&svfull[j]);
         }
       }
     }
@@ -938,8 +978,8 @@ bool fits(int nk, int wgroup, bool scr) {
          WLayout<NT>(nk, wgroup, scr).total <= kMaxDynSmem;
 }
 
-template <int NT>
-int launch(Args a, int nkmax, cudaStream_t s) {
+template <int NT, int MT>
+int launch_tiles(Args a, int nkmax, cudaStream_t s) {
   const bool scr = a.screened != 0;
   if (!fits<NT>(nkmax, a.wgroup, scr))
     return set_error(PSB_ERR_SIZE,
@@ -947,7 +987,7 @@ int launch(Args a, int nkmax, cudaStream_t s) {
                      a.wgroup);
   const uint32_t smem = WLayout<NT>(nkmax, a.wgroup, scr).total;
   cudaFuncAttributes fa{};
-  cudaError_t e = cudaFuncGetAttributes(&fa, split_wire_kernel<NT>);
+  cudaError_t e = cudaFuncGetAttributes(&fa, split_wire_kernel<NT, MT>);
   if (e != cudaSuccess)
     return set_error(PSB_ERR_CUDA, "cudaFuncGetAttributes: %s", cudaGetErrorString(e));
   if (fa.numRegs != kRegsLaunch || fa.maxThreadsPerBlock < kThreadsS)
@@ -955,13 +995,20 @@ int launch(Args a, int nkmax, cudaStream_t s) {
                      "split_wire_kernel built with %d registers per thread (needs %d) and at "
                      "most %d threads (needs %d)",
                      fa.numRegs, kRegsLaunch, fa.maxThreadsPerBlock, kThreadsS);
-  e = cudaFuncSetAttribute(split_wire_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  e = cudaFuncSetAttribute(split_wire_kernel<NT, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smem);
   if (e != cudaSuccess)
     return set_error(PSB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
   a.smem_bytes = smem;
-  split_wire_kernel<NT><<<a.ngroups, kThreadsS, smem, s>>>(a);
+  split_wire_kernel<NT, MT><<<a.ngroups, kThreadsS, smem, s>>>(a);
   return check_cuda("split_wire_kernel");
+}
+
+template <int NT>
+int launch(Args a, int nkmax, cudaStream_t s) {
+  if constexpr (NT == 1)
+    if (nkmax > 4 * kTileRows) return launch_tiles<NT, 4>(a, nkmax, s);
+  return launch_tiles<NT, 2>(a, nkmax, s);
 }
 
 }  // namespace splitw

@@ -47,3 +47,29 @@ def test_split_edges(cuda, nk):
                 assert relerr(y[:, c], yr[:, c]) < 1e-5
         np.testing.assert_array_equal(y, first[0])
         np.testing.assert_array_equal(P, first[1])
+
+
+@pytest.mark.parametrize("nk", [64, 66, 126, 130, 254, 258, 510, 512, 514, 1022, 1024])
+def test_split_wire_edges(cuda, nk):
+    """Screened wires (a matrix each): groups of 1, an odd and an even number
+    of wires give the same bits, at the edges of the row tiles and on both
+    sides of Nk 512, where an epilogue warp's tiles double."""
+    steps, dt = 6, 1e-15
+    grids, w = uneven_case([nk] * 4, seed=nk, screened=True, nsteps=steps)
+    w["t0"] = 3e-15
+    ref = WireBatch(grids, w, screened=True, p_cap=steps)
+    ref.rk4(steps, dt)
+    yr, Pr = ref.state(), ref.P.cpu().numpy()
+    first = None
+    for width in (4, 3, 1):
+        b = WireBatch(grids, w, screened=True, p_cap=steps, form="split", split_w={nk: width})
+        b.rk4(steps, dt)
+        assert (b.wires()["status"] == 0).all() and (b.wires()["steps"] == steps).all()
+        y, P = b.state(), b.P.cpu().numpy()
+        if first is None:
+            first = y, P
+            assert relerr(P, Pr) < 1e-6
+            for c in (slice(0, 2), slice(2, 3), slice(3, 4)):
+                assert relerr(y[:, c], yr[:, c]) < 1e-5
+        np.testing.assert_array_equal(y, first[0])
+        np.testing.assert_array_equal(P, first[1])
