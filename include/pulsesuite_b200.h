@@ -435,6 +435,15 @@ int psb_full_sources_batch_f64(int nw, int nk, int nr, const double* d_kr, const
 int psb_spline_rows_c128(const double* x0, int n0, const double* z0, int m, const double* x1,
                          int n1, double* out);
 
+/*
+ * Host function (no device work): the signs and the scale of the centred
+ * transforms FFTG / iFFTG (usefulsubs.py:2265-2334) on m signals f [m][n]
+ * in place, in one pass with numpy's complex arithmetic.  stage 0, before the
+ * transform: odd elements negated; stage 1, after FFTG's: odd elements, then
+ * all, negated and divided by n; stage 2, after iFFTG's: the same, times n.
+ */
+int psb_centred_c128(double* f, int m, int n, int stage);
+
 /* ---- split-precision tensor-core form (sm_100a tcgen05, kind::i8) --------- */
 /*
  * The batched form of the same RK4 step: per group of wires sharing one k

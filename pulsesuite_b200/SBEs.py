@@ -650,7 +650,10 @@ class SBESolver:
         out = self.full["bout"][:n].cpu().numpy()
         if self.Optics:
             # QWPolarization3's factor and transform, all wires at once
-            P = out[:, :3] * 2 * self.ehint / self.area / self.L   # contiguous [n][3][Nr]
+            P = out[:, :3] * 2   # contiguous [n][3][Nr]
+            P *= self.ehint
+            P /= self.area
+            P /= self.L
             wirespace.fftg(P.reshape(3 * n, self.Nr))
             srcs[:, :3] = P
         if self.LF:
@@ -660,7 +663,10 @@ class SBESolver:
             # two densities at once (each row the bits of its own rho_post)
             A = np.ascontiguousarray(out[:, 3:5]).reshape(2 * n, self.Nr)
             wirespace.rho_post_rows(A, diag.reshape(2 * n, -1), self.r[1] - self.r[0])
-            srcs[:, 3:5] = 2.0 * _e0 * A.reshape(n, 2, self.Nr) / self.area * self.ehint
+            A *= 2.0 * _e0
+            A /= self.area
+            A *= self.ehint
+            srcs[:, 3:5] = A.reshape(n, 2, self.Nr)
         return srcs
 
     def _drive(self, Ex, Ey, Ez):
@@ -829,8 +835,12 @@ class SBESolver:
                                                       (Exx, Eyy, Ezz, Vrr)]), self.r, self.window)
             wf = np.broadcast_to(f1, (n,) + f1.shape)
         else:
-            F = np.stack([np.stack([np.asarray(col(a, w), np.complex128)
-                                    for a in (Exx, Eyy, Ezz, Vrr)]) for w in range(w0, nw)])
+            # columns w0 .. Nw - 1 of each field, [4][Nx][n] -> [n][4][Nx]
+            col(Exx, nw - 1), col(Eyy, nw - 1), col(Ezz, nw - 1), col(Vrr, nw - 1)
+            F = np.stack([np.broadcast_to(a[:, None], a.shape + (n,)) if a.ndim == 1
+                          else a[:, w0:nw] for a in (np.asarray(a, np.complex128)
+                                                     for a in (Exx, Eyy, Ezz, Vrr))])
+            F = np.ascontiguousarray(F.transpose(2, 0, 1))
             wf = wirespace.prop2qw_rows(rr, F.reshape(4 * n, -1), self.r,
                                         self.window).reshape(n, 4, -1)
         if self.full is None and not self._many_body and all(

@@ -32,15 +32,36 @@ QW_SMALL = 1e-100  # QWOptics._small (qwoptics.py:604)
 def fftg(F):
     """FFTG in place: alternate-sign shift, FFT, shift, -F/N.  F is one
     signal or (m, n) rows of signals."""
+    if _centred(F, np.fft.fft, 1):
+        return
     F[..., 1::2] = -F[..., 1::2]
     F[...] = np.fft.fft(F, axis=-1)
     F[..., 1::2] = -F[..., 1::2]
     F[...] = -F / float(F.shape[-1])
 
 
+def _centred(F, fft, stage):
+    """fftg / ifftg of one contiguous complex128 block: the transform in place
+    between the library's two sign-and-scale passes (psb_centred_c128: the
+    operations below, the same bits).  False when F is laid out otherwise."""
+    if not (isinstance(F, np.ndarray) and F.dtype == np.complex128 and F.flags.c_contiguous
+            and F.flags.writeable and F.ndim >= 1 and 0 < F.size < 2**31):
+        return False
+    from . import _lib
+
+    n = F.shape[-1]
+    m = F.size // n
+    _lib.call("psb_centred_c128", F.ctypes.data, m, n, 0)
+    fft(F, axis=-1, out=F)
+    _lib.call("psb_centred_c128", F.ctypes.data, m, n, stage)
+    return True
+
+
 def ifftg(F):
     """iFFTG in place: alternate-sign shift, inverse FFT, shift, -F*N.  F is
     one signal or (m, n) rows of signals."""
+    if _centred(F, np.fft.ifft, 2):
+        return
     F[..., 1::2] = -F[..., 1::2]
     F[...] = np.fft.ifft(F, axis=-1)
     F[..., 1::2] = -F[..., 1::2]
@@ -173,8 +194,9 @@ def rescale_1d(x0, z0, x1):
 def prop2qw_rows(RR, F, R, window):
     """prop2qw of (m, len(RR)) rows of propagation-space fields at once:
     (m, len(R)) windowed, real, transformed wire-space fields."""
-    f = rescale_rows(RR, F, R) * window
-    f = np.real(f).astype(np.complex128)
+    f = rescale_rows(RR, F, R)
+    f *= window
+    f.imag[...] = 0.0
     fftg(f)
     return f
 
@@ -205,9 +227,11 @@ def rho_post_rows(A, N, dr):
     row gets the bits of its own rho_post call."""
     nr = A.shape[-1]
     tot = np.sum(np.abs(N), axis=-1) + 1e-50
-    A[...] = A - (np.real(np.sum(A[:, 0:10], axis=-1) + np.sum(A[:, nr - 10:nr], axis=-1))
-                  / 20.0)[:, None]
-    A[...] = A * tot[:, None] / (np.sum(np.abs(A), axis=-1) * dr + QW_SMALL)[:, None]
+    A -= (np.real(np.sum(A[:, 0:10], axis=-1) + np.sum(A[:, nr - 10:nr], axis=-1))
+          / 20.0)[:, None]
+    norm = np.sum(np.abs(A), axis=-1) * dr + QW_SMALL
+    A *= tot[:, None]
+    A /= norm[:, None]
     fftg(A)
 
 
