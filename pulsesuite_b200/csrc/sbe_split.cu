@@ -71,11 +71,11 @@
 // and now:
 //   Nk        64    128    256    512   1024
 //   W = 4   2.09   2.41   3.92  11.32   35.1
-//           1.70   1.96   3.15   7.55   21.0
+//           1.70   1.92   3.17   7.51   20.8
 //   W = 8   3.16   3.76   6.27  18.52   50.9
-//           2.52   2.94   5.15  14.54   40.6
+//           2.51   2.87   5.04  14.30   39.4
 //   W = 16  6.30   6.69  16.87  37.41
-//           4.03   4.70  12.11  26.00
+//           4.02   4.66  11.90  25.56
 // Tried and slower: 8 epilogue warps with twice the registers (Nk 256, W = 8:
 // 5.9), column maxima by redux.sync (~32 cycles each: Nk 64, W = 16 4.07 to
 // 4.58) or by votes against the last exponent (+4 %), band energies loaded at
@@ -115,12 +115,20 @@ constexpr int kRegsHigh = 96;
 static_assert(kEpiWarps * kRegsHigh + 4 * kRegsGen + 4 * kRegsMma <= 24 * kRegsLaunch,
               "register split exceeds the launch allocation");
 
-// Byte offset of element (k, col) in one digit plane of X (K-major: 16 k of
-// a column contiguous in a core-matrix row, 8 columns per core matrix; core
-// matrices at 128 B along k, column groups at sbo = 8 kpad).
+// Byte offset of element (k, col) in one digit plane of X, K-major with the
+// 32-byte swizzle: 32 k of a column are a row of two 16-byte chunks, eight
+// columns an atom of 256 B in which the columns 4..7 have their chunks
+// exchanged; atoms at 256 B along k, column groups at sbo = 8 kpad.  A warp's
+// 32 lanes (32 k of one column) so store their bytes to 32 adjacent ones; as
+// two core matrices of 16 k the halves fell on the same banks (1-2.5 % of a
+// stage: Nk 256, W = 8 5.12 -> 5.04 us, Nk 1024 40.4 -> 39.4).
 __device__ __forceinline__ uint32_t x_off(int k, int col, uint32_t sbo) {
-  return (uint32_t)((col >> 3) * sbo + (k >> 4) * 128 + (col & 7) * 16 + (k & 15));
+  return (uint32_t)((col >> 3) * sbo + (k >> 5) * 256 + (col & 7) * 32 +
+                    ((((k >> 4) ^ (col >> 2)) & 1) << 4) + (k & 15));
 }
+
+// Layout type of a shared-memory matrix descriptor: 32-byte swizzle.
+constexpr uint64_t kSwizzle32 = 6ull << 61;
 
 // TMEM columns: accumulator sets of a row tile (D2, D3, D4: 3 N columns), then
 // the A slots (3 digit planes each), in one of three arrangements:
@@ -592,7 +600,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
       if (elect_one()) {
         // B descriptor of X[s & 1] at k' = 0; +32 per 64-wide slice, +16 per
         // K step (start address in 16-byte units: 256 B per 32 k')
-        const uint64_t bdesc0 = smem_desc(smem_u32(xbase + (s & 1) * L.xbuf), 128, xsbo);
+        const uint64_t bdesc0 = smem_desc(smem_u32(xbase + (s & 1) * L.xbuf), 16, xsbo) | kSwizzle32;
         // one 64-wide K slice into the accumulator set at d2: K step 0 (the
         // row tile's first slice overwrites its accumulators), then K step 1
         auto slice = [&](uint32_t d2, uint32_t a1, uint64_t bd, bool acc) {
@@ -833,7 +841,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
         band(mi + 1 < nM ? mi + 1 : 0);  // the next row's, used a tile later
         // this lane's row takes part in this tile (abort read once per tile)
         const bool live = got && k < nk && !*abort;
-        const uint32_t kofs = (uint32_t)(k >> 4) * 128 + (uint32_t)(k & 15);
+        const uint32_t kofs = (uint32_t)(k >> 5) * 256 + (uint32_t)(k & 31);
         constexpr int JW = WH < 2 ? WH : 2;  // wires of one TMEM read
 #pragma unroll
         for (int jp = 0; jp < WH; jp += JW) {
@@ -918,13 +926,14 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
             // digits of the next stage point with the lagged column scales
             const float4 sc = *reinterpret_cast<const float4*>(scw + 4 * w);
             const float xv[4] = {nxt.x * sc.x, nxt.y * sc.y, nxt.z * sc.z, nxt.w * sc.w};
-            // x_off(k, 4w + c): columns 4w..4w+3 share a core matrix
-            const uint32_t obase = (uint32_t)(w >> 1) * xsbo + (uint32_t)(w & 1) * 64 + kofs;
+            // x_off(k, 4w + c): columns 4w..4w+3 are half an atom
+            const uint32_t obase =
+                (uint32_t)(w >> 1) * xsbo + (uint32_t)(w & 1) * 128 + (kofs ^ (16u * (w & 1)));
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
               int d1, d2, d3;
               digits3(xv[c], d1, d2, d3);
-              const uint32_t o = obase + 16 * c;
+              const uint32_t o = obase + 32 * c;
               xn[o] = (uint8_t)d1;
               xn[L.plane + o] = (uint8_t)d2;
               xn[2 * L.plane + o] = (uint8_t)d3;
