@@ -18,6 +18,28 @@ from scipy.constants import hbar
 from . import _lib, abi, coulomb, device
 
 
+def wire_cost(nk):
+    """Time of one wire and stage in a full group of the per-wire split kernel,
+    relative (2.2, 2.3, 2.9, 5.0, 11.7 us at Nk 64, 128, 256, 512, 1024)."""
+    return 2.0 + 2.6e-3 * nk + 6.5e-6 * nk * nk
+
+
+def wire_group(n, wmax, sms):
+    """Wires per group of the per-wire split kernel for n wires of one grid on
+    its share of the SMs: the fewest waves of CTAs times a CTA's time, which
+    grows as w + 1 (Nk 512: one wire 8.8 us a stage, ten 50).  Against the
+    largest group that a full wave of CTAs leaves, 8 steps of screened wires:
+    1600 at Nk 512 3.37 -> 2.12 ms (2 waves of 6, not 2 of 10 with a second of
+    12 CTAs), 16384 20.1 -> 19.2, 1024 of Nk 64..512 1.61 -> 1.11 (15 grids
+    on ten SMs each, not one wire per CTA)."""
+    sms = max(1, int(round(sms)))
+
+    def time(w):
+        return -(-(-(-n // w)) // sms) * (w + 1)
+
+    return min(range(1, wmax + 1), key=lambda w: (time(w), -w))
+
+
 class WireBatch:
     """``form`` selects the step kernel: "plain" (FP64 throughout,
     psb_rk4_f64) or "split" (exchange sums on the int8 tensor cores as exact
@@ -106,8 +128,8 @@ class WireBatch:
 
         Screened grids and grids with distinct Veh, Vee, Vhh use
         psb_rk4_split_wire (one matrix per wire, the wires of a group
-        contracted one after another): W is the largest group that fits, but
-        no more wires per CTA than a full wave of CTAs leaves
+        contracted one after another): W by ``wire_group``, each grid on the
+        share of the SMs that its wires' work has in the batch
         (``split_w`` overrides it, 1 .. psb_split_wire_max_group).
 
         All classes run concurrently on side streams, the one with the
@@ -122,6 +144,11 @@ class WireBatch:
         counts = np.bincount(self.h_wires["table"], minlength=len(nks))
         sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
         target = float(np.sum(counts * nks.astype(np.float64) ** 2)) / (2.0 * sms)
+        # the per-wire kernel's work in this batch, by which its grids share the SMs
+        per_wire_t = [(f[t] & abi.PSB_TAB_SCREENED) or not (f[t] & abi.PSB_TAB_SHARED_V)
+                      for t in range(len(nks))]
+        wire_work = sum(wire_cost(int(nks[t])) * int(counts[t]) for t in range(len(nks))
+                        if per_wire_t[t]) or 1.0
         classes = {}
         wclasses = {}
         for t in np.argsort(-nks, kind="stable"):
@@ -137,7 +164,7 @@ class WireBatch:
                 if wmax < 1:
                     raise _lib.PsbError(f"split form: nk {nk} exceeds the supported maximum "
                                         "for screened or distinct Coulomb matrices")
-                wg = max(1, min(wmax, -(-len(ws) // sms)))
+                wg = wire_group(len(ws), wmax, sms * wire_cost(nk) * len(ws) / wire_work)
                 if nk in self.split_w:
                     wg = int(self.split_w[nk])
                     if not 1 <= wg <= wmax:
