@@ -59,16 +59,16 @@ L2_FLUSH_BYTES = 256 << 20
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of the step
 # kernels, from one ncu capture of a 20-step call on the configuration-4
 # request mix (16384 solves; profiles/split_rk4_kernel_c4_mix.md,
-# profiles/sbe_f64_kernel_c4_mix.md):
+# profiles/sbe_conv_kernel_c4_mix.md):
 #   split, state resident in shared memory: per element and launch (the
 #     FP64 state read once and written once)
 #   split, state in the workspace (groups whose grid does not fit shared
 #     memory): per element and time step (the FP32 stage state streams
 #     through L2 and, beyond its capacity, DRAM every stage)
 #   plain: per element and launch
-DRAM_SPLIT_RES_PER_ELEMENT = 75.0e6 / 1.770048e6
-DRAM_SPLIT_WS_PER_ELEMENT_STEP = 2.043e9 / (2.116608e6 * 20)
-DRAM_PLAIN_PER_ELEMENT = (72.03e6 + 43.39e6) / (1.770048e6 + 1.267712e6)
+DRAM_SPLIT_RES_PER_ELEMENT = 112.0e6 / 3.037760e6
+DRAM_SPLIT_WS_PER_ELEMENT_STEP = 0.8996e9 / (0.848896e6 * 20)
+DRAM_PLAIN_PER_ELEMENT = 133.0e6 / 3.886656e6
 TRAFFIC_SOURCE = ("ncu dram bytes per element (resident state, per launch) and per element "
                   "and step (workspace state) of a 20-step capture on the c4 mix, applied to "
                   "this step's launches")

@@ -60,8 +60,8 @@ extern "C" {
 #define PSB_TAB_SHARED_V 4 /* Veh == Vee == Vhh (one table serves all three sums)        */
 /* In a launch's tab_flags only: every wire's nk lies in the size class of
  * nkmax (2..64, 65..128, 129..256, 257..512, 513..1024), so one kernel of
- * that class serves the launch; a wire of another class may be refused with PSB_ERR_SIZE.
- * Without it the FP64 entry points issue one kernel per class up to nkmax's. */
+ * that class serves the launch; a wire of another class may be refused
+ * with PSB_ERR_SIZE.  Without it the FP64 entry points issue one kernel per class up to nkmax's. */
 #define PSB_TAB_ONE_CLASS 8
 
 /*

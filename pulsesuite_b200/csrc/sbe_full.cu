@@ -1196,7 +1196,7 @@ __device__ __forceinline__ double2 cm_rn(double2 a, double2 b) {
 // b) mod nk] it needs sit in shared memory, and a lane's eight sums share the
 // operand that varies along the columns (the other is a broadcast).  Bound by
 // the FP64 pipe.  Each element sums with the summation index ascending.
-// 64 wires of Nk 114: 0.12 ms each, 0.23 with one element per thread.
+// 64 wires of Nk 114: 0.16 ms each, 0.23 with one element per thread.
 constexpr int kST = 16, kSB = 32, kSR = 8, kSThreads = kSB / kSR * 32;
 
 // ROWS: T[x][a][j] = sum_b X3[x][a][b] s[(j - b) mod nk], into tr;

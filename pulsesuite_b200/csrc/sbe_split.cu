@@ -985,7 +985,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_rk4_kernel(Args a) {
   }
 
   // ---- teardown -----------------------------------------------------------------
-  // every MMA of every issuer has completed before TMEM is released
+  // every MMA has completed before TMEM is released
   if (warp == kMmaWarp && elect_one()) umma_commit(final_bar);
   if (warp == kMmaWarp && lane == 0) {
     bool done = false;

@@ -45,11 +45,15 @@ class Workload:
         return int(self.nks.sum())
 
     def flops_per_step(self):
-        """Algorithmic FP64 flops of one RK4 step of the batch: per unit
-        32 Nk + 150 (4 right-hand sides of 8 Nk exchange flops plus ~30
-        elementwise flops each, plus the RK combination)."""
+        """Algorithmic FP64 flops of one RK4 step of the batch: 4 right-hand
+        sides whose exchange sums take 8 Nk^2 flops directly or, where that
+        is less, four transforms of 2 Nk points (5 M log2 M each) and their
+        product with the tables' spectra; plus ~30 elementwise flops per
+        point each, and the RK combination."""
         nk = self.nks.astype(np.float64)
-        return float(np.sum(nk * (32.0 * nk + 150.0)))
+        m = 2.0 * nk
+        sums = np.minimum(8.0 * nk * nk, 4 * 5.0 * m * np.log2(m) + 4 * m)
+        return float(np.sum(4.0 * sums + 150.0 * nk))
 
 
 def _grids_for(nks):
