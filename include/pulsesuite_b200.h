@@ -61,7 +61,8 @@ extern "C" {
 /* In a launch's tab_flags only: every wire's nk lies in the size class of
  * nkmax (2..64, 65..128, 129..256, 257..512, 513..1024), so one kernel of
  * that class serves the launch; a wire of another class may be refused
- * with PSB_ERR_SIZE.  Without it the FP64 entry points issue one kernel per class up to nkmax's. */
+ * with PSB_ERR_SIZE.  Without it the FP64 entry points issue one kernel per
+ * class up to nkmax's. */
 #define PSB_TAB_ONE_CLASS 8
 
 /*
@@ -461,8 +462,8 @@ int psb_centred_c128(double* f, int m, int n, int stage);
  */
 #define PSB_SPLIT_WMAX 16
 /* One CTA's work: 1..wgroup wires of one table (same k grid); wire slots
- * past nw are ignored.  wgroup is 4, 8 or 16 (wider groups make every MMA
- * wider at the same issue cost; 16 needs nk <= psb_split_max_nk(16)). */
+ * past nw are ignored.  wgroup is 4, 8 or 16 (16 needs
+ * nk <= psb_split_max_nk(16)). */
 typedef struct PsbSplitGroup {
   int32_t table;
   int32_t nw;

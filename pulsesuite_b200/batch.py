@@ -20,8 +20,8 @@ from . import _lib, abi, coulomb, device
 
 def wire_cost(nk):
     """Time of one wire and stage in a full group of the per-wire split kernel,
-    relative (2.2, 2.3, 2.9, 5.0, 11.7 us at Nk 64, 128, 256, 512, 1024)."""
-    return 2.0 + 2.6e-3 * nk + 6.5e-6 * nk * nk
+    relative (2.2, 2.3, 2.9, 4.6, 10.7 us at Nk 64, 128, 256, 512, 1024)."""
+    return 2.0 + 2.6e-3 * nk + 6.0e-6 * nk * nk
 
 
 def wire_group(n, wmax, sms):

@@ -50,8 +50,9 @@
 //                digits of the next stage point, the n1D and P(t) sums; for
 //                screened tables, then n1D -> eps(q) (coulomb.py:1172-1193)
 //                -> V/eps and VS of the wire's next stage;
-//   warps 16..19 A-tile generators; for a screened wire they first write
-//                the digits of its V/eps / VS into its byte arrays;
+//   warps 16..19 A-tile generators; for a screened wire of Nk <= 256 they
+//                first write the digits of its V/eps / VS into its byte
+//                arrays, which above that the team does;
 //   warps 20..23 MMA issuers (one elected lane each), one per row tile mi
 //                (mod 4); warp 20 owns TMEM.
 // What bounds it: up to Nk 256 the epilogue, a chain of ~8000 cycles a wire
@@ -59,8 +60,8 @@
 // of eps) that the second team hides; from Nk 512 the generators (~500
 // cycles a tile, 14 tiles a wire and stage).  us per wire-stage of a screened
 // CTA, one team of 8 epilogue warps -> now: Nk 64 4.1 -> 2.2, 128 4.0 ->
-// 2.3, 256 4.5 -> 2.9, 512 6.5 -> 5.0, 1024 15.6 -> 11.7; distinct screened
-// matrices, Nk 300: 9.9 -> 8.5.  Tried and slower: eight generator warps (72
+// 2.3, 256 4.5 -> 2.9, 512 6.5 -> 4.6, 1024 15.6 -> 10.7; distinct screened
+// matrices, Nk 300: 9.9 -> 7.4.  Tried and slower: eight generator warps (72
 // registers at launch: Nk 128 +7 %, Nk 512 -2 %), two digit planes in flight
 // per generator (Nk 512 +4 %).
 // While one wire's epilogue and table run, the tensor cores work on the
@@ -330,6 +331,11 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
     return;
   }
   const int nk = tb.nk, nw = grp.nw, kpad = kpad_of(nk), nM = mtiles_of(nk);
+  // Who writes the digits of a wire's V/eps: the generators while the epilogue
+  // sets the pace, its team from three row tiles on, where they do (the
+  // pass and its hand-over are 1600 of their 10000 cycles a wire at Nk 512:
+  // 5.0 -> 4.6 us a wire-stage; at Nk 128 the team would be 5 % slower).
+  const bool epi_digits = scr && nM > 2;
   const int nK = kpad / kTileK;
   const WLayout<NT> L(nk, a.wgroup, scr);
   const int nslot = slots_of<NT>(nk), G = nslot / 2;
@@ -382,7 +388,7 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
     mbar_init(final_bar, kIssuers);
     for (int j = 0; j < kMaxW; ++j) {
       mbar_init(&xfull[j], kTeamWarps);
-      mbar_init(&svfull[j], 1);
+      mbar_init(&svfull[j], epi_digits ? kTeamWarps : 1);
       mbar_init(&gdone[j], kGenWarps);
     }
     *abort = 0;
@@ -620,19 +626,21 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
     for (int s = 0; s < total_stages && go; ++s) {
       for (int j = 0; j < nw && go; ++j) {
         if (scr && s >= 1) {
-          // the wire's next-stage digits, from the V/eps the epilogue wrote
+          // the wire's next-stage digits, or the V/eps they follow from, are there
           go = __all_sync(0xffffffffu, mbar_wait_sleep(&svfull[j], (s - 1) & 1, abort, lim));
           if (!go) break;
-          table_digits<NT>(svb + (uint32_t)j * (L.svsz / 8), vsw + 3 * j, nk, (int)c0,
-                           tabq + (uint32_t)(j * NT) * L.tabsz, L.plane, 32 * kGenWarp0,
-                           32 * kGenWarps);
-          // all four warps' digits are written before any tile reads them (a
-          // bounded mbarrier, not a named barrier: a warp that stops on an
-          // abort must not leave the others waiting)
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&gdone[j]);
-          go = __all_sync(0xffffffffu, mbar_wait(&gdone[j], (s - 1) & 1, abort, lim));
-          if (!go) break;
+          if (!epi_digits) {
+            table_digits<NT>(svb + (uint32_t)j * (L.svsz / 8), vsw + 3 * j, nk, (int)c0,
+                             tabq + (uint32_t)(j * NT) * L.tabsz, L.plane, 32 * kGenWarp0,
+                             32 * kGenWarps);
+            // all four warps' digits are written before any tile reads them (a
+            // bounded mbarrier, not a named barrier: a warp that stops on an
+            // abort must not leave the others waiting)
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&gdone[j]);
+            go = __all_sync(0xffffffffu, mbar_wait(&gdone[j], (s - 1) & 1, abort, lim));
+            if (!go) break;
+          }
         }
         const uint8_t* tq = tabq + (scr ? (uint32_t)(j * NT) * L.tabsz : 0u);
         for (int d0 = dmin; d0 <= dmax; d0 += G) {
@@ -928,7 +936,15 @@ __global__ void __launch_bounds__(kThreadsS, 1) split_wire_kernel(Args a) {
           table_scaled<NT>(qcs, vts, nk, true, n1d, svb + (uint32_t)j * (L.svsz / 8), vsw + 3 * j,
                            sred + 4 * kTeamWarps * team, team * kTeamThreads, kTeamThreads,
                            1 + team);
-          if (ttid == 0) mbar_arrive(&svfull[j]);
+          if (epi_digits) {
+            table_digits<NT>(svb + (uint32_t)j * (L.svsz / 8), vsw + 3 * j, nk, (int)c0,
+                             tabq + (uint32_t)(j * NT) * L.tabsz, L.plane,
+                             team * kTeamThreads, kTeamThreads);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&svfull[j]);
+          } else if (ttid == 0) {
+            mbar_arrive(&svfull[j]);
+          }
         }
       }
     }
