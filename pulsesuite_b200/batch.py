@@ -187,13 +187,15 @@ class WireBatch:
                     raise _lib.PsbError(f"split form: nk {nk} exceeds the supported maximum")
                 key = (wg, nk <= resnk[wg])
                 target_classes = classes
-            for i in range(0, len(ws), wg):
-                g = np.zeros(1, dtype=abi.SPLIT_GROUP_DTYPE)
-                g["table"] = t
-                g["nw"] = len(ws[i:i + wg])
-                g["wire"][0, :] = -1
-                g["wire"][0, :g["nw"][0]] = ws[i:i + wg]
-                target_classes.setdefault(key, []).append(g)
+            g = np.zeros(-(-len(ws) // wg), dtype=abi.SPLIT_GROUP_DTYPE)
+            g["table"] = t
+            g["nw"] = wg
+            g["nw"][-1] = len(ws) - (len(g) - 1) * wg
+            slots = np.full(len(g) * wg, -1, dtype=np.int64)
+            slots[:len(ws)] = ws
+            g["wire"] = -1
+            g["wire"][:, :wg] = slots.reshape(len(g), wg)
+            target_classes.setdefault(key, []).append(g)
         self.split_launches = []
         for key in classes:
             ga = np.concatenate(classes[key])

@@ -76,8 +76,9 @@
 //           2.51   2.87   5.04  14.30   39.4
 //   W = 16  6.30   6.69  16.87  37.41
 //           4.02   4.66  11.90  25.56
-// Tried and slower: 8 epilogue warps with twice the registers (Nk 256, W = 8:
-// 5.9), column maxima by redux.sync (~32 cycles each: Nk 64, W = 16 4.07 to
+// Tried and slower: eight generator warps for the classes whose state is in
+// the workspace (72 registers at launch; Nk 1024, W = 8: 59), 8 epilogue warps
+// with twice the registers (Nk 256, W = 8: 5.9), column maxima by redux.sync (~32 cycles each: Nk 64, W = 16 4.07 to
 // 4.58) or by votes against the last exponent (+4 %), band energies loaded at
 // the row tile's start (Nk 256 +2 %).
 // Every mbarrier wait is bounded; on a timeout the CTA records
