@@ -101,11 +101,11 @@ class WireBatch:
             if (tf & abi.PSB_TAB_SHARED_V).all():
                 flags |= abi.PSB_TAB_SHARED_V
             self.classes.append((torch.as_tensor(sel, device="cuda"), int(nks[sel].max()), flags))
-        self.side_streams = []
+        most = len(self.classes)  # launches of one call: leapfrog's, rk4's
         if form == "split":
             self._setup_split()
-        elif len(self.classes) > 1:
-            self.side_streams = self._streams(len(self.classes))
+            most = max(most, len(self.split_launches) + len(self.wire_launches))
+        self.side_streams = self._streams(most) if most > 1 else []
         self.tab_flags = 0
         if (self.h_tables["flags"] & abi.PSB_TAB_SCREENED).any():
             self.tab_flags |= abi.PSB_TAB_SCREENED
@@ -210,7 +210,6 @@ class WireBatch:
             nkmax = int(nks[ga["table"]].max())
             self.wire_launches.append((key[0], device.to_device(ga), len(ga), nkmax, key[1]))
         self.wire_launches.sort(key=lambda l: -l[3])
-        self.side_streams = self._streams(len(self.split_launches) + len(self.wire_launches))
         self.ws = torch.zeros(int(lib.psb_split_ws_bytes(self.n_state)), dtype=torch.uint8,
                               device="cuda")
 
@@ -225,12 +224,13 @@ class WireBatch:
         """Run ``calls`` (one per class, each taking its stream) concurrently
         on the side streams, ordered after the work queued on ``stream``
         (default: the current stream) and before what follows on it; a single
-        class without a side stream runs on it."""
+        call runs on that stream itself."""
         main = stream if stream is not None else torch.cuda.current_stream()
-        if not self.side_streams:
-            for c in calls:
-                c(main)
+        if len(calls) == 1:
+            calls[0](main)
             return
+        if len(calls) > len(self.side_streams):
+            raise _lib.PsbError(f"{len(calls)} launches on {len(self.side_streams)} side streams")
         fork = torch.cuda.Event()
         fork.record(main)
         for c, s in zip(calls, self.side_streams):
