@@ -16,6 +16,20 @@ int set_error(int code, const char* fmt, ...);
 // Checks the last CUDA launch/runtime error; returns PSB_OK or PSB_ERR_CUDA.
 int check_cuda(const char* what);
 
+// Lets a kernel's launches use up to `limit` bytes of dynamic shared memory, if
+// this launch needs more than the 48 KB that every launch may use.  The limit is
+// a property of the kernel on the current device, shared by all host threads:
+// `limit` is the most that any launch of the kernel can ask for, the same in
+// every call, so that no thread lowers it between another's call and launch.
+template <class... A>
+int allow_smem(void (*kern)(A...), size_t bytes, size_t limit) {
+  if (bytes <= 48 * 1024) return PSB_OK;
+  const cudaError_t e =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
+  if (e == cudaSuccess) return PSB_OK;
+  return set_error(PSB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+}
+
 // ---------------------------------------------------------------------------
 // Bessel K0 as the reference evaluates it.
 //

@@ -821,12 +821,8 @@ template <int L, int MODE>
 int launch_lanes(const Batch& bt, int mode, int grid, bool screened, bool shared, bool check,
                  bool strict, cudaStream_t st) {
   const uint32_t smem = smem_of<L>(shared);
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(
-        sbe_conv_kernel<L, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess)
-      return set_error(PSB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-  }
+  const int rc = allow_smem(sbe_conv_kernel<L, MODE>, smem, Lay<L>::total3);
+  if (rc != PSB_OK) return rc;
   sbe_conv_kernel<L, MODE><<<grid, 32 * L, smem, st>>>(bt, mode, screened, shared, check, strict);
   return check_cuda("sbe_conv_kernel");
 }

@@ -355,21 +355,25 @@ size_t smem_bytes_for(int nk, int ntab) {
   return sizeof(double) * (size_t)smem_layout<kR>(g, ntab).total;
 }
 
-template <int MODE, bool SCREEN, int NT>
-static int launch_direct(const Batch& bt, int grid, int nkmax, bool check, cudaStream_t st) {
+// Shared memory of a launch over grids of up to nkmax points.
+static size_t smem_up_to(int nkmax, int ntab) {
   size_t smem = 0;
   for (int nk = 2; nk <= nkmax && nk <= kDirectNk; ++nk) {
-    const size_t b = smem_bytes_for(nk, NT);
+    const size_t b = smem_bytes_for(nk, ntab);
     if (b > smem) smem = b;
   }
-  auto kern = nkmax <= 128 ? sbe_f64_kernel<kR, MODE, SCREEN, NT, 4>
-                           : sbe_f64_kernel<kR, MODE, SCREEN, NT, 2>;
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(
-        kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess)
-      return set_error(PSB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-  }
+  return smem;
+}
+
+template <int MODE, bool SCREEN, int NT>
+static int launch_direct(const Batch& bt, int grid, int nkmax, bool check, cudaStream_t st) {
+  static const size_t most[2] = {smem_up_to(128, NT), smem_up_to(kDirectNk, NT)};
+  const bool small = nkmax <= 128;
+  auto kern =
+      small ? sbe_f64_kernel<kR, MODE, SCREEN, NT, 4> : sbe_f64_kernel<kR, MODE, SCREEN, NT, 2>;
+  const size_t smem = smem_up_to(nkmax, NT);
+  const int rc = allow_smem(kern, smem, most[small ? 0 : 1]);
+  if (rc != PSB_OK) return rc;
   kern<<<grid, kThreads, smem, st>>>(bt, check);
   return check_cuda("sbe_f64_kernel");
 }

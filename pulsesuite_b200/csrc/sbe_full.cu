@@ -25,8 +25,6 @@
 // Every sum runs in the reference's order; results agree with it to
 // rounding (numpy's pairwise sums and the kernels' sequential ones differ
 // in the last bits).
-#include <mutex>
-
 #include "dmma.cuh"
 #include "psb_common.cuh"
 
@@ -1458,40 +1456,29 @@ int check_mb(const PsbFullMB* mb, bool deph, bool relax, bool dct) {
   return PSB_OK;
 }
 
+template <int TM>
+int launch_derivs_tm(const full::Step& s, int nw, cudaStream_t st) {
+  constexpr size_t sm = (size_t)full::kDStages * full::kDStage<TM> * sizeof(double2);
+  const int n = (s.nk + TM - 1) / TM, rc = allow_smem(full::derivs_kernel<TM>, sm, sm);
+  if (rc != PSB_OK) return rc;
+  full::derivs_kernel<TM><<<dim3(n, nw, n), TM * 8, sm, st>>>(s);
+  return PSB_OK;
+}
 // Blocks of 32 x 32 elements once they fill the GPU twice over, else of
 // 16 x 16: 64 wires of Nk 114 have 1024 blocks of 32, one wire 16 (64 of 16).
 int launch_derivs(const full::Step& s, int nw, cudaStream_t st) {
-  static std::once_flag once;
-  static cudaError_t attr = cudaSuccess;
-  constexpr size_t sm32 = (size_t)full::kDStages * full::kDStage<32> * sizeof(double2);
-  constexpr size_t sm16 = (size_t)full::kDStages * full::kDStage<16> * sizeof(double2);
-  std::call_once(once, [] {
-    attr = cudaFuncSetAttribute(full::derivs_kernel<32>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm32);
-    if (attr == cudaSuccess)
-      attr = cudaFuncSetAttribute(full::derivs_kernel<16>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm16);
-  });
-  if (attr != cudaSuccess) return set_error(PSB_ERR_CUDA, "derivs_kernel: shared memory");
-  const int n32 = (s.nk + 31) / 32, n16 = (s.nk + 15) / 16;
-  if ((int64_t)n32 * n32 * nw >= 592)
-    full::derivs_kernel<32><<<dim3(n32, nw, n32), 256, sm32, st>>>(s);
-  else
-    full::derivs_kernel<16><<<dim3(n16, nw, n16), 128, sm16, st>>>(s);
-  return PSB_OK;
+  const int n32 = (s.nk + 31) / 32;
+  return (int64_t)n32 * n32 * nw >= 592 ? launch_derivs_tm<32>(s, nw, st)
+                                        : launch_derivs_tm<16>(s, nw, st);
 }
 
 // mb_offd_kernel with 8 wires per CTA where the batch has them
 int launch_offd(const full::MBView& v, int nk, int nw, cudaStream_t st) {
   const int W = nw >= 4 ? 8 : 1, th = 128;
   auto kern = W == 8 ? full::mb_offd_kernel<8> : full::mb_offd_kernel<1>;
-  const size_t sm = (size_t)nk * (2 + 2 * W) * 8;
-  if (sm > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(
-        kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess)
-      return set_error(PSB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-  }
+  const size_t per_k = (2 + 2 * (size_t)W) * 8, sm = nk * per_k;
+  const int rc = allow_smem(kern, sm, PSB_MAX_NK * per_k);
+  if (rc != PSB_OK) return rc;
   const int nd = (2 * nk + 1) * nk;
   kern<<<dim3((nd + th - 1) / th, (nw + W - 1) / W), th, sm, st>>>(v, nw);
   return PSB_OK;
@@ -1501,12 +1488,8 @@ int launch_offd(const full::MBView& v, int nk, int nw, cudaStream_t st) {
 template <int NT>
 int launch_scatter_nt(const full::MBView& v, int nk, int nw, cudaStream_t st) {
   const size_t sm = (size_t)full::kScK * full::sc_ld(NT) * 8;
-  if (sm > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(
-        full::mb_scatter_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess)
-      return set_error(PSB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-  }
+  const int rc = allow_smem(full::mb_scatter_kernel<NT>, sm, sm);
+  if (rc != PSB_OK) return rc;
   full::mb_scatter_kernel<NT>
       <<<dim3(2 * nk - 1, 4, (nw + 8 * NT - 1) / (8 * NT)), 32 * full::kScWarps, sm, st>>>(v, nw);
   return PSB_OK;
@@ -1601,18 +1584,14 @@ int full_launch(const Launch& a, cudaStream_t st) {
     s.st_x3 = s.st_sc;
   }
   {
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-      attr = cudaFuncSetAttribute(full::calch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  227 * 1024);
-    });
-    if (attr != cudaSuccess) return set_error(PSB_ERR_CUDA, "calch_kernel: shared memory");
     // two CTAs per SM where that leaves several diagonals in one
+    constexpr size_t most = 110 * 1024;  // (one diagonal of the largest grid fits)
     int nd = full::kHDiags;
-    while (nd > 1 && full::h_smem(nk, nd) > 110 * 1024) nd /= 2;
-    full::calch_kernel<<<dim3((2 * nk - 1 + nd - 1) / nd, nw), 32 * nd, full::h_smem(nk, nd),
-                         st>>>(s);
+    while (nd > 1 && full::h_smem(nk, nd) > most) nd /= 2;
+    const size_t sm = full::h_smem(nk, nd);
+    rc_ = allow_smem(full::calch_kernel, sm, most);
+    if (rc_ != PSB_OK) return rc_;
+    full::calch_kernel<<<dim3((2 * nk - 1 + nd - 1) / nd, nw), 32 * nd, sm, st>>>(s);
   }
   // dephasing from the level the right-hand side reads (SBEs.py:5225-5232)
   if (mb && mb->diag_dph) {
@@ -1767,15 +1746,9 @@ int launch_sources(int nw, int nk, int nr, const double* kr, const double* r,
   const int R = wide ? 8 : 4;
   auto dens = wide ? full::densities_kernel<8> : full::densities_kernel<4>;
   const size_t sp = (size_t)2 * (2 * nk - 1) * 16, sd = (size_t)R * nk * 16;
-  const size_t big = sp > sd ? sp : sd;
-  if (big > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(full::polarisation_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(dens, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sd);
-    if (e != cudaSuccess)
-      return set_error(PSB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-  }
+  int rc = allow_smem(full::polarisation_kernel, sp, (size_t)2 * (2 * PSB_MAX_NK - 1) * 16);
+  if (rc == PSB_OK) rc = allow_smem(dens, sd, (size_t)R * PSB_MAX_NK * 16);
+  if (rc != PSB_OK) return rc;
   const double2* lv = reinterpret_cast<const double2*>(lev);
   double2* o = reinterpret_cast<double2*>(out);
   const int fit = (int)(sp / ((size_t)nk * 16));  // 3: warps of the general sums

@@ -1037,7 +1037,7 @@ int launch_res(Args a, int nkmax, cudaStream_t s) {
   // registers per thread at launch (an increase beyond what the warpgroups
   // gave down would never complete), so a build that differs is refused
   cudaFuncAttributes fa{};
-  cudaError_t e = cudaFuncGetAttributes(&fa, split_rk4_kernel<W, RES>);
+  const cudaError_t e = cudaFuncGetAttributes(&fa, split_rk4_kernel<W, RES>);
   if (e != cudaSuccess)
     return set_error(PSB_ERR_CUDA, "cudaFuncGetAttributes: %s", cudaGetErrorString(e));
   if (fa.numRegs != kRegsLaunch || fa.maxThreadsPerBlock < kThreadsS)
@@ -1045,10 +1045,8 @@ int launch_res(Args a, int nkmax, cudaStream_t s) {
                      "split_rk4_kernel built with %d registers per thread (needs %d) and at "
                      "most %d threads (needs %d)",
                      fa.numRegs, kRegsLaunch, fa.maxThreadsPerBlock, kThreadsS);
-  e = cudaFuncSetAttribute(split_rk4_kernel<W, RES>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess)
-    return set_error(PSB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  const int rc = allow_smem(split_rk4_kernel<W, RES>, smem, kMaxDynSmem);
+  if (rc != PSB_OK) return rc;
   a.smem_bytes = smem;
   split_rk4_kernel<W, RES><<<a.ngroups, kThreadsS, smem, s>>>(a);
   return check_cuda("split_rk4_kernel");

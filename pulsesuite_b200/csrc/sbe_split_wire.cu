@@ -1003,7 +1003,7 @@ int launch_tiles(Args a, int nkmax, cudaStream_t s) {
                      a.wgroup);
   const uint32_t smem = WLayout<NT>(nkmax, a.wgroup, scr).total;
   cudaFuncAttributes fa{};
-  cudaError_t e = cudaFuncGetAttributes(&fa, split_wire_kernel<NT, MT>);
+  const cudaError_t e = cudaFuncGetAttributes(&fa, split_wire_kernel<NT, MT>);
   if (e != cudaSuccess)
     return set_error(PSB_ERR_CUDA, "cudaFuncGetAttributes: %s", cudaGetErrorString(e));
   if (fa.numRegs != kRegsLaunch || fa.maxThreadsPerBlock < kThreadsS)
@@ -1011,10 +1011,8 @@ int launch_tiles(Args a, int nkmax, cudaStream_t s) {
                      "split_wire_kernel built with %d registers per thread (needs %d) and at "
                      "most %d threads (needs %d)",
                      fa.numRegs, kRegsLaunch, fa.maxThreadsPerBlock, kThreadsS);
-  e = cudaFuncSetAttribute(split_wire_kernel<NT, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem);
-  if (e != cudaSuccess)
-    return set_error(PSB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  const int rc = allow_smem(split_wire_kernel<NT, MT>, smem, kMaxDynSmem);
+  if (rc != PSB_OK) return rc;
   a.smem_bytes = smem;
   split_wire_kernel<NT, MT><<<a.ngroups, kThreadsS, smem, s>>>(a);
   return check_cuda("split_wire_kernel");
