@@ -25,6 +25,8 @@
 // Every sum runs in the reference's order; results agree with it to
 // rounding (numpy's pairwise sums and the kernels' sequential ones differ
 // in the last bits).
+#include <type_traits>
+
 #include "dmma.cuh"
 #include "psb_common.cuh"
 
@@ -452,13 +454,33 @@ __global__ void __launch_bounds__(kLfThreads) leapfrog_kernel(Step s0) {
 // terms of one position after another, the diagonals d and -d together: nk^2 +
 // nk nr operations instead of nk^2 nr.  gridDim.x CTAs share the positions of a
 // wire; each makes its own diagonal sums.  Phases advance by a rotation of 32
-// dk r from an exact first value per lane.  Any other k grid takes the sums
-// over (i, c) as they stand, a warp per position.
+// dk r from an exact first value per lane.  On any other k grid
+// densities_kernel takes the sums over (i, c) as they stand, beside its own.
+
+// Whether kr[k] = kr[0] + k dk for all k; every thread of the CTA calls it (a
+// barrier).  Two kernels ask, so its rounding is spelled out.
+__device__ __forceinline__ bool equidistant(int nk, const double* kr) {
+  const double k0 = kr[0], dk = (kr[nk - 1] - k0) / (nk - 1);
+  const double tol = 0x1p-47 * fmax(fabs(k0), fabs(kr[nk - 1]));
+  bool off = !(fabs(dk) > 0.0);
+  for (int k = threadIdx.x; k < nk; k += blockDim.x)
+    off |= !(fabs(kr[k] - fma((double)k, dk, k0)) <= tol);
+  return !__syncthreads_or(off);
+}
+
+// the three components at position r from the sums with and without Xcv's sign
+__device__ __forceinline__ void put_polarisation(double2* out, int nr, int r, double W, double dcv,
+                                                 double yw, double sgnw, double sx, double sp) {
+  out[r] = make_double2(W * dcv * sx, 0.0);
+  out[nr + r] = make_double2(W * yw * dcv * sp, 0.0);
+  out[2 * nr + r] = make_double2(W * sgnw * -dcv * sp, 0.0);
+}
+
 constexpr int kPolThreads = 512, kPolLanes = 128, kPolGroups = kPolThreads / kPolLanes;
 __global__ void __launch_bounds__(kPolThreads) polarisation_kernel(
     int nk, int nr, const double* kr, const double* rpos, const double* window, double dcv,
-    double yw, double sgnw, const double* wpar, const double2* lev, double2* out, int fit) {
-  extern __shared__ __align__(16) double2 ssm[];  // [2][2 nk - 1], or [fit][nk] phases
+    double yw, double sgnw, const double* wpar, const double2* lev, double2* out) {
+  extern __shared__ __align__(16) double2 ssm[];  // [2][2 nk - 1]
   const int nd = 2 * nk - 1, tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
   const int64_t w = blockIdx.y;
   const double2* p = lev + w * 3 * nk * nk;
@@ -467,44 +489,11 @@ __global__ void __launch_bounds__(kPolThreads) polarisation_kernel(
     yw = wpar[4 * w];
     sgnw = wpar[4 * w + 1];
   }
-  const double k0 = kr[0], dk = (kr[nk - 1] - k0) / (nk - 1);
-  const double tol = 0x1p-47 * fmax(fabs(k0), fabs(kr[nk - 1]));
-  bool off = !(fabs(dk) > 0.0);
-  for (int k = tid; k < nk; k += kPolThreads) off |= !(fabs(kr[k] - (k0 + k * dk)) <= tol);
-  const bool uniform = !__syncthreads_or(off);
+  if (!equidistant(nk, kr)) return;  // densities_kernel's
+  const double dk = (kr[nk - 1] - kr[0]) / (nk - 1);
   const int npos = (nr + gridDim.x - 1) / gridDim.x, r0 = blockIdx.x * npos,
             r1 = min(nr, r0 + npos);
   const double2 z = make_double2(0.0, 0.0);
-  auto store = [&](int r, double sx, double sp) {
-    const double W = window[r];
-    out[r] = make_double2(W * dcv * sx, 0.0);
-    out[nr + r] = make_double2(W * yw * dcv * sp, 0.0);
-    out[2 * nr + r] = make_double2(W * sgnw * -dcv * sp, 0.0);
-  };
-  if (!uniform) {
-    // `fit` warps have room for their position's phases
-    double2* ph = ssm + wp * nk;
-    for (int r = r0 + wp; wp < fit && r < r1; r += fit) {
-      for (int k = lane; k < nk; k += 32) {
-        double sn, cn;
-        sincos(kr[k] * rpos[r], &sn, &cn);
-        ph[k] = make_double2(cn, sn);
-      }
-      __syncwarp();
-      double sx = 0.0, sp = 0.0;
-      for (int c = lane; c < nk; c += 32)
-        for (int i = 0; i < nk; ++i) {
-          const double x = cm(cm(p[i * nk + c], ph[c]), cconj(ph[i])).x;
-          sx += ((i + 1) & 1) ? -x : x;  // conj(Xcv) / dcv at kh = i
-          sp += x;
-        }
-      sx = warp_sum(sx);
-      sp = warp_sum(sp);
-      if (lane == 0) store(r, sx, sp);
-      __syncwarp();
-    }
-    return;
-  }
   // diagonal sums: d = c - i at d + nk - 1; row groups add up in turn
   const int grp = tid / kPolLanes;
   for (int d0 = 0; d0 < nd; d0 += kPolLanes) {
@@ -547,7 +536,7 @@ __global__ void __launch_bounds__(kPolThreads) polarisation_kernel(
     }
     sx = warp_sum(sx);
     sp = warp_sum(sp);
-    if (lane == 0) store(r, sx, sp);
+    if (lane == 0) put_polarisation(out, nr, r, window[r], dcv, yw, sgnw, sx, sp);
   }
 }
 
@@ -558,12 +547,15 @@ __global__ void __launch_bounds__(kPolThreads) polarisation_kernel(
 // over the column k2 so the rows of C, D are read coalesced, each element once
 // for all R positions and four rows ahead, then a block reduction.  64 wires,
 // Nk 114, 230 positions: 0.29 ms (FP64 floor of these products 0.21), with the
-// polarisation 0.03 ms; 0.43 with all sums in one kernel of 4 positions.
+// polarisation 0.03 ms; 0.43 with all sums in one kernel of 4 positions.  On a
+// k grid that is not equidistant the same pass takes the polarisation's sums
+// over (i, c) too: 0.44 ms, one wire of Nk 288 0.17 (1.68 and 2.55 with three
+// warps of polarisation_kernel on them).
 constexpr int kSrcThreads = 128;
 template <int kSrcR>
 __global__ void __launch_bounds__(kSrcThreads) densities_kernel(
     int nk, int nr, const double* kr, const double* rpos, const double* window, double L,
-    const double2* lev, double2* out) {
+    double dcv, double yw, double sgnw, const double* wpar, const double2* lev, double2* out) {
   extern __shared__ double2 ph[];  // [kSrcR][nk]
   __shared__ double red[kSrcR][4][kSrcThreads / 32];
   const int n2 = nk * nk, r0 = blockIdx.x * kSrcR;
@@ -577,41 +569,60 @@ __global__ void __launch_bounds__(kSrcThreads) densities_kernel(
     sincos(kr[k] * rpos[r], &sn, &cn);
     ph[e] = make_double2(cn, sn);
   }
-  __syncthreads();
+  const bool even = equidistant(nk, kr);  // (a barrier)
   const double2* C = lev + n2;
   const double2* D = lev + 2 * n2;
   double2 se[kSrcR], sh[kSrcR];
+  double sx[kSrcR], sp[kSrcR];
 #pragma unroll
-  for (int j = 0; j < kSrcR; ++j) se[j] = sh[j] = make_double2(0.0, 0.0);
-  for (int c = threadIdx.x; c < nk; c += kSrcThreads) {
-    double2 ec[kSrcR];
+  for (int j = 0; j < kSrcR; ++j) {
+    se[j] = sh[j] = make_double2(0.0, 0.0);
+    sx[j] = sp[j] = 0.0;
+  }
+  auto sums = [&](auto P) {
+    constexpr bool POL = decltype(P)::value;  // with the polarisation
+    for (int c = threadIdx.x; c < nk; c += kSrcThreads) {
+      double2 ec[kSrcR];
 #pragma unroll
-    for (int j = 0; j < kSrcR; ++j) ec[j] = ph[j * nk + c];
-    constexpr int kAhead = 4;
-    double2 cb[kAhead], db[kAhead];
-#pragma unroll
-    for (int u = 0; u < kAhead; ++u) {
-      const int i = min(u, nk - 1);
-      cb[u] = C[i * nk + c];
-      db[u] = D[i * nk + c];
-    }
-    for (int i0 = 0; i0 < nk; i0 += kAhead) {
+      for (int j = 0; j < kSrcR; ++j) ec[j] = ph[j * nk + c];
+      constexpr int kAhead = 4;
+      double2 cb[kAhead], db[kAhead], pb[kAhead];
 #pragma unroll
       for (int u = 0; u < kAhead; ++u) {
-        const int i = i0 + u, n = min(i + kAhead, nk - 1);
-        const double2 cv = cb[u], dv = cconj(db[u]);
-        cb[u] = C[n * nk + c];
-        db[u] = D[n * nk + c];
-        if (i >= nk) break;
+        const int i = min(u, nk - 1);
+        cb[u] = C[i * nk + c];
+        db[u] = D[i * nk + c];
+        if (POL) pb[u] = lev[i * nk + c];
+      }
+      for (int i0 = 0; i0 < nk; i0 += kAhead) {
 #pragma unroll
-        for (int j = 0; j < kSrcR; ++j) {
-          const double2 ei = cconj(ph[j * nk + i]);
-          se[j] = ca(se[j], cm(cm(cv, ei), ec[j]));
-          sh[j] = ca(sh[j], cm(cm(dv, ei), ec[j]));
+        for (int u = 0; u < kAhead; ++u) {
+          const int i = i0 + u, n = min(i + kAhead, nk - 1);
+          const double2 cv = cb[u], dv = cconj(db[u]);
+          cb[u] = C[n * nk + c];
+          db[u] = D[n * nk + c];
+          const double2 pv = POL ? pb[u] : make_double2(0.0, 0.0);
+          if (POL) pb[u] = lev[n * nk + c];
+          if (i >= nk) break;
+#pragma unroll
+          for (int j = 0; j < kSrcR; ++j) {
+            const double2 ei = cconj(ph[j * nk + i]);
+            se[j] = ca(se[j], cm(cm(cv, ei), ec[j]));
+            sh[j] = ca(sh[j], cm(cm(dv, ei), ec[j]));
+            if (POL) {
+              const double x = cm(cm(pv, ec[j]), ei).x;
+              sx[j] += ((i + 1) & 1) ? -x : x;  // conj(Xcv) / dcv at kh = i
+              sp[j] += x;
+            }
+          }
         }
       }
     }
-  }
+  };
+  if (even)
+    sums(std::false_type{});
+  else
+    sums(std::true_type{});
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
 #pragma unroll
   for (int j = 0; j < kSrcR; ++j) {
@@ -636,6 +647,29 @@ __global__ void __launch_bounds__(kSrcThreads) densities_kernel(
       out[4 * nr + r] = make_double2(h * t[2], h * t[3]);
     }
   }
+  if (even) return;  // polarisation_kernel's
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kSrcR; ++j) {
+    const double ux = warp_sum(sx[j]), up = warp_sum(sp[j]);
+    if (lane == 0) {
+      red[j][0][wp] = ux;
+      red[j][1][wp] = up;
+    }
+  }
+  __syncthreads();
+  const int r = r0 + threadIdx.x;
+  if (threadIdx.x >= kSrcR || r >= nr) return;
+  double t[2] = {0.0, 0.0};
+  for (int u = 0; u < kSrcThreads / 32; ++u) {
+    t[0] += red[threadIdx.x][0][u];
+    t[1] += red[threadIdx.x][1][u];
+  }
+  if (wpar) {
+    yw = wpar[4 * w];
+    sgnw = wpar[4 * w + 1];
+  }
+  put_polarisation(out, nr, r, window[r], dcv, yw, sgnw, t[0], t[1]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1751,11 +1785,11 @@ int launch_sources(int nw, int nk, int nr, const double* kr, const double* r,
   if (rc != PSB_OK) return rc;
   const double2* lv = reinterpret_cast<const double2*>(lev);
   double2* o = reinterpret_cast<double2*>(out);
-  const int fit = (int)(sp / ((size_t)nk * 16));  // 3: warps of the general sums
   const int nb = nw >= 148 ? 1 : (148 / nw < 16 ? 148 / nw : 16);
-  dens<<<dim3((nr + R - 1) / R, nw), full::kSrcThreads, sd, st>>>(nk, nr, kr, r, window, L, lv, o);
+  dens<<<dim3((nr + R - 1) / R, nw), full::kSrcThreads, sd, st>>>(nk, nr, kr, r, window, L, dcv, yw,
+                                                                 sgnw, wpar, lv, o);
   full::polarisation_kernel<<<dim3(nb, nw), full::kPolThreads, sp, st>>>(
-      nk, nr, kr, r, window, dcv, yw, sgnw, wpar, lv, o, fit);
+      nk, nr, kr, r, window, dcv, yw, sgnw, wpar, lv, o);
   return check_cuda("sources kernels");
 }
 }  // namespace
