@@ -62,7 +62,8 @@ extern "C" {
  * nkmax (2..64, 65..128, 129..256, 257..512, 513..1024), so one kernel of
  * that class serves the launch; a wire of another class may be refused
  * with PSB_ERR_SIZE.  Without it the FP64 entry points issue one kernel per
- * class up to nkmax's. */
+ * class up to nkmax's, which overlap (each starts once the CTAs of the one
+ * before have). */
 #define PSB_TAB_ONE_CLASS 8
 
 /*

@@ -40,6 +40,17 @@ def wire_group(n, wmax, sms):
     return min(range(1, wmax + 1), key=lambda w: (time(w), -w))
 
 
+# Wires times right-hand sides of a call up to which the size classes of an FP64
+# step go out in one library call, chained on the caller's stream, and above
+# which each has a side stream.  The fork and join cost the host 20 (two classes)
+# to 60 us (five); the library's launches cover every class for all wires, and
+# the CTAs without a wire cost up to 20 % of a leapfrog step of 20480 wires.  us
+# per call, side streams / chained: one leapfrog step of 192 wires of Nk 64, 128,
+# 256 52 / 18, of 1536 53 / 25; one RK4 step of 192 46 / 21, four 46 / 54; one
+# leapfrog step of 2560 wires of Nk 64 .. 1024 94 / 105.
+CHAIN_STAGES = 2048
+
+
 class WireBatch:
     """``form`` selects the step kernel: "plain" (FP64 throughout,
     psb_rk4_f64) or "split" (exchange sums on the int8 tensor cores as exact
@@ -271,7 +282,8 @@ class WireBatch:
     # -- entry points -----------------------------------------------------------
     @property
     def launches_per_call(self):
-        """Kernel launches one rk4/leapfrog call issues (one per size class)."""
+        """Kernel launches of an rk4 call (one per size class; a short FP64
+        call over several, CHAIN_STAGES, covers every class up to the largest)."""
         if self.form == "split":
             return len(self.split_launches) + len(self.wire_launches)
         return len(self.classes)
@@ -297,11 +309,19 @@ class WireBatch:
                 calls.append(lambda s, a=(device.ptr(groups), ng, wg, nkmax, tflags): _lib.call(
                     "psb_rk4_split_wire", *self._common(), *a, *ws, *tail, device.stream_ptr(s)))
         else:
-            for order, nkmax, flags in self.classes:
-                calls.append(lambda s, o=order, nkm=nkmax, f=flags: _lib.call(
-                    "psb_rk4_f64", *self._common(), device.ptr(o), o.numel(), device.ptr(self.y),
-                    self.n_state, nkm, f, *tail, device.stream_ptr(s)))
+            for order, n, nkmax, flags in self._fp64_launches(4 * int(nsteps)):
+                calls.append(lambda s, a=(device.ptr(order), n), b=(nkmax, flags): _lib.call(
+                    "psb_rk4_f64", *self._common(), *a, device.ptr(self.y), self.n_state, *b,
+                    *tail, device.stream_ptr(s)))
         self._concurrent(calls, stream)
+
+    def _fp64_launches(self, stages):
+        """(order, n_order, nkmax, tab_flags) of the library calls of an FP64
+        step of ``stages`` right-hand sides: one per size class, or one for all
+        (see CHAIN_STAGES)."""
+        if len(self.classes) > 1 and self.nw * stages <= CHAIN_STAGES:
+            return [(None, 0, self.nkmax, self.tab_flags)]
+        return [(order, order.numel(), nkmax, flags) for order, nkmax, flags in self.classes]
 
     def capture(self, nsteps, dt, p_stride=1):
         """A CUDA graph of one ``rk4(nsteps, dt, p_stride)`` call (every size
@@ -328,10 +348,10 @@ class WireBatch:
         if self.y1 is None:
             self.y1 = self.y.clone()
         assert field.is_cuda and field.dtype == torch.float64 and field.dim() == 2
-        calls = [lambda s, o=order, nkm=nkmax, f=flags: _lib.call(
-            "psb_leapfrog_f64", *self._common(), device.ptr(o), o.numel(), device.ptr(self.y1),
-            device.ptr(self.y), self.n_state, nkm, f, device.ptr(field), field.shape[1],
-            field.numel(), int(nsteps), float(dt), device.ptr(self.P), self.P.shape[0],
-            int(p_stride), self.p_cap, abi.as_ptr(self.model), device.stream_ptr(s))
-            for order, nkmax, flags in self.classes]
+        calls = [lambda s, a=(device.ptr(order), n), b=(nkmax, flags): _lib.call(
+            "psb_leapfrog_f64", *self._common(), *a, device.ptr(self.y1), device.ptr(self.y),
+            self.n_state, *b, device.ptr(field), field.shape[1], field.numel(), int(nsteps),
+            float(dt), device.ptr(self.P), self.P.shape[0], int(p_stride), self.p_cap,
+            abi.as_ptr(self.model), device.stream_ptr(s))
+            for order, n, nkmax, flags in self._fp64_launches(int(nsteps))]
         self._concurrent(calls, stream)

@@ -785,9 +785,8 @@ __device__ __forceinline__ void wire_steps(const Batch& bt, int mode, bool scr, 
 // are another launch's, unless the caller said that there are none (strict).
 // check: this launch reports bad descriptors.
 template <int L, int MODE>
-__global__ void __launch_bounds__(32 * L, ctas_of(L))
-    sbe_conv_kernel(Batch bt, int mode, bool screened, bool shared, bool check, bool strict) {
-  extern __shared__ __align__(16) uint8_t smem[];
+__device__ __forceinline__ void wire_of_cta(const Batch& bt, int mode, bool screened, bool shared,
+                                            bool check, bool strict, uint8_t* smem) {
   const int wi = bt.order ? bt.order[blockIdx.x] : (int)blockIdx.x;
   if (wi < 0 || wi >= bt.nw) return;
   PsbWire* wp = bt.wires + wi;
@@ -812,6 +811,23 @@ __global__ void __launch_bounds__(32 * L, ctas_of(L))
   if (lanes_of(tb.nk) == L) wire_steps<L, MODE>(bt, mode, screened, smem, wi, tb);
 }
 
+// The launches of one call over several classes follow one another on the
+// stream, but their wires are different ones: each lets the next start once its
+// CTAs have, and a chained one reads nothing that the one before writes.  Its
+// first CTA stays until the launch before is complete, so that what follows on
+// the stream finds the whole call done.  One RK4 step of 192 wires of Nk 64, 128
+// and 256: 46 us one after another, 21 chained (31 with direct sums in one
+// launch).
+template <int L, int MODE>
+__global__ void __launch_bounds__(32 * L, ctas_of(L))
+    sbe_conv_kernel(Batch bt, int mode, bool screened, bool shared, bool check, bool strict,
+                    bool chained) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  asm volatile("griddepcontrol.launch_dependents;");
+  wire_of_cta<L, MODE>(bt, mode, screened, shared, check, strict, smem);
+  if (chained && blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 template <int L>
 uint32_t smem_of(bool shared) {
   return shared ? Lay<L>::total1 : Lay<L>::total3;
@@ -819,11 +835,22 @@ uint32_t smem_of(bool shared) {
 
 template <int L, int MODE>
 int launch_lanes(const Batch& bt, int mode, int grid, bool screened, bool shared, bool check,
-                 bool strict, cudaStream_t st) {
+                 bool strict, bool chained, cudaStream_t st) {
   const uint32_t smem = smem_of<L>(shared);
   const int rc = allow_smem(sbe_conv_kernel<L, MODE>, smem, Lay<L>::total3);
   if (rc != PSB_OK) return rc;
-  sbe_conv_kernel<L, MODE><<<grid, 32 * L, smem, st>>>(bt, mode, screened, shared, check, strict);
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(32 * L);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = chained ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, sbe_conv_kernel<L, MODE>, bt, mode, screened, shared, check, strict,
+                     chained);
   return check_cuda("sbe_conv_kernel");
 }
 
@@ -834,8 +861,8 @@ int launch_down(const Batch& bt, int mode, int grid, int nkmax, int nkmin, bool 
                 bool shared, bool one_class, cudaStream_t st) {
   const int top = lanes_of(nkmax);
   if (L <= top && L >= lanes_of(nkmin + 1)) {
-    const int rc =
-        launch_lanes<L, MODE>(bt, mode, grid, screened, shared, L == top, one_class, st);
+    const int rc = launch_lanes<L, MODE>(bt, mode, grid, screened, shared, L == top, one_class,
+                                         L < top, st);
     if (rc != PSB_OK || one_class) return rc;
   }
   if constexpr (L > (MODE == kRhs ? lanes_of(kDirectNk + 1) : 1))
