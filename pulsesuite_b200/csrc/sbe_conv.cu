@@ -529,7 +529,48 @@ __device__ __forceinline__ void wire_steps(const Batch& bt, int mode, bool scr, 
     double v[2] = {nsum, 0.0};
     put_sums<2>(v, par.red[0], lane, warp);
   }
+  // CalcH returns the two sums of a signal (of Re p and Im p, of n_e and n_h) as
+  // numbers of their own: the second is brought to the size of the first by a
+  // power of two on its way through the transforms, whose rounding error is that
+  // of the larger one, and the sum of a column of zeros is zero.
+  const bool apart = ONCE && exc && mode == kCalcH;
+  int up[2] = {0, 0};         // of Im p, of n_h
+  bool some[4] = {1, 1, 1, 1};  // the column is not all zeros
+  if (apart) {
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      double top = 0.0;
+#pragma unroll
+      for (int e = 0; e < kEpt; ++e) {
+        const double x = fabs(yb[e][v]);
+        top = fmax(top, isfinite(x) ? x : HUGE_VAL);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+      if (lane == 0) par.red[1][v][warp] = top;
+    }
+  }
   cta_sync<L>();
+  if (apart) {
+    double top[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      top[v] = par.red[1][v][0];
+      for (int i = 1; i < L; ++i) top[v] = fmax(top[v], par.red[1][v][i]);
+      some[v] = top[v] > 0.0;
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+      if (some[2 * c] && some[2 * c + 1] && isfinite(top[2 * c]) && isfinite(top[2 * c + 1]))
+        up[c] = ilogb(top[2 * c]) - ilogb(top[2 * c + 1]);
+#pragma unroll
+    for (int e = 0; e < kEpt; ++e) {
+      const int k = tid + e * T;
+      yp[k].y = ldexp(yb[e][1], up[0]);
+      yn[k].y = ldexp(yb[e][3], up[1]);
+    }
+    // (read by others after the barrier behind the tables)
+  }
 
   for (int s = 0; s < nst; ++s) {
     double2 m_lf = make_double2(0.0, 0.0);
@@ -641,10 +682,16 @@ __device__ __forceinline__ void wire_steps(const Batch& bt, int mode, bool scr, 
           // k = a + q r: rows 2 r and 2 r + 1, column a
           const double2* o = E + 2 * (k / q) * rs + k % q;
           const double2 p0 = o[0], p1 = o[rs], n0 = o[16 * rs], n1 = o[17 * rs];
-          om.x += p0.x + p1.x;
-          om.y += p0.y + p1.y;
+          double2 dp = make_double2(p0.x + p1.x, p0.y + p1.y);
           xe = n0.x + n1.x;
           xh = n0.y + n1.y;
+          if (apart) {
+            dp = make_double2(some[0] ? dp.x : 0.0, some[1] ? ldexp(dp.y, -up[0]) : 0.0);
+            xe = some[2] ? xe : 0.0;
+            xh = some[3] ? xh : 0.0;
+          }
+          om.x += dp.x;
+          om.y += dp.y;
         }
         if (ONCE && mode == kCalcH) {
           // renormalised H diagonals (CalcH, SBEs.py:819-935): Heh (Rabi
@@ -654,7 +701,7 @@ __device__ __forceinline__ void wire_steps(const Batch& bt, int mode, bool scr, 
             double2* d2 = reinterpret_cast<double2*>(bt.dy + 4 * off);
             d2[2 * k] = make_double2(om.x * hb, om.y * hb);
             d2[2 * k + 1] = make_double2((blk[3 * nk + k] + par.gap) - xe * hb,
-                                         blk[4 * nk + k] - xh * hb);
+                                         blk[4 * nk + k] - ldexp(xh * hb, -up[1]));
           }
           continue;
         }
