@@ -24,7 +24,12 @@ The SBE arithmetic itself (the O(Nk^2)/O(Nk^3) right-hand side and the
 O(Nr Nk^2) source sums) runs in the sm_100a kernels.
 """
 
+import inspect
+
 import numpy as np
+
+# numpy's transforms write in place from 2.0 on
+_FFT_OUT = "out" in inspect.signature(np.fft.fft).parameters
 
 QW_SMALL = 1e-100  # QWOptics._small (qwoptics.py:604)
 
@@ -43,9 +48,11 @@ def fftg(F):
 def _centred(F, fft, stage):
     """fftg / ifftg of one contiguous complex128 block: the transform in place
     between the library's two sign-and-scale passes (psb_centred_c128: the
-    operations below, the same bits).  False when F is laid out otherwise."""
-    if not (isinstance(F, np.ndarray) and F.dtype == np.complex128 and F.flags.c_contiguous
-            and F.flags.writeable and F.ndim >= 1 and 0 < F.size < 2**31):
+    operations below, the same bits).  False, F untouched, when F is laid out
+    otherwise or numpy's transforms cannot write in place."""
+    if not (_FFT_OUT and isinstance(F, np.ndarray) and F.dtype == np.complex128
+            and F.flags.c_contiguous and F.flags.writeable and F.ndim >= 1
+            and 0 < F.size < 2**31):
         return False
     from . import _lib
 

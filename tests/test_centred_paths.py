@@ -1,0 +1,32 @@
+"""Which arrays fftg / ifftg hand to the library's in-place passes: the rest
+takes the same operations in numpy, with the same bits."""
+
+import importlib.util
+
+import numpy as np
+import pytest
+from test_centred_host import written_out
+
+from pulsesuite_b200 import _lib
+from pulsesuite_b200 import wirespace as ws
+
+
+def signals(shape, seed=3):
+    rng = np.random.default_rng(seed)
+    return rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+
+
+def test_numpy_whose_transforms_take_no_out(monkeypatch):
+    """numpy 1.x: the transforms have no out= argument."""
+    fft, ifft = np.fft.fft, np.fft.ifft
+    monkeypatch.setattr(np.fft, "fft", lambda a, n=None, axis=-1, norm=None: fft(a, n, axis, norm))
+    monkeypatch.setattr(np.fft, "ifft",
+                        lambda a, n=None, axis=-1, norm=None: ifft(a, n, axis, norm))
+    spec = importlib.util.spec_from_file_location("pulsesuite_b200.wirespace_again", ws.__file__)
+    again = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(again)
+    F = signals((8, 230))
+    for f, inverse in ((again.fftg, False), (again.ifftg, True)):
+        G = F.copy()
+        f(G)
+        np.testing.assert_array_equal(G, written_out(F, inverse))
