@@ -46,13 +46,13 @@ def fftg(F):
 
 
 def _centred(F, fft, stage):
-    """fftg / ifftg of one contiguous complex128 block: the transform in place
-    between the library's two sign-and-scale passes (psb_centred_c128: the
-    operations below, the same bits).  False, F untouched, when F is laid out
-    otherwise or numpy's transforms cannot write in place."""
+    """fftg / ifftg of one contiguous, aligned complex128 block: the transform
+    in place between the library's two sign-and-scale passes
+    (psb_centred_c128: the operations below, the same bits).  False, F
+    untouched, when F is laid out otherwise or numpy's transforms cannot write
+    in place."""
     if not (_FFT_OUT and isinstance(F, np.ndarray) and F.dtype == np.complex128
-            and F.flags.c_contiguous and F.flags.writeable and F.ndim >= 1
-            and 0 < F.size < 2**31):
+            and F.flags.carray and F.ndim >= 1 and 0 < F.size < 2**31):
         return False
     from . import _lib
 

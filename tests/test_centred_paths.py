@@ -30,3 +30,22 @@ def test_numpy_whose_transforms_take_no_out(monkeypatch):
         G = F.copy()
         f(G)
         np.testing.assert_array_equal(G, written_out(F, inverse))
+
+
+def test_arrays_the_library_cannot_take(monkeypatch):
+    """Signals whose doubles do not lie on 8-byte boundaries, in rows apart, or
+    read-only: never handed over."""
+    monkeypatch.setattr(_lib, "call", lambda *a: pytest.fail("handed to the library"))
+    F = signals((8, 230))
+    raw = np.empty(F.nbytes + 4, np.uint8)[4:].view(np.complex128).reshape(F.shape)
+    assert not raw.flags.aligned
+    strided = np.empty((8, 460), np.complex128)[:, ::2]
+    for G in (raw, strided):
+        for f, inverse in ((ws.fftg, False), (ws.ifftg, True)):
+            G[...] = F
+            f(G)
+            np.testing.assert_array_equal(G, written_out(F, inverse))
+    G = F.copy()
+    G.flags.writeable = False
+    with pytest.raises(ValueError):
+        ws.fftg(G)
