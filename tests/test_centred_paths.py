@@ -49,3 +49,17 @@ def test_arrays_the_library_cannot_take(monkeypatch):
     G.flags.writeable = False
     with pytest.raises(ValueError):
         ws.fftg(G)
+
+
+@pytest.mark.parametrize("shape,library", [((64,), False), ((3, 85), False), ((256,), True),
+                                           ((8, 32), True), ((5, 230), True)])
+def test_small_signals_stay_in_numpy(monkeypatch, shape, library):
+    """Below 256 values the library's two calls cost more than they save."""
+    real, calls = _lib.call, []
+    monkeypatch.setattr(_lib, "call", lambda *a: calls.append(a[0]) or real(*a))
+    F = signals(shape)
+    for f, inverse in ((ws.fftg, False), (ws.ifftg, True)):
+        G = F.copy()
+        f(G)
+        np.testing.assert_array_equal(G, written_out(F, inverse))
+    assert calls == (["psb_centred_c128"] * 4 if library else [])
