@@ -40,6 +40,20 @@ def wire_group(n, wmax, sms):
     return min(range(1, wmax + 1), key=lambda w: (time(w), -w))
 
 
+def groups_of(table, wires, wg):
+    """Split-form groups (SPLIT_GROUP_DTYPE) of wg of the given wires each, all
+    of one table; the last holds what is left.  Unused slots are -1."""
+    g = np.zeros(-(-len(wires) // wg), dtype=abi.SPLIT_GROUP_DTYPE)
+    g["table"] = table
+    g["nw"] = wg
+    g["nw"][-1] = len(wires) - (len(g) - 1) * wg
+    slots = np.full(len(g) * wg, -1, dtype=np.int64)
+    slots[:len(wires)] = wires
+    g["wire"] = -1
+    g["wire"][:, :wg] = slots.reshape(len(g), wg)
+    return g
+
+
 # Wires times right-hand sides of a call up to which the size classes of an FP64
 # step go out in one library call, chained on the caller's stream, and above
 # which each has a side stream.  The fork and join cost the host 20 (two classes)
@@ -198,15 +212,7 @@ class WireBatch:
                     raise _lib.PsbError(f"split form: nk {nk} exceeds the supported maximum")
                 key = (wg, nk <= resnk[wg])
                 target_classes = classes
-            g = np.zeros(-(-len(ws) // wg), dtype=abi.SPLIT_GROUP_DTYPE)
-            g["table"] = t
-            g["nw"] = wg
-            g["nw"][-1] = len(ws) - (len(g) - 1) * wg
-            slots = np.full(len(g) * wg, -1, dtype=np.int64)
-            slots[:len(ws)] = ws
-            g["wire"] = -1
-            g["wire"][:, :wg] = slots.reshape(len(g), wg)
-            target_classes.setdefault(key, []).append(g)
+            target_classes.setdefault(key, []).append(groups_of(t, ws, wg))
         self.split_launches = []
         for key in classes:
             ga = np.concatenate(classes[key])
