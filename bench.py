@@ -58,8 +58,7 @@ sys.path.insert(0, REPO)
 L2_FLUSH_BYTES = 256 << 20
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of the step
 # kernels, from one ncu capture of a 20-step call on the configuration-4
-# request mix (16384 solves; profiles/split_rk4_kernel_c4_mix.md,
-# profiles/sbe_conv_kernel_c4_mix.md):
+# request mix (16384 solves):
 #   split, state resident in shared memory: per element and launch (the
 #     FP64 state read once and written once)
 #   split, state in the workspace (groups whose grid does not fit shared

@@ -201,7 +201,9 @@ int psb_rhs_f64(const PsbTable* d_tables, int ntab, const double* d_tabdata, int
  * d_h[e] = (Re Heh, Im Heh, Hee, Hhh) per element, where Heh = M(t_w) +
  * sum_{q!=0} Veh(q) p_{k+q}, Hee = Ee + gap - sum Vee(q) n_e,k+q and
  * Hhh = Eh - sum Vhh(q) n_h,k+q.  M(t_w) is the wire's drive at its own t
- * (zero for npulse = 0).
+ * (zero for npulse = 0).  Above 256 points the sums go through transforms:
+ * their rounding error is 4e-15 of the largest sum of Re Heh, Im Heh, Hee or
+ * Hhh each, no longer of every element.
  */
 int psb_calch_f64(const PsbTable* d_tables, int ntab, const double* d_tabdata, int64_t n_tabdata,
                   const PsbWire* d_wires, int nw, const double* d_y, double* d_h,
@@ -277,7 +279,8 @@ typedef struct PsbFullParams {
   int32_t lf;       /* mb.params LF: full Hee/Hhh with the direct terms        */
 } PsbFullParams;
 
-/* Work bytes psb_full_step_f64 needs for a grid of nk (Meh, H, dX). */
+/* Work bytes psb_full_step_f64 needs for a grid of nk (sums of the
+ * occupations, H, X1 + 2 dt dX). */
 int64_t psb_full_work_bytes(int nk);
 /*
  * One step of the reference's integrator for one wire with full Nk x Nk
@@ -315,7 +318,7 @@ int psb_full_sources_f64(int nk, int nr, const double* d_kr, const double* d_r,
 
 /*
  * The many-body terms of the full-matrix step that mb.params switches on,
- * all FP64 and in the reference's summation order:
+ * all FP64, sums regrouped (equal to the reference's to rounding):
  *  - diag_dph:    k-dependent dephasing rates GamE, GamH replace gam_e, gam_h
  *                 in dpdt (CalcGammaE / CalcGammaH, dephasing.py:28-105,
  *                 540-625; SBEs.py:5225-5228);

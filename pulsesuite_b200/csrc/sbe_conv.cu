@@ -6,12 +6,19 @@
 //   Omega_k += sum_k' Veh p_k'   Se_k -= sum Vee ne   Sh_k -= sum Vhh nh
 // i.e. 8 Nk FP64 flops per point when summed directly.  As cyclic
 // convolutions of length M >= 2 Nk of the complex signals p and ne + i nh
-// (zero beyond Nk) they take one forward and one inverse transform each:
-// about 100 log2(M) flops per point, in FP64 as before (the rounding error
-// is that of a sum: ~1e-16 of the largest term).  A real, even table has a
-// real spectrum, so with one shared table both signals are multiplied by the
+// (zero beyond Nk) they take one forward and one inverse transform each, four
+// of 5 M log2 M flops: 40 log2 M per point at M = 2 Nk.  A real, even table has
+// a real spectrum, so with one shared table both signals are multiplied by the
 // same real numbers; with distinct Vee and Vhh the second signal's product
 // is Z (Vee + Vhh)/2 + conj(Z(-f)) (Vee - Vhh)/2.
+//
+// Rounding.  All in FP64, as the direct sums, but the error is relative to the
+// largest sum of a signal, about 2^-53 3 log2 M (4e-15) of it at most, not to
+// each sum: sums far from the carriers that are small beside it have fewer
+// digits.  The two parts of a complex signal share it too, n_h's sums that of
+// n_e's; a step adds these up, and CalcH, which returns them, brings the parts
+// to one size first.  Whole passes are as close to 64-bit references as with
+// direct sums (1e-16 to 1e-15 of the largest value).
 //
 // Transform.  M = 16 q, q = 8 L with L = 1, 2, 4, 8, 16 lanes (Nk <= 64 L);
 // T = 32 L threads with 8 complex points each:
@@ -42,13 +49,13 @@
 // stage (86 % of the pipe at Nk 512), with the FP64 pipe at 54 % beside it; a
 // lone wire is bound by the latency of its stages.  Measured
 // on B200 against the direct sums it replaces (us per wire-stage and SM, 3552
-// wires; in brackets us per stage of one wire; screened):
-//   Nk      direct                transforms
-//   64      1.44 (2.47)  2.1      0.22 (1.88)  0.45
-//   128     1.98 (3.07)  2.9      0.52 (2.15)  0.96
-//   256     4.49 (5.79)  5.7      1.08 (2.39)  1.85
-//   512     14.9 (16.6)  17.0     2.35 (3.56)  3.98
-//   1024    60.0 (60.2)  58.7     6.10 (6.44)  9.98
+// wires; in brackets us per stage of one wire):
+//   Nk     direct       screened       transforms    screened
+//   64     1.42 (2.07)  2.01 (3.31)    0.20 (1.45)   0.39 (3.11)
+//   128    1.97 (2.68)  2.83 (4.24)    0.50 (1.71)   0.88 (3.46)
+//   256    4.49 (5.45)  5.65 (7.59)    1.08 (2.05)   1.76 (4.03)
+//   512    14.9 (16.2)  16.9 (21.3)    2.37 (3.12)   3.91 (6.79)
+//   1024   60.0 (59.9)  58.8 (58.4)    6.21 (6.01)   10.1 (9.89)
 #include <math.h>
 
 #include "fft64.cuh"

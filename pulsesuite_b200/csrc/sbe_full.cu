@@ -22,9 +22,11 @@
 // psb_full_sources_f64 evaluates the wire-space source terms of the new
 // level: the polarisation components of QWPolarization3 and the charge
 // densities of QWRho5 before their transforms (qwoptics.py:56-84, 367-381).
-// Every sum runs in the reference's order; results agree with it to
-// rounding (numpy's pairwise sums and the kernels' sequential ones differ
-// in the last bits).
+// FP64 throughout.  The sums are regrouped for the machine and agree with the
+// reference's to rounding (tests: 1e-10 of its own runs, 1e-12 of 64-bit
+// restatements).  Three keep one fixed order and rounding whatever the launch,
+// because the charge density is a difference that cancels to their last digits:
+// the density sums, the occupations' sums and the DC shift.
 #include <type_traits>
 
 #include "dmma.cuh"
@@ -673,8 +675,9 @@ __global__ void __launch_bounds__(kSrcThreads) densities_kernel(
 }
 
 // ---------------------------------------------------------------------------
-// Many-body terms switched on by mb.params (PsbFullMB).  Each kernel keeps
-// the reference's loop order for every accumulated value.
+// Many-body terms switched on by mb.params (PsbFullMB).  Their sums are split
+// over lanes and regrouped (each kernel says how): the reference's values to
+// rounding, and the same bits for a wire alone and in any batch.
 // ---------------------------------------------------------------------------
 struct MBView {
   int nk;
@@ -1446,7 +1449,9 @@ extern "C" int psb_mb_tables_f64(int nk, const double* d_Ee, const double* d_Eh,
 }
 
 namespace {
-// per-wire work of a batch: Meh, H, dX, then the screened V3 and eps
+// per-wire work of a batch: seven matrices' room (the occupations' sums in the
+// first, H in the next three, X1 + 2 dt dX in the last three), then the screened
+// V3 and eps
 struct BatchWork {
   size_t v3, eps, total;
   explicit BatchWork(int nk) {
